@@ -19,7 +19,7 @@ constexpr int64_t kChunkElems = 4 << 20;     // staging chunk (elements)
 using rp::kMaxNp;
 
 struct GridBuf {
-    int nx = 0, ny = 0, N = 0, vtransform = 2;
+    int nx = 0, ny = 0, N = 0, vtransform = 2, asc = 0;
     double hc = 0.0;
     double *h = nullptr, *pm = nullptr, *pn = nullptr;
     double *sr = nullptr, *csr = nullptr, *sw = nullptr, *csw = nullptr;
@@ -231,7 +231,7 @@ void fill_grids(const rp_ctx* c, RpStepArgs& A, int tb, int tc, int tf) {
     for (int k = 0; k < c->ngrid; k++) {
         const GridBuf& G = c->g[k];
         RpGridDev& d = A.g[k];
-        d.nx = G.nx; d.ny = G.ny; d.N = G.N; d.vtransform = G.vtransform; d.hc = G.hc;
+        d.nx = G.nx; d.ny = G.ny; d.N = G.N; d.vtransform = G.vtransform; d.hc = G.hc; d.asc = G.asc;
         d.h = G.h; d.pm = G.pm; d.pn = G.pn;
         d.mrho = G.mrho; d.mu = G.mu; d.mv = G.mv;
         d.sr = G.sr; d.csr = G.csr; d.sw = G.sw; d.csw = G.csw;
@@ -826,6 +826,10 @@ int rp_create(const rp_params* params, int32_t ngrid, const rp_grid* grids, rp_c
             cudaMemcpy(G.scs_r, pr.data(), G.N * sizeof(float2), cudaMemcpyHostToDevice);
             cudaMemcpy(G.scs_w, pw.data(), sw * sizeof(float2), cudaMemcpyHostToDevice);
         }
+        G.asc = R.vtransform == 2 && R.hc >= 0.0 && R.hc < 1e30;
+        for (int k = 1; k < G.N; k++)
+            G.asc = G.asc && R.s_rho[k] >= R.s_rho[k - 1] && R.cs_r[k] >= R.cs_r[k - 1];
+        for (int k = 1; k < sw; k++) G.asc = G.asc && R.s_w[k] >= R.s_w[k - 1] && R.cs_w[k] >= R.cs_w[k - 1];
         if (!mask8(R.mask_rho, n2)) return bail(RP_ERR_ARG, "mask_rho values must be 0 or 1");
         cudaMemcpy(G.mrho, m8.data(), n2, cudaMemcpyHostToDevice);
         {
@@ -1120,8 +1124,7 @@ int step_launch(rp_ctx* ctx, const double ex[3], const double ix[3], int32_t ets
         CK(rp::launch_step_mixed(A, ctx->npmax, ctx->i16, (float*)ctx->turbv, ctx->prm.reserved[0], s,
                                  ctx->num_sms, nl));
     else if (ctx->n > 0)
-        CK(rp::launch_step(A, ctx->prm.field_dtype, ctx->npmax, ctx->turbv, ctx->prm.reserved[0] == 1 ? 0 : 1, s,
-                           ctx->num_sms, nl));
+        CK(rp::launch_step(A, ctx->prm.field_dtype, ctx->npmax, ctx->turbv, s, ctx->num_sms, nl));
     ctx->step_index++;
     if (ctx->hook) ctx->hook_pos++;
     return RP_OK;

@@ -41,6 +41,7 @@
 struct RpGridDev {
     int nx, ny, N;                 // rho dims, s_rho
     int vtransform;
+    int asc;                       // Vtransform 2, hc >= 0 and s, Cs ascend: the level depths ascend (rp_walk2)
     double hc;
     const double* h;
     const double* pm;
@@ -235,31 +236,105 @@ __device__ __forceinline__ double rp_ld(const void* base, int64_t idx) {
 
 // ------------------------------------------------------ exact division
 //
-// a / b rounded to nearest, given y = RN(1/b) (CUDA's __drcp_rn): two
+// a / b rounded to nearest, given y = RN(1/b) (rp_rcp): two
 // residual corrections q <- q + (a - b q) y with the residual formed exactly
 // by an FMA.  By Markstein's theorem (P. Markstein, "Computation of
 // elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
 // Dev. 34(1), 1990), if y = RN(1/b) and q is within one ulp of a/b, then
 // RN(q + (a - bq) y) = RN(a/b); the first correction brings RN(a y) within
-// one ulp.  Operands outside [1e-150, 1e150] in magnitude (where a residual
+// one ulp.  Operands outside about [1e-150, 1e150] in magnitude (where a residual
 // could underflow), zero, Inf or NaN take the IEEE division instead, so the
 // result is always the correctly rounded quotient -- the value `a / b`
 // gives -- while divisions sharing a denominator share one reciprocal.
-__device__ __forceinline__ bool rp_div_safe(double b) {
-    const double ab = fabs(b);
-    return ab > 1e-150 && ab < 1e150;
+// (2^-498 and 2^498 here: the test is one of the biased exponent, in the
+// integer pipe.)
+__device__ __forceinline__ uint32_t rp_exp_off(double b) {
+    return ((uint32_t)__double2hiint(b) << 1) - 0x41a00000u;
+}
+constexpr uint32_t kDivSpan = 0xbe200000u - 0x41a00000u;
+
+__device__ __forceinline__ bool rp_div_safe(double b) { return rp_exp_off(b) < kDivSpan; }
+
+// 1 / b within 1 ulp for b in range: Newton-Raphson twice (2^-19, 2^-38,
+// rounding) on the hardware's approximation of the leading bits.
+__device__ __forceinline__ double rp_rcp_near(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    y = fma(y, fma(-b, y, 1.0), y);
+    return fma(y, fma(-b, y, 1.0), y);
 }
 
-__device__ __forceinline__ double rp_rcp(double b) { return __drcp_rn(b); }
+// True where the correction below need not round correctly: a significand of
+// all ones (Markstein's exception).
+__device__ __forceinline__ uint32_t rp_ones(double b) {
+    return ((uint32_t)__double2hiint(b) | 0xfff00000u) & (uint32_t)__double2loint(b);
+}
+__device__ __forceinline__ bool rp_all_ones(double b) { return rp_ones(b) == 0xffffffffu; }
 
-__device__ __forceinline__ double rp_div_by(double a, double b, double y) {
-    const double aa = fabs(a);
-    if (!(aa > 1e-150 && aa < 1e150) || !rp_div_safe(b)) return a / b;
-    const double q0 = a * y;
+// RN(1 / b) from y within 1 ulp of it, b in range and not all ones (the
+// reciprocal counterpart of the theorem above, from the same paper)
+__device__ __forceinline__ double rp_rcp_round(double b, double y) { return fma(y, fma(-b, y, 1.0), y); }
+
+// RN(1 / b).  Inlined, and free of branches but for the cold one: __drcp_rn
+// took 61 cycles on B200 whatever stood beside it (4 independent ones 243),
+// which a row of the spline factorisation, one reciprocal deep, waited for.
+__device__ __forceinline__ double rp_rcp(double b) {
+    if (!rp_div_safe(b) || rp_all_ones(b)) return 1.0 / b;
+    return rp_rcp_round(b, rp_rcp_near(b));
+}
+
+// RN(a / b) for operands in range; y = RN(1 / b), y0 within 1 ulp of it
+__device__ __forceinline__ double rp_div_fast(double a, double b, double y, double y0) {
+    const double q0 = a * y0;
     const double r0 = fma(-b, q0, a);
-    const double q1 = fma(r0, y, q0);
+    const double q1 = fma(r0, y0, q0);
     const double r1 = fma(-b, q1, a);
     return fma(r1, y, q1);
+}
+
+// rp_exp_off where the value may also be 0.  A dividend of 0 gives a 0 by
+// rp_div_fast, +0 where IEEE division may give -0; no result that is not
+// itself 0 can show the difference.
+__device__ __forceinline__ uint32_t rp_exp_off_z(double a) {
+    const uint32_t hi2 = (uint32_t)__double2hiint(a) << 1;
+    return ((hi2 | (uint32_t)__double2loint(a)) == 0u) ? 0u : hi2 - 0x41a00000u;
+}
+
+// 1 / b for several dividends in flight: y0 about 2^-38 and y1 within 1 ulp
+// of 1 / b, y = RN(1 / b); rp_div_rcp(a, b, R) = RN(a / b).  The quotient
+// starts on y0 while y1 and y are still being formed, so that a / b is seven
+// dependent operations behind the approximation of 1 / b.
+struct RpRcp {
+    double y0, y1, y;
+};
+__device__ __forceinline__ RpRcp rp_rcp3(double b) {
+    RpRcp R;
+    double s;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(s) : "d"(b));
+    R.y0 = fma(s, fma(-b, s, 1.0), s);
+    R.y1 = fma(R.y0, fma(-b, R.y0, 1.0), R.y0);
+    R.y = rp_rcp_round(b, R.y1);
+    return R;
+}
+__device__ __forceinline__ double rp_div_rcp(double a, double b, const RpRcp& R) {
+    const double q0 = a * R.y0;
+    const double r0 = fma(-b, q0, a);
+    const double q1 = fma(r0, R.y1, q0);
+    const double r1 = fma(-b, q1, a);
+    return fma(r1, R.y, q1);
+}
+
+// RN(a / b) given y = RN(1 / b)
+__device__ __forceinline__ double rp_div_by(double a, double b, double y) {
+    if (max(rp_exp_off_z(a), rp_exp_off(b)) >= kDivSpan) return a / b;
+    return (a == 0.0) ? a * y : rp_div_fast(a, b, y, y);
+}
+
+// RN(a / b), inlined (as rp_rcp)
+__device__ __forceinline__ double rp_quot(double a, double b) {
+    if (max(rp_exp_off_z(a), rp_exp_off(b)) >= kDivSpan || rp_all_ones(b)) return a / b;
+    const double y0 = rp_rcp_near(b);
+    return (a == 0.0) ? a * y0 : rp_div_fast(a, b, rp_rcp_round(b, y0), y0);
 }
 
 __device__ __forceinline__ double rp_polintd(const RpPolint& P, double y0, double y1, double y2) {
@@ -271,6 +346,25 @@ __device__ __forceinline__ double rp_polintd(const RpPolint& P, double y0, doubl
     const double a = (P.ns == 2) ? q12 : q01;
     const double yns = (P.ns == 0) ? y0 : ((P.ns == 1) ? y1 : y2);
     return yns + P.dns * a + P.b * c;
+}
+
+// Two of them side by side, the quotients' operands tested together
+__device__ __forceinline__ void rp_polintd2(const RpPolint& P, const double (&u)[3], const double (&v)[3], double& ru,
+                                            double& rv) {
+    const double ua = u[2] - u[1], ub = u[1] - u[0], va = v[2] - v[1], vb = v[1] - v[0];
+    double uq12 = rp_div_fast(ua, P.e12, P.re12, P.re12), uq01 = rp_div_fast(ub, P.e01, P.re01, P.re01);
+    double vq12 = rp_div_fast(va, P.e12, P.re12, P.re12), vq01 = rp_div_fast(vb, P.e01, P.re01, P.re01);
+    double uc = P.d1 * uq12 - P.d1 * uq01, vc = P.d1 * vq12 - P.d1 * vq01;
+    double ur = rp_div_fast(uc, P.e02, P.re02, P.re02), vr = rp_div_fast(vc, P.e02, P.re02, P.re02);
+    const uint32_t off = max(max(max(rp_exp_off_z(ua), rp_exp_off_z(ub)), max(rp_exp_off_z(va), rp_exp_off_z(vb))),
+                             max(rp_exp_off_z(uc), rp_exp_off_z(vc)));
+    if (off >= kDivSpan || max(max(rp_exp_off(P.e12), rp_exp_off(P.e01)), rp_exp_off(P.e02)) >= kDivSpan) {
+        ru = rp_polintd(P, u[0], u[1], u[2]);
+        rv = rp_polintd(P, v[0], v[1], v[2]);
+        return;
+    }
+    ru = ((P.ns == 0) ? u[0] : ((P.ns == 1) ? u[1] : u[2])) + P.dns * ((P.ns == 2) ? uq12 : uq01) + P.b * ur;
+    rv = ((P.ns == 0) ? v[0] : ((P.ns == 1) ? v[1] : v[2])) + P.dns * ((P.ns == 2) ? vq12 : vq01) + P.b * vr;
 }
 
 // getcoeff (interpolation_module.f90:1230-1273) with the exact-node pin.
@@ -576,6 +670,66 @@ __device__ __forceinline__ void rp_walk_w(const RpGridDev& g, double zeta, doubl
     }
 }
 
+// Both brackets.  With Vtransform 2, ascending s and Cs (RpGridDev::asc), hc
+// >= 0, h > 0 and zeta + h > 0 every operation of the level formula is
+// monotone in the level and rounding keeps that, so the depths ascend and the
+// first one above zpar is found by bisection; w level k lies between rho
+// levels k-1 and k, so the w bracket is one of two, checked.  Eight depths
+// instead of the walks' 31 on average at 30 levels; anything else walks.
+__device__ __forceinline__ void rp_walk2(const RpGridDev& g, double zeta, double depth, double zpar, LevelPick& Lr,
+                                         LevelPick& Lw, uint32_t& fl) {
+    const double h = -1.0 * depth;
+    const int N = g.N;
+    if (!(g.asc && h > 0.0 && h < 1e30 && zeta + h > 0.0 && zeta < 1e30 && zpar == zpar)) {
+        rp_walk_rho(g, zeta, depth, zpar, Lr);
+        rp_walk_w(g, zeta, depth, zpar, Lw, fl);
+        return;
+    }
+    const ZCtx zc = rp_zctx(2, g.hc, h);
+    auto zr = [&](int k) -> double { return rp_zlevel_c(zc, __ldg(g.sr + k - 1), __ldg(g.csr + k - 1), zeta); };
+    auto zw = [&](int k) -> double { return rp_zlevel_c(zc, __ldg(g.sw + k - 1), __ldg(g.csw + k - 1), zeta); };
+    int lo = 0, hi = N + 1;                      // zr(lo) <= zpar < zr(hi), the ends virtual
+    double zlo = 0.0, zhi = 0.0;
+#pragma unroll 1
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        const double z = zr(mid);
+        if (z > zpar) {
+            hi = mid;
+            zhi = z;
+        } else {
+            lo = mid;
+            zlo = z;
+        }
+    }
+    if (hi > N) {
+        Lr.ibot = N; Lr.itop = N; Lr.z1 = 0.5; Lr.z2 = 0.5;
+    } else if (hi == 1) {
+        Lr.ibot = 1; Lr.itop = 1; Lr.z1 = 0.5; Lr.z2 = 0.5;
+    } else {
+        const double Z = rp_quot(zpar - zlo, zhi - zlo);
+        Lr.ibot = hi - 1; Lr.itop = hi; Lr.z1 = 1.0 - Z; Lr.z2 = Z;
+    }
+    // the first w level above zpar: hi or hi + 1 (N + 2: none)
+    const double wm = zw(hi);
+    const bool up = !(wm > zpar);
+    const int iw = up ? hi + 1 : hi;
+    const double wo = up ? ((iw <= N + 1) ? zw(iw) : 0.0) : ((iw > 1) ? zw(iw - 1) : 0.0);
+    const double w1 = up ? wm : wo, w2 = up ? wo : wm;   // zw(iw - 1), zw(iw)
+    if ((iw <= N + 1 && !(w2 > zpar)) || (iw > 1 && !(w1 <= zpar))) {
+        rp_walk_w(g, zeta, depth, zpar, Lw, fl);
+    } else if (iw > N + 1) {
+        fl |= RP_FL_WTOP;
+        Lw.ibot = N + 1; Lw.itop = N + 1; Lw.z1 = 0.5; Lw.z2 = 0.5;
+    } else if (iw == 1) {
+        fl |= RP_FL_WBOT;
+        Lw.ibot = 1; Lw.itop = 1; Lw.z1 = 0.5; Lw.z2 = 0.5;
+    } else {
+        const double Z = rp_quot(zpar - w1, w2 - w1);
+        Lw.ibot = iw - 1; Lw.itop = iw; Lw.z1 = 1.0 - Z; Lw.z2 = Z;
+    }
+}
+
 // zprof(ibot/itop) blend of one slot: zcff1*zprof(Ibot) + zcff2*zprof(Itop)
 template <typename T>
 __device__ __forceinline__ double rp_col_uv(const void* f, const UVCell& c, int nlev, const LevelPick& L,
@@ -711,7 +865,7 @@ __device__ __forceinline__ double rp_log_pos(double x) {
     int e = (int)((b >> 52) & 0x7ffull) - 1023;
     double m = __longlong_as_double((long long)((b & 0x000fffffffffffffull) | 0x3ff0000000000000ull));
     if (m > RP_SQRT2) { m = m * 0.5; e = e + 1; }
-    const double z = (m - 1.0) / (m + 1.0);
+    const double z = rp_quot(m - 1.0, m + 1.0);
     const double z2 = RP_MUL(z, z);
     double p = 1.0 / 23.0;
     p = RP_ADD(RP_MUL(p, z2), 1.0 / 21.0);

@@ -12,9 +12,14 @@ namespace rp {
 
 constexpr int kStepBlock = 128;
 #ifndef RP_VTURB_MIN_BLOCKS
-#define RP_VTURB_MIN_BLOCKS 8
+#define RP_VTURB_MIN_BLOCKS 16
 #endif
-constexpr int kVturbMinBlocks = RP_VTURB_MIN_BLOCKS;   // resident 128-thread blocks per SM
+constexpr int kVturbMinBlocks = RP_VTURB_MIN_BLOCKS;   // exact form: VTurb's one-warp blocks per SM
+constexpr int kVturbSharedBlocks = 10;                 // the same where u is in shared memory
+#ifndef RP_ADVECT_MIN_BLOCKS
+#define RP_ADVECT_MIN_BLOCKS 5
+#endif
+constexpr int kAdvectMinBlocks = RP_ADVECT_MIN_BLOCKS; // exact form: 128-thread blocks of the rest of the step
 #ifndef RP_MIXED_MIN_BLOCKS
 #define RP_MIXED_MIN_BLOCKS 8
 #endif
@@ -26,10 +31,10 @@ constexpr int kMixedVtMinBlocks = RP_MIXED_VT_BLOCKS;  // split mixed form: VTur
 
 constexpr int kMaxNp = 144;   // largest spline point count int(s_w*sub)
 
-// variant 1: fused single kernel with a local-memory spline workspace;
-// variant 0: split (k_vturb + k_advect, `turbv` is n doubles of scratch)
-cudaError_t launch_step(const RpStepArgs& A, int field_dtype, int npmax, double* turbv, int variant,
-                        cudaStream_t s, int num_sms, int* nlaunch);
+// k_vturb (with VTurb on) and k_advect; np: the largest spline point count
+// of the grids, turbv: n doubles of scratch
+cudaError_t launch_step(const RpStepArgs& A, int field_dtype, int np, double* turbv, cudaStream_t s, int num_sms,
+                        int* nlaunch);
 // Split step with the scratch array in a static device buffer (no device
 // allocation); at most kNoallocMaxParticles particles and np <= 128.
 constexpr int64_t kNoallocMaxParticles = 1048576;

@@ -10,40 +10,41 @@ namespace rp {
 
 // ------------------------------------------------------------ the step
 //
-// Split form: k_vturb_local (VTurb of each particle, spline workspace in
-// local memory, many resident warps) writes each particle's displacement to
-// scratch; k_advect (RK4, HTurb, hand-off, vertical update, status) then
-// runs at its own register count.  Fused form: one kernel per particle.
+// With VTurb on, k_vturb writes each particle's displacement to scratch;
+// k_advect (RK4, HTurb, hand-off, vertical update, status) then runs at its
+// own register count.
+//
+// k_vturb: eight chol1d passes of some 124 rows per particle.  With few
+// particles a warp's chain of dependent FP64 operations sets the time, with
+// many the passes' traffic: 72 B a row and pass through L2 and DRAM, about
+// 5 TB/s.  On the 512x384x30 grid with 1,048,576 particles the step (both
+// kernels) takes 14.3 ms, 24.9 as one kernel whose rows divided by the IEEE
+// operator four times (102,000 FP64 instructions per warp and fit, 65,000
+// now); on the 130x98x20 grid with 10,000 particles 0.33 ms, 0.73 before.
+//
+// k_advect: four stages of gathers.  Five 128-thread blocks an SM (96
+// registers) took 0.78 ms at 1,048,576 particles, four 0.83, six 0.79, eight
+// 0.82; its stages unrolled and its levels walked, 2.1 ms in blocks of 168
+// registers and 1.1 ms fused at 64.
 
-// VTurb alone with the spline workspace in local memory, at high occupancy
-// (the latency of the FP64 dependency chains and of the workspace loads is
-// hidden by many resident warps).
-template <typename T, int NPMAX>
-__global__ void __launch_bounds__(kStepBlock, kVturbMinBlocks) k_vturb_local(const __grid_constant__ RpStepArgs A,
-                                                                            double* __restrict__ turbv) {
-    double buf[kSplineArrays * (NPMAX + 1)];
-    const SplineView<NPMAX, 1> w{buf};
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < A.p.n; n += stride)
+// VTurb alone, one warp per block.  SU: the fits' u in shared memory.
+template <typename T, int NPMAX, bool SU>
+__global__ void __launch_bounds__(32, SU ? kVturbSharedBlocks : kVturbMinBlocks) k_vturb(const __grid_constant__ RpStepArgs A,
+                                                               double* __restrict__ turbv) {
+    extern __shared__ double su[];
+    __align__(16) double buf[SplineLocal<NPMAX, SU>::kDoubles];
+    const SplineLocal<NPMAX, SU> w{buf, su + threadIdx.x};
+    const int64_t stride = (int64_t)gridDim.x * 32;
+    for (int64_t n = (int64_t)blockIdx.x * 32 + threadIdx.x; n < A.p.n; n += stride)
         rp_vturb_one<T>(A, n, w, turbv);
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kStepBlock) k_advect(const __grid_constant__ RpStepArgs A,
+__global__ void __launch_bounds__(kStepBlock, kAdvectMinBlocks) k_advect(const __grid_constant__ RpStepArgs A,
                                                       const double* __restrict__ turbv) {
-    const SplineView<1, 1> none{nullptr};
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < A.p.n; n += stride)
-        rp_update_one<T>(A, n, none, turbv);
-}
-
-template <typename T, int NPMAX>
-__global__ void __launch_bounds__(kStepBlock, kVturbMinBlocks) k_step_fused(const __grid_constant__ RpStepArgs A) {
-    double buf[kSplineArrays * (NPMAX + 1)];
-    const SplineView<NPMAX, 1> w{buf};
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < A.p.n; n += stride)
-        rp_update_one<T>(A, n, w, nullptr);
+        rp_update_one<T>(A, n, turbv);
 }
 
 template <class K>
@@ -59,40 +60,51 @@ static int64_t grid_for(K kernel, int block, size_t smem, int64_t n, int num_sms
 }
 
 template <typename T, int NPMAX>
-static cudaError_t launch_step_t(const RpStepArgs& A, double* turbv, int variant, cudaStream_t s, int num_sms,
+static cudaError_t launch_vturb(const RpStepArgs& A, int np, double* turbv, cudaStream_t s, int num_sms) {
+    cudaError_t e = cudaSuccess;
+    const int cap = A.grid_cap * (kStepBlock / 32);
+    const size_t smem = (size_t)np * 32 * sizeof(double);      // the warp's u
+    // Where every warp can be resident with its u in shared memory (1 KB a
+    // particle at 124 points: 7 warps an SM) it is: the rows then wait for
+    // L2 less often (130x98x20 grid, 10,000 particles: 0.33 ms a step, 0.37
+    // with u in local memory).  With more particles than that, 16 warps an
+    // SM with u in local memory hide more than shared memory saves
+    // (512x384x30, 1,048,576 particles: 14.3 ms against 18.3).
+    const int64_t need = (A.p.n + 31) / 32;
+    const int64_t fit = grid_for(k_vturb<T, NPMAX, true>, 32, smem, A.p.n, num_sms, &e, cap);
+    if (e != cudaSuccess) return e;
+    if (need <= fit) {
+        k_vturb<T, NPMAX, true><<<(unsigned)fit, 32, smem, s>>>(A, turbv);
+    } else {
+        const int64_t blocks = grid_for(k_vturb<T, NPMAX, false>, 32, 0, A.p.n, num_sms, &e, cap);
+        if (e != cudaSuccess) return e;
+        k_vturb<T, NPMAX, false><<<(unsigned)blocks, 32, 0, s>>>(A, turbv);
+    }
+    return cudaGetLastError();
+}
+
+template <typename T>
+static cudaError_t launch_step_t(const RpStepArgs& A, int np, double* turbv, cudaStream_t s, int num_sms,
                                  int* nlaunch) {
     cudaError_t e = cudaSuccess;
-    if (variant == 1) {
-        const int64_t blocks = grid_for(k_step_fused<T, NPMAX>, kStepBlock, 0, A.p.n, num_sms, &e, A.grid_cap);
-        if (e != cudaSuccess) return e;
-        k_step_fused<T, NPMAX><<<(unsigned)blocks, kStepBlock, 0, s>>>(A);
-        *nlaunch += 1;
-        return cudaGetLastError();
-    }
     if (A.vturb_on) {
-        const int64_t blocks = grid_for(k_vturb_local<T, NPMAX>, kStepBlock, 0, A.p.n, num_sms, &e, A.grid_cap);
-        if (e != cudaSuccess) return e;
-        k_vturb_local<T, NPMAX><<<(unsigned)blocks, kStepBlock, 0, s>>>(A, turbv);
+        if (np <= 88) e = launch_vturb<T, 88>(A, np, turbv, s, num_sms);
+        else if (np <= 128) e = launch_vturb<T, 128>(A, np, turbv, s, num_sms);
+        else e = launch_vturb<T, kMaxNp>(A, np, turbv, s, num_sms);
         *nlaunch += 1;
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        if (e != cudaSuccess) return e;
     }
     const int64_t blocks = grid_for(k_advect<T>, kStepBlock, 0, A.p.n, num_sms, &e, A.grid_cap);
     if (e != cudaSuccess) return e;
-    k_advect<T><<<(unsigned)blocks, kStepBlock, 0, s>>>(A, A.vturb_on ? turbv : nullptr);
+    k_advect<T><<<(unsigned)blocks, kStepBlock, 0, s>>>(A, turbv);
     *nlaunch += 1;
     return cudaGetLastError();
 }
 
-cudaError_t launch_step(const RpStepArgs& A, int field_dtype, int npmax, double* turbv, int variant,
-                        cudaStream_t s, int num_sms, int* nlaunch) {
-    if (field_dtype == 1) {
-        if (npmax <= 88) return launch_step_t<float, 88>(A, turbv, variant, s, num_sms, nlaunch);
-        if (npmax <= 128) return launch_step_t<float, 128>(A, turbv, variant, s, num_sms, nlaunch);
-        return launch_step_t<float, 144>(A, turbv, variant, s, num_sms, nlaunch);
-    }
-    if (npmax <= 88) return launch_step_t<double, 88>(A, turbv, variant, s, num_sms, nlaunch);
-    if (npmax <= 128) return launch_step_t<double, 128>(A, turbv, variant, s, num_sms, nlaunch);
-    return launch_step_t<double, 144>(A, turbv, variant, s, num_sms, nlaunch);
+cudaError_t launch_step(const RpStepArgs& A, int field_dtype, int np, double* turbv, cudaStream_t s, int num_sms,
+                        int* nlaunch) {
+    return field_dtype == 1 ? launch_step_t<float>(A, np, turbv, s, num_sms, nlaunch)
+                            : launch_step_t<double>(A, np, turbv, s, num_sms, nlaunch);
 }
 
 // -------------------------------------------- initial ownership (init)

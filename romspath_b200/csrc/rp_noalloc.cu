@@ -64,7 +64,7 @@ cudaError_t scratch_for_device(int device, double** out) {
 template <typename T, int NPMAX>
 __global__ void __launch_bounds__(32, 1) k_vturb_na(const __grid_constant__ RpStepArgs A, double* __restrict__ turbv) {
     extern __shared__ double sm[];
-    const SplineView<NPMAX, 32> w{sm + threadIdx.x};
+    const SplineShared<NPMAX> w{sm + threadIdx.x};
     const int64_t stride = (int64_t)gridDim.x * 32;
     for (int64_t n = (int64_t)blockIdx.x * 32 + threadIdx.x; n < A.p.n; n += stride)
         rp_vturb_one<T>(A, n, w, turbv);
@@ -73,17 +73,16 @@ __global__ void __launch_bounds__(32, 1) k_vturb_na(const __grid_constant__ RpSt
 template <typename T>
 __global__ void __launch_bounds__(kStepBlock) k_advect_na(const __grid_constant__ RpStepArgs A,
                                                          const double* __restrict__ turbv) {
-    const SplineView<1, 1> none{nullptr};
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < A.p.n; n += stride)
-        rp_update_one<T>(A, n, none, turbv);
+        rp_update_one<T>(A, n, turbv);
 }
 
 template <typename T, int NPMAX>
 static cudaError_t launch_na(const RpStepArgs& A, double* scratch, cudaStream_t s, int num_sms, int* nlaunch) {
     cudaError_t e = cudaSuccess;
     if (A.vturb_on) {
-        const size_t smem = (size_t)kSplineArrays * (NPMAX + 1) * 32 * sizeof(double);
+        const size_t smem = SplineShared<NPMAX>::kBytes;
         e = cudaFuncSetAttribute(k_vturb_na<T, NPMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         int occ = 0;

@@ -21,6 +21,29 @@ __device__ __forceinline__ double rp_normal(const RpStepArgs& A, uint32_t pid, u
     return sqrt(-2.0 * rp_log_pos(u1)) * rp_cos2pi(u2);
 }
 
+// Normal deviates d and d+1 (d even) by one Philox call; d+1 only with
+// `both` (the hook holds no more than the step's draws).
+__device__ __forceinline__ void rp_normal2(const RpStepArgs& A, uint32_t pid, uint32_t d, bool both, double& n0,
+                                           double& n1) {
+    n1 = 0.0;
+    if (A.hook) {
+        const double* h = A.hook + (int64_t)(pid - A.pid_base) * A.ndraw + d;
+        n0 = h[0];
+        if (both) n1 = h[1];
+        return;
+    }
+    uint32_t c[4] = {pid, (uint32_t)A.step_index, (uint32_t)(A.step_index >> 32), d >> 1};
+    rp_philox(c, (uint32_t)A.seed, (uint32_t)(A.seed >> 32));
+    const double u1 = ((double)c[0] + 0.5) / 4294967296.0;
+    const double u2 = ((double)c[1] + 0.5) / 4294967296.0;
+    n0 = sqrt(-2.0 * rp_log_pos(u1)) * rp_cos2pi(u2);
+    if (both) {
+        const double u3 = ((double)c[2] + 0.5) / 4294967296.0;
+        const double u4 = ((double)c[3] + 0.5) / 4294967296.0;
+        n1 = sqrt(-2.0 * rp_log_pos(u3)) * rp_cos2pi(u4);
+    }
+}
+
 // Uniform k (0..4) of behave's draws: the hook's entry d0 + 2 + k (d0 =
 // 2 + idt/deltat, after the HTurb and VTurb normals and behave's two), else
 // Philox4x32-10 at counter (pid, step, 0x40000000 + k/4), word k%4.
@@ -94,8 +117,7 @@ __device__ __forceinline__ void rp_find_currents(const RpStepArgs& A, const RpGr
     if (Z > S.zeta) Z = S.zeta - RP_F_0P001;
 
     LevelPick Lr, Lw;
-    rp_walk_rho(g, S.zeta, S.tdepth, Z, Lr);
-    rp_walk_w(g, S.zeta, S.tdepth, Z, Lw, fl);
+    rp_walk2(g, S.zeta, S.tdepth, Z, Lr, Lw, fl);
     if (A.wetdry) {
         rp_gather_wd<T>(A, g, X, Y, Lr, Lw, S.rc, Uad, Vad, Wad, fl);
         return;
@@ -139,244 +161,450 @@ __device__ __forceinline__ void rp_find_currents(const RpStepArgs& A, const RpGr
 }
 
 // ----------------------------------------------------------- spline
+//
+// The smoothing-spline fit of one particle.  Its arrays (1-based element i):
+//   fitz  the breaks             y    the resampled data fitKH
+//   qty   Q'y                    r12  the factor's two ratios v(i,2), v(i,3)
+//   u     u(i)/v(i,1), then u(i)
+// The column's lines (slope, intercept) sit in r12 and its levels z(k) in u
+// until the fit overwrites them.
 
-// Workspace of one particle's smoothing-spline fit: six arrays of
-// (NPMAX+1) doubles with 1-based element i of array a at
-// base[(a*(NPMAX+1) + i) * S].  S = 1 for a private array, S = 32 for a
-// warp's lane-interleaved shared-memory block (bank-conflict free).
-constexpr int kSplineArrays = 6;
-
-template <int NPMAX, int S>
-struct SplineView {
-    double* base;
-    __device__ __forceinline__ double& at(int a, int i) const { return base[(a * (NPMAX + 1) + i) * S]; }
-    __device__ __forceinline__ double& fitz(int i) const { return at(0, i); }  // breaks fitz(1..np)
-    __device__ __forceinline__ double& y(int i) const { return at(1, i); }     // fitKH(1..np)
-    __device__ __forceinline__ double& qty(int i) const { return at(2, i); }   // Q'y
-    __device__ __forceinline__ double& r1(int i) const { return at(3, i); }    // v(i,2) after factorisation
-    __device__ __forceinline__ double& r2(int i) const { return at(4, i); }    // v(i,3) after factorisation
-    __device__ __forceinline__ double& u(int i) const { return at(5, i); }     // u(i)/v(i,1), then u(i)
+// A warp's fits in a private array each; SU: u in the warp's shared memory
+// instead (element i of lane l at su[(i - 1) * 32 + l]: no bank conflicts).
+template <int NPMAX, bool SU>
+struct SplineLocal {
+    static constexpr int kDoubles = (SU ? 5 : 6) * (NPMAX + 2);
+    double* base;                  // kDoubles doubles, 16-byte aligned
+    double* su;
+    __device__ __forceinline__ double2* rr() const { return reinterpret_cast<double2*>(base); }
+    __device__ __forceinline__ double2 r12(int i) const { return rr()[i]; }
+    __device__ __forceinline__ void set_r12(int i, double a, double b) const { rr()[i] = make_double2(a, b); }
+    __device__ __forceinline__ double& fitz(int i) const { return base[2 * (NPMAX + 2) + i]; }
+    __device__ __forceinline__ double& y(int i) const { return base[3 * (NPMAX + 2) + i]; }
+    __device__ __forceinline__ double& qty(int i) const { return base[4 * (NPMAX + 2) + i]; }
+    __device__ __forceinline__ double& u(int i) const { return SU ? su[(i - 1) * 32] : base[5 * (NPMAX + 2) + i]; }
 };
 
-// The breaks fitz(1..np) as VTurb's resampling forms them
-// (ver_turb_module.f90:126-136): fitz(1) = z1, fitz(k) = fitz(k-1) + dz for
-// k = 2..np-1, fitz(np) = zend.  The chol1d passes re-form them by the same
-// additions, ascending, instead of reading them back from the workspace.
-struct RpBreaks {
-    double z1, dz, zend;
+// The same with every array in a warp's shared memory (element i of array a
+// of lane l at sm[(a * (NPMAX + 1) + i) * 32 + l]).
+template <int NPMAX>
+struct SplineShared {
+    static constexpr size_t kBytes = (size_t)(NPMAX + 1) * 32 * 6 * sizeof(double);
+    double* sm;                    // this lane's first element
+    __device__ __forceinline__ double& at(int a, int i) const { return sm[(a * (NPMAX + 1) + i) * 32]; }
+    __device__ __forceinline__ double2 r12(int i) const { return make_double2(at(0, i), at(1, i)); }
+    __device__ __forceinline__ void set_r12(int i, double a, double b) const { at(0, i) = a; at(1, i) = b; }
+    __device__ __forceinline__ double& fitz(int i) const { return at(2, i); }
+    __device__ __forceinline__ double& y(int i) const { return at(3, i); }
+    __device__ __forceinline__ double& qty(int i) const { return at(4, i); }
+    __device__ __forceinline__ double& u(int i) const { return at(5, i); }
 };
 
-// chol1d (pppack.f90:1428-1566) for p.  The setupq bands are rebuilt on the
-// fly: with all data weights dy(i) = serr, v(i,1) = r(i-1),
-// v(i,2) = -r(i) - r(i-1), v(i,3) = r(i) where r(k) = serr / v(k,4) and
-// v(k,4) = fitz(k+1) - fitz(k), each formed by the same operation as in
-// setupq.  Factorisation and forward substitution run in one ascending
-// sweep that stores v(i,2), v(i,3) and u(i)/v(i,1); back substitution runs
-// descending; then Q u and sum_i qu(i)^2 dy(i)^2 are formed ascending (the
-// reference's summation order), with utru (pppack.f90:5219-5223) on request.
-template <class W>
-__device__ __forceinline__ double rp_chol1d(const W& w, int np, const RpBreaks& B, double p, double serr,
-                                            double dy2, double* utru_out) {
-    const double six1mp = 6.0 * (1.0 - p);
-    const double twop = 2.0 * p;
-    double acc = B.z1;                           // the running sum of the breaks
-    auto brk = [&](int k) -> double {            // fitz(k), k = 2, 3, ... in turn
-        acc = acc + B.dz;
-        return (k == np) ? B.zend : acc;
-    };
-    const double f2 = brk(2), f3 = brk(3), f4 = brk(4);
-    double v4a = f2 - B.z1;                      // v4(1)
-    double v4b = f3 - f2;                        // v4(2)
-    double v4c = f4 - f3;                        // v4(3)
-    double fprev = f4;                           // fitz(i+2)
-    const double r1_ = serr / v4a;               // r(1)
-    double ri = serr / v4b;                      // r(i),   i = 2
-    double rn = serr / v4c;                      // r(i+1)
-    double v4n = v4c;                            // v4(i+1)
-    double a1, a2, b1;
-    {
-        const double v2s2 = -ri - r1_;
-        const double v2s3 = -rn - ri;
-        const double v5_2 = r1_ * r1_ + v2s2 * v2s2 + ri * ri;
-        a1 = six1mp * v5_2 + twop * (v4a + v4b);                         // V1(2)
-        const double v6_2 = (2 <= np - 2) ? (v2s2 * ri + ri * v2s3) : 0.0;
-        a2 = six1mp * v6_2 + p * v4b;                                     // V2(2)
-        const double v5_3 = ri * ri + v2s3 * v2s3 + rn * rn;
-        b1 = six1mp * v5_3 + twop * (v4b + v4c);                         // V1(3)
+// What a fit's passes share.  The breaks are fitz(1) = z1, fitz(k) =
+// fitz(k-1) + dz, fitz(np) = zend (ver_turb_module.f90:126-136); the passes
+// re-form them by the same additions.  fitz(k-1) + dz rounds the same way
+// while |fitz| stays in one binade, so v4(k) = fitz(k+1) - fitz(k) changes
+// its value a handful of times down a column (4 on average at 124 points),
+// and what is formed from v4 alone is formed again only there: at the rows
+// flagged in chg, which holds the changes of every lane of the warp, so that
+// the lanes take either path together (a lane whose v4 does not change forms
+// the same values again).
+constexpr int kChgWords = 5;       // 160 bits >= kMaxNp + 1 (rp_internal.h)
+struct RpFit {
+    int np;
+    bool mono;                     // the breaks ascend: ppvalu may guess its piece
+    double z1, dz, zend, rdz;      // rdz: about 1 / dz
+    double f4;                     // fitz(4)
+    double v1, v2, v3;             // v4(1..3)
+    double r1, r2, r3;             // serr / v4(1..3)
+    double y1;                     // 1 / v4(1), correctly rounded
+    double serr, dy2;
+    uint32_t chg[kChgWords];       // bit k: v4(k) != v4(k-1) in some lane, k >= 2
+    // V1(2), V2(2), V1(3) of setupq's matrix
+    __device__ __forceinline__ void first_rows(double p, double& a1, double& a2, double& b1) const {
+        const double six1mp = 6.0 * (1.0 - p), twop = 2.0 * p;
+        const double v2s2 = -r2 - r1, v2s3 = -r3 - r2;
+        a1 = six1mp * (r1 * r1 + v2s2 * v2s2 + r2 * r2) + twop * (v1 + v2);
+        a2 = six1mp * (v2s2 * r2 + r2 * v2s3) + p * v2;
+        b1 = six1mp * (r2 * r2 + v2s3 * v2s3 + r3 * r3) + twop * (v2 + v3);
     }
-    double uprev = 0.0, ucur = w.qty(2), r2prev = 0.0;
-    w.u(1) = 0.0;
-    // The sweeps are written without branches on the element index (values
-    // past the ends are formed from clamped in-range loads and discarded by
-    // the selects), so that unrolled iterations issue their independent
-    // workspace loads together.
-#pragma unroll 4
-    for (int i = 2; i <= np - 2; i++) {
-        // r(i+2), v4(i+2) (used while i+2 <= np-1)
-        const bool has2 = (i + 2 <= np - 1);
-        double v4nn = v4n;                        // past the end: discarded by the selects
-        if (has2) {
-            const double f = brk(i + 3);
-            v4nn = f - fprev;
-            fprev = f;
+    // bits i .. i + 31 of chg
+    __device__ __forceinline__ uint32_t bits(int i) const {
+        const int w = i >> 5;
+        uint32_t lo = 0, hi = 0;
+#pragma unroll
+        for (int q = 0; q < kChgWords; q++) {
+            lo = (q == w) ? chg[q] : lo;
+            hi = (q == w + 1) ? chg[q] : hi;
         }
-        const double rnn = serr / v4nn;
-        const double qn = w.qty(i + 1);
-        const double V3i = six1mp * ((i <= np - 3) ? (ri * rn) : 0.0);
-        const double ratio1 = a2 / a1;
-        b1 = b1 - ratio1 * a2;
-        const double v2sn = -rn - ri;             // v(i+1,2) of setupq
-        const double v2snn = -rnn - rn;           // v(i+2,2)
-        const double v6n = (i + 1 <= np - 2) ? (v2sn * rn + rn * v2snn) : 0.0;
-        const double c2 = (six1mp * v6n + p * v4n) - ratio1 * V3i;
-        const double ratio2 = V3i / a1;
-        const double v5nn = rn * rn + v2snn * v2snn + rnn * rnn;
-        const double c1 = has2 ? ((six1mp * v5nn + twop * (v4n + v4nn)) - ratio2 * V3i) : 0.0;
-        w.r1(i) = ratio1;
-        w.r2(i) = ratio2;
-        w.u(i) = ucur / a1;                       // u(i)/v(i,1)
-        const double unext = qn - ratio1 * ucur - r2prev * uprev;
+        return __funnelshift_r(lo, hi, i & 31);
+    }
+};
+
+// The pass below with every division left to the IEEE operator, for fits
+// whose operands leave the shared-reciprocal division's range (NaN frames,
+// subnormal diffusivities).
+template <class W>
+__device__ __noinline__ double rp_chol1d_ieee(const W w, const RpFit& F, double p) {
+    const int np = F.np;
+    const double six1mp = 6.0 * (1.0 - p), twop = 2.0 * p;
+    double ri = F.r2, rn = F.r3, v4n = F.v3;
+    double a1, a2, b1;
+    F.first_rows(p, a1, a2, b1);
+    double uprev = 0.0, ucur = w.qty(2), r2prev = 0.0;
+    for (int i = 2; i <= np - 2; i++) {
+        const bool in = i <= np - 3;             // rows with a third band
+        const double v4nn = in ? w.fitz(i + 3) - w.fitz(i + 2) : 0.0;
+        const double rnn = in ? F.serr / v4nn : 0.0;
+        const double V3 = six1mp * (in ? ri * rn : 0.0);
+        const double v2sn = -rn - ri, v2snn = -rnn - rn;
+        const double ratio1 = a2 / a1, ratio2 = V3 / a1;
+        w.set_r12(i, ratio1, ratio2);
+        w.u(i) = ucur / a1;
+        const double a1n = b1 - ratio1 * a2;
+        a2 = (six1mp * (v2sn * rn + rn * v2snn) + p * v4n) - ratio1 * V3;
+        b1 = (six1mp * (rn * rn + v2snn * v2snn + rnn * rnn) + twop * (v4n + v4nn)) - ratio2 * V3;
+        a1 = a1n;
+        const double unext = w.qty(i + 1) - ratio1 * ucur - r2prev * uprev;
         uprev = ucur;
         ucur = unext;
         r2prev = ratio2;
-        a1 = b1;
-        a2 = c2;
-        b1 = c1;
         ri = rn;
         rn = rnn;
         v4n = v4nn;
     }
-    // back substitution
-    const double unm1 = ucur / a1;                // u(np-1)/v(np-1,1)
-    w.u(np - 1) = unm1;
-    w.u(np) = 0.0;
-    double up2 = 0.0, up1 = unm1;
-#pragma unroll 4
+    double up2 = 0.0, up1 = ucur / a1;
+    w.u(np - 1) = up1;
     for (int i = np - 2; i >= 2; i--) {
-        const double qi = w.u(i), s1 = w.r1(i), s2 = w.r2(i);
-        const double ui = qi - up1 * s1 - up2 * s2;
+        const double2 r = w.r12(i);
+        const double ui = w.u(i) - up1 * r.x - up2 * r.y;
         w.u(i) = ui;
         up2 = up1;
         up1 = ui;
     }
-    // qu = Q u and the weighted sum of squares, i = 1..np in order
-    double prev = 0.0, sum = 0.0, utru = 0.0;
-    double ulast = 0.0;                           // u(1)
-    double flast = B.z1;
-    acc = B.z1;
-#pragma unroll 4
+    double prev = 0.0, sum = 0.0, ulast = 0.0;
     for (int i = 2; i <= np; i++) {
-        const double ui = w.u(i);
-        const double fi = brk(i);
-        const double v4i = fi - flast;
-        const double raw = (ui - ulast) / v4i;
+        const double ui = (i < np) ? w.u(i) : 0.0;
+        const double raw = (ui - ulast) / (w.fitz(i) - w.fitz(i - 1));
         const double fin = raw - prev;
-        sum = sum + (fin * fin) * dy2;
-        if (utru_out) utru = utru + v4i * (ulast * (ulast + ui) + ui * ui);
+        sum = sum + (fin * fin) * F.dy2;
         prev = raw;
         ulast = ui;
-        flast = fi;
+    }
+    return sum + (-prev * -prev) * F.dy2;
+}
+
+// chol1d (pppack.f90:1428-1566) for p.  With all data weights dy(i) = serr
+// setupq's bands are v(i,1) = r(i-1), v(i,2) = -r(i) - r(i-1), v(i,3) = r(i);
+// the band values of a row (V1, V2, V3 below) are formed by setupq's own
+// operations.  Factorisation and forward substitution run in one ascending
+// sweep that keeps v(i,2), v(i,3) and u(i)/v(i,1); back substitution runs
+// descending; then Q u and sum_i qu(i)^2 dy(i)^2 are formed ascending (the
+// reference's summation order).
+//
+// A row is one chain of dependent FP64 operations (pivot, reciprocal,
+// quotient, next pivot: about 95 cycles at 8 a step on B200), so the rows
+// hold no branch: the quotients share the pivot's reciprocal and are formed
+// whether their operands are in range or not, and the pass is made again by
+// the IEEE operator when one was not (with a test and a cold branch in each
+// row a row took 320 cycles alone, without 190).  What the rows read from
+// memory is loaded a group of rows ahead.
+template <class W>
+__device__ __forceinline__ double rp_chol1d(const W& w, const RpFit& F, double p) {
+    const int np = F.np;
+    const double six1mp = 6.0 * (1.0 - p);
+    const double twop = 2.0 * p;
+    double ri = F.r2;                            // r(i),   i = 2
+    double rn = F.r3;                            // r(i+1)
+    double v4n = F.v3;                           // v4(i+1)
+    double a1, a2, b1;
+    F.first_rows(p, a1, a2, b1);
+    double uprev = 0.0, ucur = w.qty(2), r2prev = 0.0;
+    double acc = F.f4;                           // the running sum of the breaks, fitz(i+2)
+    double V3 = 0.0, V2n = 0.0, V1nn = 0.0;      // V3(i), V2(i+1), V1(i+2)
+    uint32_t off = 0;                            // largest exponent distance of an operand
+    uint32_t ones = 0;                           // all bits: a significand of all ones
+    // the band values of row i, whose v4(i), v4(i+1) or v4(i+2) may be new
+    auto bands = [&](int i) {
+        const double f = (i + 3 == np) ? F.zend : acc + F.dz;
+        const double v4nn = f - acc;             // v4(i+2)
+        const double rnn = rp_div_rcp(F.serr, v4nn, rp_rcp3(v4nn));
+        off = max(off, rp_exp_off(v4nn));
+        ones = max(ones, rp_ones(v4nn));
+        V3 = six1mp * (ri * rn);
+        const double v2sn = -rn - ri;            // v(i+1,2) of setupq
+        const double v2snn = -rnn - rn;          // v(i+2,2)
+        V2n = six1mp * (v2sn * rn + rn * v2snn) + p * v4n;
+        V1nn = six1mp * (rn * rn + v2snn * v2snn + rnn * rnn) + twop * (v4n + v4nn);
+        ri = rn;
+        rn = rnn;
+        v4n = v4nn;
+    };
+    auto row = [&](int i, double qn) {
+        acc = acc + F.dz;
+        off = max(max(off, rp_exp_off(a1)), max(rp_exp_off(a2), rp_exp_off_z(ucur)));
+        ones = max(ones, rp_ones(a1));
+        const RpRcp y = rp_rcp3(a1);
+        const double ratio1 = rp_div_rcp(a2, a1, y);
+        const double ratio2 = rp_div_rcp(V3, a1, y);
+        w.u(i) = rp_div_rcp(ucur, a1, y);        // u(i)/v(i,1)
+        w.set_r12(i, ratio1, ratio2);
+        const double a1n = b1 - ratio1 * a2;
+        a2 = V2n - ratio1 * V3;
+        b1 = V1nn - ratio2 * V3;
+        a1 = a1n;
+        const double unext = qn - ratio1 * ucur - r2prev * uprev;
+        uprev = ucur;
+        ucur = unext;
+        r2prev = ratio2;
+    };
+    constexpr int G = 4;
+    double q[G];
+#pragma unroll
+    for (int k = 0; k < G; k++) q[k] = w.qty(min(3 + k, np - 1));
+    int i = 2;
+    for (; i + G - 1 <= np - 3; i += G) {
+        double qx[G];
+#pragma unroll
+        for (int k = 0; k < G; k++) qx[k] = w.qty(min(i + 1 + G + k, np - 1));
+        // a change of v4 at k concerns rows k-2 .. k
+        if (i == 2 || (F.bits(i) & ((1u << (G + 2)) - 1u))) {
+#pragma unroll
+            for (int k = 0; k < G; k++) {
+                bands(i + k);
+                row(i + k, q[k]);
+            }
+            off = max(off, rp_exp_off(V3));
+        } else {
+#pragma unroll
+            for (int k = 0; k < G; k++) row(i + k, q[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < G; k++) q[k] = qx[k];
+    }
+    for (; i <= np - 3; i++) {
+        bands(i);
+        row(i, w.qty(i + 1));
+    }
+    off = max(off, rp_exp_off(V3));
+    {                                             // row np-2: V3 = six1mp * 0
+        const double ratio1 = a2 / a1;
+        w.set_r12(np - 2, ratio1, (six1mp * 0.0) / a1);
+        w.u(np - 2) = ucur / a1;
+        a1 = b1 - ratio1 * a2;
+        ucur = w.qty(np - 1) - ratio1 * ucur - r2prev * uprev;
+    }
+    // back substitution, the ratios read a group of rows ahead
+    double up2 = 0.0, up1 = ucur / a1;            // u(np-1)/v(np-1,1)
+    w.u(np - 1) = up1;
+    constexpr int B = 8;
+    double2 sa[B], sb[B];
+    auto load = [&](double2(&t)[B], int j) {
+#pragma unroll
+        for (int k = 0; k < B; k++) t[k] = w.r12(max(j - k, 2));
+    };
+    auto solve = [&](const double2(&t)[B], int j) {
+#pragma unroll
+        for (int k = 0; k < B; k++) {
+            const double ui = w.u(j - k) - up1 * t[k].x - up2 * t[k].y;
+            w.u(j - k) = ui;
+            up2 = up1;
+            up1 = ui;
+        }
+    };
+    int j = np - 2;
+    load(sa, j);
+    for (; j - 2 * B + 1 >= 2; j -= 2 * B) {
+        load(sb, j - B);
+        solve(sa, j);
+        load(sa, j - 2 * B);
+        solve(sb, j - B);
+    }
+    for (; j >= 2; j--) {
+        const double2 t = w.r12(j);
+        const double ui = w.u(j) - up1 * t.x - up2 * t.y;
+        w.u(j) = ui;
+        up2 = up1;
+        up1 = ui;
+    }
+    // qu = Q u and the weighted sum of squares, i = 1..np in order
+    // (u(1) = u(np) = 0)
+    double prev = 0.0, sum = 0.0, ulast = 0.0;
+    double v4 = F.v1, yv = F.y1;
+    acc = F.z1;                                   // fitz(i-1)
+    off = max(off, rp_exp_off(v4));
+    constexpr int R = 8;                          // rows whose quotients are formed side by side
+    for (i = 2; i + R - 1 < np; i += R) {
+        double us[R + 1], du[R], raw[R];
+        us[0] = ulast;
+#pragma unroll
+        for (int k = 0; k < R; k++) {
+            us[k + 1] = w.u(i + k);
+            du[k] = us[k + 1] - us[k];
+            off = max(off, rp_exp_off_z(du[k]));
+        }
+        ulast = us[R];
+        if (F.bits(i - 1) & ((1u << R) - 1u)) {
+#pragma unroll
+            for (int k = 0; k < R; k++) {
+                const double f = acc + F.dz;
+                v4 = f - acc;                     // v4(i+k-1)
+                acc = f;
+                const RpRcp y = rp_rcp3(v4);
+                yv = y.y;
+                off = max(off, rp_exp_off(v4));
+                ones = max(ones, rp_ones(v4));
+                raw[k] = rp_div_rcp(du[k], v4, y);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < R; k++) {
+                raw[k] = rp_div_fast(du[k], v4, yv, yv);
+                acc = acc + F.dz;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < R; k++) {
+            const double fin = raw[k] - prev;
+            sum = sum + (fin * fin) * F.dy2;
+            prev = raw[k];
+        }
+    }
+    for (; i <= np; i++) {
+        const double ui = (i < np) ? w.u(i) : 0.0;
+        const double f = (i == np) ? F.zend : acc + F.dz;
+        const double raw = rp_quot(ui - ulast, f - acc);
+        acc = f;
+        ulast = ui;
+        const double fin = raw - prev;
+        sum = sum + (fin * fin) * F.dy2;
+        prev = raw;
     }
     const double finn = -prev;
-    sum = sum + (finn * finn) * dy2;
-    if (utru_out) *utru_out = utru;
+    sum = sum + (finn * finn) * F.dy2;
+    if (off >= kDivSpan || ones == 0xffffffffu) sum = rp_chol1d_ieee(w, F, p);
     return sum;
 }
 
-// smooth (pppack.f90:5108-5317) on fitz/y already in w; dy(i) = serr for
-// all i.  Returns p; w.u holds the final u; passes = chol1d passes made.
+// utru (pppack.f90:5219-5223) of the pass just made
 template <class W>
-__device__ __forceinline__ double rp_smooth(const W& w, int np, const RpBreaks& B, double serr, double s,
-                                            int max_iter, uint32_t& fl, int& passes) {
-    const double dy2 = serr * serr;
-    // setupq's Q'y (pppack.f90:4816-4822)
-    {
-        double prev = (w.y(2) - w.y(1)) / (w.fitz(2) - w.fitz(1));
-        for (int i = 2; i <= np - 1; i++) {
-            const double diff = (w.y(i + 1) - w.y(i)) / (w.fitz(i + 1) - w.fitz(i));
-            w.qty(i) = diff - prev;
-            prev = diff;
-        }
+__device__ __forceinline__ double rp_utru(const W& w, const RpFit& F) {
+    double utru = 0.0, ulast = 0.0, acc = F.z1;
+    for (int i = 2; i <= F.np; i++) {
+        const double ui = (i < F.np) ? w.u(i) : 0.0;
+        const double f = (i == F.np) ? F.zend : acc + F.dz;
+        utru = utru + (f - acc) * (ulast * (ulast + ui) + ui * ui);
+        acc = f;
+        ulast = ui;
     }
-    double p, q, sfq;
-    passes = 1;
-    if (s <= 0.0) {
-        p = 1.0;
-        rp_chol1d(w, np, B, p, serr, dy2, nullptr);
-    } else {
-        p = 0.0;
-        double utru = 0.0;
-        sfq = 36.0 * rp_chol1d(w, np, B, p, serr, dy2, &utru);
-        if (s < sfq) {
-            const double ooss = 1.0 / sqrt(s);
-            double oosf = 1.0 / sqrt(sfq);
-            q = -(oosf - ooss) * sfq / (6.0 * utru * oosf);
-            double prevq = 0.0, prevsf = oosf;
-            int it = 0;
-            for (;;) {
-                const double sum = rp_chol1d(w, np, B, q / (1.0 + q), serr, dy2, nullptr);
-                sfq = 36.0 * sum / ((1.0 + q) * (1.0 + q));
-                it++;
-                passes++;
-                if (fabs(sfq - s) <= 0.01 * s) break;
-                if (it >= max_iter) { fl |= RP_FL_SPLINE; break; }
-                oosf = 1.0 / sqrt(sfq);
-                const double change = (q - prevq) / (oosf - prevsf) * (oosf - ooss);
-                prevq = q;
-                q = q - change;
-                prevsf = oosf;
-            }
-            p = q / (1.0 + q);
+    return utru;
+}
+
+// smooth (pppack.f90:5108-5317) on the fit's Q'y; dy(i) = serr for all i.
+// Returns p; w.u holds the final u; passes = chol1d passes made.
+template <class W>
+__device__ __forceinline__ double rp_smooth(const W& w, const RpFit& F, double s, int max_iter, uint32_t& fl,
+                                            int& passes) {
+    // one call site of chol1d: the passes of p = 1 (s <= 0), p = 0 and the
+    // secant search follow one another in the same loop
+    const double ooss = 1.0 / sqrt(s);
+    double p = (s <= 0.0) ? 1.0 : 0.0;
+    double q = 0.0, prevq = 0.0, prevsf = 0.0;
+    passes = 0;
+    for (int it = 0;; it++) {
+        const double sum = rp_chol1d(w, F, p);
+        passes++;
+        if (s <= 0.0) break;
+        if (it == 0) {
+            const double sfq = 36.0 * sum;
+            if (!(s < sfq)) break;
+            const double oosf = 1.0 / sqrt(sfq);
+            q = -(oosf - ooss) * sfq / (6.0 * rp_utru(w, F) * oosf);
+            prevsf = oosf;
+        } else {
+            const double sfq = 36.0 * sum / ((1.0 + q) * (1.0 + q));
+            if (fabs(sfq - s) <= 0.01 * s) break;
+            if (it >= max_iter) { fl |= RP_FL_SPLINE; break; }
+            const double oosf = 1.0 / sqrt(sfq);
+            const double change = (q - prevq) / (oosf - prevsf) * (oosf - ooss);
+            prevq = q;
+            q = q - change;
+            prevsf = oosf;
         }
+        p = q / (1.0 + q);
     }
     return p;
 }
 
-// ppvalu (pppack.f90:4246-4362) of the smoothing spline at x, with the
-// coefficients of the one piece it needs formed from u and y exactly as
-// smooth's epilogue forms a(:,1..4) (pppack.f90:5303-5316).
+// One piece of the fit: its breaks and the coefficients a(i,1..4) that
+// smooth's epilogue forms (pppack.f90:5303-5316), kept between the sub-steps
+// (consecutive positions mostly share their piece).
+struct RpPiece {
+    double x0, x1;                 // fitz(i), fitz(i+1); x0 > x1: none yet
+    double a1, a2, a3, a4;
+};
+
+// interv (pppack.f90:3363-3576): the largest i <= np-1 with fitz(i) <= x,
+// 1 below the first break (and for a NaN x)
 template <class W>
-__device__ __forceinline__ double rp_ppvalu(const W& w, int np, double p, double serr, double x, int jderiv) {
-    // interv (pppack.f90:3363-3576) for strictly increasing breaks
-    int i;
-    if (!(x >= w.fitz(1))) {
-        i = 1;
-    } else {
-        int lo = 1, hi = np;   // fitz(lo) <= x; answer in [lo, hi-1]
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (w.fitz(mid) <= x) lo = mid; else hi = mid;
-        }
-        i = lo;
+__device__ __forceinline__ int rp_interv(const W& w, const RpFit& F, double x) {
+    const int np = F.np;
+    if (!(x >= w.fitz(1))) return 1;
+    if (F.mono) {                  // ascending breaks: from the uniform guess to the piece
+        const double t = (x - F.z1) * F.rdz;
+        int i = (t < (double)(np - 2)) ? (int)t + 1 : np - 1;
+        while (i > 1 && w.fitz(i) > x) i--;
+        while (i < np - 1 && w.fitz(i + 1) <= x) i++;
+        return i;
     }
-    const double dy2 = serr * serr;
-    const double K1 = 6.0 * (1.0 - p) * dy2;
-    auto v4 = [&](int k) -> double { return w.fitz(k + 1) - w.fitz(k); };
-    auto raw = [&](int k) -> double { return (w.u(k) - w.u(k - 1)) / v4(k - 1); };  // k >= 2
-    auto fin = [&](int k) -> double {
-        if (k == 1) return raw(2) - 0.0;
-        if (k == np) return -raw(np);
-        return raw(k + 1) - raw(k);
-    };
-    const double a1i = w.y(i) - K1 * fin(i);
-    const double a1n = w.y(i + 1) - K1 * fin(i + 1);
-    const double a3i = w.u(i) * 6.0 * p;
-    const double a3n = w.u(i + 1) * 6.0 * p;
-    const double h4 = v4(i);
-    const double a4i = (a3n - a3i) / h4;
-    const double a2i = (a1n - a1i) / h4 - (a3i + a4i / 3.0 * h4) / 2.0 * h4;
+    int lo = 1, hi = np;           // fitz(lo) <= x; answer in [lo, hi-1]
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (w.fitz(mid) <= x) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+
+// ppvalu (pppack.f90:4246-4362) of the smoothing spline at x
+template <class W>
+__device__ __forceinline__ double rp_ppvalu(const W& w, const RpFit& F, double p, double x, int jderiv, RpPiece& pc) {
+    if (!(x >= pc.x0 && x < pc.x1)) {
+        const int np = F.np;
+        const int i = rp_interv(w, F, x);
+        const double K1 = 6.0 * (1.0 - p) * F.dy2;
+        auto uu = [&](int k) -> double { return (k <= 1 || k >= np) ? 0.0 : w.u(k); };
+        const double fm = w.fitz(max(i - 1, 1)), f0 = w.fitz(i), f1 = w.fitz(i + 1), f2 = w.fitz(min(i + 2, np));
+        const double um = uu(i - 1), u0 = uu(i), u1 = uu(i + 1), u2 = uu(i + 2);
+        const double y0 = w.y(i), y1 = w.y(i + 1);
+        const double h4 = f1 - f0;
+        const double yh = rp_rcp(h4);
+        const double rm = rp_div_by(u1 - u0, h4, yh);                              // raw(i+1)
+        const double fi = (i == 1) ? rm - 0.0 : rm - rp_quot(u0 - um, f0 - fm);
+        const double fn = (i + 1 == np) ? -rm : rp_quot(u2 - u1, f2 - f1) - rm;
+        const double a1i = y0 - K1 * fi;
+        const double a1n = y1 - K1 * fn;
+        const double a3i = u0 * 6.0 * p;
+        const double a3n = u1 * 6.0 * p;
+        const double a4i = rp_div_by(a3n - a3i, h4, yh);
+        pc.a1 = a1i;
+        pc.a2 = rp_div_by(a1n - a1i, h4, yh) - (a3i + rp_div_by(a4i, 3.0, 1.0 / 3.0) * h4) / 2.0 * h4;
+        pc.a3 = a3i;
+        pc.a4 = a4i;
+        pc.x0 = f0;
+        pc.x1 = f1;
+    }
     // Horner loop of ppvalu with k = 4: value = (value/fmmjdr)*h + coef(m)
-    const double h = x - w.fitz(i);
+    const double h = x - pc.x0;
     double value = 0.0;
     if (jderiv == 0) {
-        value = (value / 4.0) * h + a4i;
-        value = (value / 3.0) * h + a3i;
-        value = (value / 2.0) * h + a2i;
-        value = (value / 1.0) * h + a1i;
+        value = (value / 4.0) * h + pc.a4;
+        value = rp_div_by(value, 3.0, 1.0 / 3.0) * h + pc.a3;
+        value = (value / 2.0) * h + pc.a2;
+        value = (value / 1.0) * h + pc.a1;
     } else {
-        value = (value / 3.0) * h + a4i;
-        value = (value / 2.0) * h + a3i;
-        value = (value / 1.0) * h + a2i;
+        value = (value / 3.0) * h + pc.a4;
+        value = (value / 2.0) * h + pc.a3;
+        value = (value / 1.0) * h + pc.a2;
     }
     return value;
 }
@@ -386,88 +614,179 @@ __device__ __forceinline__ double rp_ppvalu(const W& w, int np, double p, double
 // VTurb (ver_turb_module.f90:31-329).  The 2-D quantities at (Xpar, Ypar)
 // are those of RK stage 1 (identical operations and operands).
 template <typename T, class W>
-__device__ double rp_vturb(const RpStepArgs& A, const RpGridDev& g, const StageState& S, double Zpar,
-                           uint32_t pid, uint32_t& fl, const W& w) {
+__device__ __forceinline__ double rp_vturb(const RpStepArgs& A, const RpGridDev& g, const StageState& S, double Zpar,
+                                           uint32_t pid, uint32_t& fl, const W& w) {
     const int sw = g.N + 1;
     const int np = (int)((double)sw * A.sub);
     const double tdepth = S.tdepth, zeta = S.zeta;
     const double h = -1.0 * tdepth;
     const ZCtx zx = rp_zctx(g.vtransform, g.hc, h);
-    // column z(k), KH(k) (ver_turb_module.f90:100-124), held in the r1/r2
-    // arrays until the fit overwrites them
-    auto zc = [&](int k) -> double& { return w.r1(k); };
-    auto kh = [&](int k) -> double& { return w.r2(k); };
+    // column z(k), KH(k) (ver_turb_module.f90:100-124)
     const double* cw = S.rc.wet4 ? S.rc.cb : S.rc.ci;
     const int64_t o[4] = {S.rc.o00, S.rc.o10, S.rc.o11, S.rc.o01};
-    for (int k = 1; k <= sw; k++) {
-        const double s = __ldg(g.sw + k - 1), cs = __ldg(g.csw + k - 1);
-        double zb, zcv, zf;
-        if (g.vtransform == 2) {
-            const double Sk = rp_div_by(g.hc * s + h * cs, zx.den, zx.yden);
-            zb = S.zb + (S.zb + h) * Sk;
-            zcv = S.zc + (S.zc + h) * Sk;
-            zf = S.zf + (S.zf + h) * Sk;
-        } else {
-            zb = rp_zlevel_c(zx, s, cs, S.zb);
-            zcv = rp_zlevel_c(zx, s, cs, S.zc);
-            zf = rp_zlevel_c(zx, s, cs, S.zf);
-        }
-        zc(k) = rp_polintd(A.pi, zb, zcv, zf);
-        double ab[4], ac[4], af[4];
+    bool asc = true;               // the levels ascend
+    double z1 = 0.0, ztop = 0.0, k1 = 0.0, ktop = 0.0;
+    // the corners' three slots of a level, loaded a level ahead of their use
+    const T* aks = reinterpret_cast<const T*>(g.aks);
+    const T* col[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) col[q] = aks + o[q] * sw * RP_SLOTS;
+    T nb[4], nc[4], nf[4];
+    double ns = __ldg(g.sw), ncs = __ldg(g.csw);
+    auto fetch = [&](int k) {
 #pragma unroll
         for (int q = 0; q < 4; q++) {
-            const int64_t base = (o[q] * sw + (k - 1)) * RP_SLOTS;
-            ab[q] = rp_ld<T>(g.aks, base + g.sb);
-            ac[q] = rp_ld<T>(g.aks, base + g.sc);
-            af[q] = rp_ld<T>(g.aks, base + g.sf);
+            const T* c = col[q] + (k - 1) * RP_SLOTS;
+            nb[q] = __ldg(c + g.sb);
+            nc[q] = __ldg(c + g.sc);
+            nf[q] = __ldg(c + g.sf);
         }
-        const double Kb = cw[0] * ab[0] + cw[1] * ab[1] + cw[2] * ab[2] + cw[3] * ab[3];
-        const double Kc = cw[0] * ac[0] + cw[1] * ac[1] + cw[2] * ac[2] + cw[3] * ac[3];
-        const double Kf = cw[0] * af[0] + cw[1] * af[1] + cw[2] * af[2] + cw[3] * af[3];
-        kh(k) = rp_polintd(A.pi, Kb, Kc, Kf);
+        ns = __ldg(g.sw + k - 1);
+        ncs = __ldg(g.csw + k - 1);
+    };
+    fetch(1);
+#pragma unroll 2
+    for (int k = 1; k <= sw; k++) {
+        const double s = ns, cs = ncs;
+        double K3[3], z3[3];
+        K3[0] = cw[0] * (double)nb[0] + cw[1] * (double)nb[1] + cw[2] * (double)nb[2] + cw[3] * (double)nb[3];
+        K3[1] = cw[0] * (double)nc[0] + cw[1] * (double)nc[1] + cw[2] * (double)nc[2] + cw[3] * (double)nc[3];
+        K3[2] = cw[0] * (double)nf[0] + cw[1] * (double)nf[1] + cw[2] * (double)nf[2] + cw[3] * (double)nf[3];
+        fetch(min(k + 1, sw));
+        if (g.vtransform == 2) {
+            const double Sk = rp_div_by(g.hc * s + h * cs, zx.den, zx.yden);
+            z3[0] = S.zb + (S.zb + h) * Sk;
+            z3[1] = S.zc + (S.zc + h) * Sk;
+            z3[2] = S.zf + (S.zf + h) * Sk;
+        } else {
+            z3[0] = rp_zlevel_c(zx, s, cs, S.zb);
+            z3[1] = rp_zlevel_c(zx, s, cs, S.zc);
+            z3[2] = rp_zlevel_c(zx, s, cs, S.zf);
+        }
+        double zk, kk;
+        rp_polintd2(A.pi, z3, K3, zk, kk);
+        w.u(k) = zk;
+        if (k == 1) {
+            z1 = zk;
+            k1 = kk;
+        } else {
+            asc = asc && (zk > ztop);
+            const double m = rp_quot(ktop - kk, ztop - zk);  // linint's line on [z(k-1), z(k)]
+            w.set_r12(k - 1, m, ktop - m * ztop);
+        }
+        ztop = zk;
+        ktop = kk;
     }
-    // resample to np points (ver_turb_module.f90:126-136), linint per point
-    const double dz = (zc(sw) - zc(1)) / (double)(np - 1);
-    w.fitz(1) = zc(1);
-    w.fitz(np) = zc(sw);
-    w.y(1) = kh(1);
-    w.y(np) = kh(sw);
-    double x = zc(1);
-    for (int i = 2; i <= np - 1; i++) {
-        x = x + dz;
-        w.fitz(i) = x;
-        int jlo = 1, jhi = sw;
-        for (;;) {
-            const int k = (jhi + jlo) / 2;
-            if (zc(k) > x) jhi = k; else jlo = k;
-            if (jhi - jlo == 1) break;
+    // resample to np points (ver_turb_module.f90:126-136), linint per point;
+    // setupq's Q'y (pppack.f90:4816-4822) on the way.  On
+    // ascending levels linint's bisection ends on the last level at or below
+    // the point, which the ascending points reach by walking up.
+    const double dz = (ztop - z1) / (double)(np - 1);
+    RpFit F;
+    F.np = np;
+    F.mono = asc && dz > 1e-9 * fmax(fabs(z1), fabs(ztop));
+    F.z1 = z1;
+    F.dz = dz;
+    F.zend = ztop;
+    F.rdz = 1.0 / dz;
+    F.serr = A.serr;
+    F.dy2 = A.serr * A.serr;
+#pragma unroll
+    for (int q = 0; q < kChgWords; q++) F.chg[q] = 0u;
+    {
+        w.fitz(1) = z1;
+        w.y(1) = k1;
+        int j = 1;                               // the point's bracket [z(j), z(j+1)]
+        double zn = w.u(2);
+        double2 ln = w.r12(1), ln2 = w.r12(2);   // its line and the next bracket's
+        double x = z1, fprev = z1, yprev = k1, dprev = 0.0;
+        double v4 = 0.0, yv = 0.0;
+        for (int i = 2; i <= np; i++) {
+            double yi;
+            if (i < np) {
+                x = x + dz;
+                if (asc) {
+                    while (j < sw - 1 && zn <= x) {
+                        j++;
+                        zn = w.u(j + 1);
+                        ln = ln2;
+                        ln2 = w.r12(j + 1);      // read a bracket ahead of its use
+                    }
+                } else {
+                    int jlo = 1, jhi = sw;
+                    for (;;) {
+                        const int k = (jhi + jlo) / 2;
+                        if (w.u(k) > x) jhi = k; else jlo = k;
+                        if (jhi - jlo == 1) break;
+                    }
+                    ln = w.r12(jlo);
+                }
+                yi = ln.x * x + ln.y;
+            } else {
+                x = ztop;
+                yi = ktop;
+            }
+            w.fitz(i) = x;
+            w.y(i) = yi;
+            const double v = x - fprev;          // v4(i-1)
+            if (i == 2 || !(v == v4)) {
+                v4 = v;
+                yv = rp_rcp(v);
+                if (i > 2) {
+#pragma unroll
+                    for (int q = 0; q < kChgWords; q++)
+                        F.chg[q] |= (((i - 1) >> 5) == q) ? 1u << ((i - 1) & 31) : 0u;
+                }
+            }
+            if (i == 2) {
+                F.v1 = v;
+                F.y1 = yv;
+            }
+            if (i == 3) F.v2 = v;
+            if (i == 4) {
+                F.v3 = v;
+                F.f4 = x;
+            }
+            const double diff = rp_div_by(yi - yprev, v, yv);
+            if (i > 2) w.qty(i - 1) = diff - dprev;
+            dprev = diff;
+            fprev = x;
+            yprev = yi;
         }
-        const double m = (kh(jlo) - kh(jhi)) / (zc(jlo) - zc(jhi));
-        const double b = kh(jlo) - m * zc(jlo);
-        w.y(i) = m * x + b;
+        F.r1 = A.serr / F.v1;
+        F.r2 = A.serr / F.v2;
+        F.r3 = A.serr / F.v3;
+        const unsigned lanes = __activemask();
+#pragma unroll
+        for (int q = 0; q < kChgWords; q++) F.chg[q] = __reduce_or_sync(lanes, F.chg[q]);
     }
     int passes;
-    const RpBreaks B{zc(1), dz, zc(sw)};
-    const double p = rp_smooth(w, np, B, A.serr, A.smth, A.spline_max_iter, fl, passes);
+    const double p = rp_smooth(w, F, A.smth, A.spline_max_iter, fl, passes);
     if (A.spl) rp_count_fit(A.spl, passes);
 
     // random displacement sub-steps (ver_turb_module.f90:231-293)
     const double deltat = A.deltat;
-    double ParZc = Zpar;
+    double ParZc = Zpar, dev_next = 0.0;
+    RpPiece pc;
+    pc.x0 = 1.0;
+    pc.x1 = 0.0;
+#pragma unroll 1
     for (int i = 1; i <= A.loop; i++) {
+        double DEV;                              // draw 1+i; pairs (2,3), (4,5), ...
+        if (i & 1) rp_normal2(A, pid, (uint32_t)(1 + i), i < A.loop, DEV, dev_next);
+        else DEV = dev_next;
         double Kprimec = 0.0;
         if (ParZc <= tdepth || ParZc >= zeta) Kprimec = 0.0;
-        else Kprimec = rp_ppvalu(w, np, p, A.serr, ParZc, 1);
+        else Kprimec = rp_ppvalu(w, F, p, ParZc, 1, pc);
         const double KprimeZc = Kprimec * deltat;
         const double Z3rdc = ParZc + 0.5 * KprimeZc;
         double KH3rdc;
         if (Z3rdc < tdepth || Z3rdc > zeta) {
             KH3rdc = A.aksback;
         } else {
-            KH3rdc = rp_ppvalu(w, np, p, A.serr, Z3rdc, 0);
+            KH3rdc = rp_ppvalu(w, F, p, Z3rdc, 0, pc);
             if (KH3rdc < A.aksback) KH3rdc = A.aksback;
         }
-        const double DEV = rp_normal(A, pid, (uint32_t)(1 + i));
         const double r = 1.0;
         const double dTz = KprimeZc + DEV * sqrt(2.0 / r * KH3rdc * deltat);
         ParZc = ParZc + dTz;
@@ -488,7 +807,7 @@ __device__ __forceinline__ bool rp_active(const RpStepArgs& A, int64_t n) {
     return true;
 }
 
-// VTurb of one particle on its own (the first kernel of the split step):
+// VTurb of one particle on its own (the first kernel of the step):
 // the stage-1 z clamp of find_currents (advection_module.f90:171-183) is
 // applied first when RK4 runs, exactly as RKAdvect hands Zpar to VTurb.
 template <typename T, class W>
@@ -714,10 +1033,10 @@ __device__ __noinline__ double rp_behave(const RpStepArgs& A, int64_t n, const R
     return rp_behave_z(A, wb);
 }
 
-// One particle of update_particles.  With turbv_in non-null the VTurb
-// displacement comes from the split kernel instead of being computed here.
-template <typename T, class W>
-__device__ void rp_update_one(const RpStepArgs& A, int64_t n, const W& w, const double* turbv_in) {
+// One particle of update_particles; with VTurb on, turbv holds the VTurb
+// kernel's displacements.
+template <typename T>
+__device__ void rp_update_one(const RpStepArgs& A, int64_t n, const double* turbv) {
     const RpParticlesDev& P = A.p;
     if (!rp_active(A, n)) return;                          // ROMSPath.f90:672-690
     P.age[n] = P.age[n] + (double)(float)A.idt;            // 693
@@ -743,36 +1062,38 @@ __device__ void rp_update_one(const RpStepArgs& A, int64_t n, const W& w, const 
     }
 
     double AdvectX = 0.0, AdvectY = 0.0, AdvectZ = 0.0;
-    StageState S1;
-    bool have_s1 = false;
     if (A.scheme == 1) {                                   // RKAdvect, advection_module.f90:20-125
+        // stages 2-4 start from the (stage-1 clamped) start position plus the
+        // previous stage's slope times idt/2; a loop, so that the stage's code
+        // (about 2,000 instructions) stays in the instruction cache
         const double didt = (double)A.idt;
-        double Uad, Vad, Wad;
-        StageState St;
-        rp_find_currents<T>(A, g, Xpar, Ypar, Zpar, Uad, Vad, Wad, S1, fl);
-        have_s1 = true;
-        const double kn1_u = Uad * pm, kn1_v = Vad * pn, kn1_w = Wad;
-        double x1 = Xpar + Uad * pm * didt / 2.0;
-        double y1 = Ypar + Vad * pn * didt / 2.0;
-        double z1 = Zpar + Wad * didt / 2.0;
-        rp_find_currents<T>(A, g, x1, y1, z1, Uad, Vad, Wad, St, fl);
-        const double kn2_u = Uad * pm, kn2_v = Vad * pn, kn2_w = Wad;
-        double x2 = Xpar + Uad * pm * didt / 2.0;
-        double y2 = Ypar + Vad * pn * didt / 2.0;
-        double z2 = Zpar + Wad * didt / 2.0;
-        rp_find_currents<T>(A, g, x2, y2, z2, Uad, Vad, Wad, St, fl);
-        const double kn3_u = Uad * pm, kn3_v = Vad * pn, kn3_w = Wad;
-        double x3 = Xpar + Uad * pm * didt / 2.0;
-        double y3 = Ypar + Vad * pn * didt / 2.0;
-        double z3 = Zpar + Wad * didt / 2.0;
-        rp_find_currents<T>(A, g, x3, y3, z3, Uad, Vad, Wad, St, fl);
-        const double kn4_u = Uad * pm, kn4_v = Vad * pn, kn4_w = Wad;
-        const double P_U = (kn1_u + 2.0 * kn2_u + 2.0 * kn3_u + kn4_u) / 6.0;
-        const double P_V = (kn1_v + 2.0 * kn2_v + 2.0 * kn3_v + kn4_v) / 6.0;
-        const double P_W = (kn1_w + 2.0 * kn2_w + 2.0 * kn3_w + kn4_w) / 6.0;
-        AdvectX = didt * P_U;
-        AdvectY = didt * P_V;
-        AdvectZ = didt * P_W;
+        double Uad = 0.0, Vad = 0.0, Wad = 0.0, P_U = 0.0, P_V = 0.0, P_W = 0.0;
+#pragma unroll 1
+        for (int st = 0; st < 4; st++) {
+            double xs = Xpar, ys = Ypar, zs = Zpar;
+            if (st > 0) {
+                xs = Xpar + Uad * pm * didt / 2.0;
+                ys = Ypar + Vad * pn * didt / 2.0;
+                zs = Zpar + Wad * didt / 2.0;
+            }
+            StageState St;
+            rp_find_currents<T>(A, g, xs, ys, zs, Uad, Vad, Wad, St, fl);
+            const double kn_u = Uad * pm, kn_v = Vad * pn, kn_w = Wad;
+            if (st == 0) {
+                Zpar = zs;                                 // Z is INOUT in find_currents
+                P_U = kn_u;
+                P_V = kn_v;
+                P_W = kn_w;
+            } else {
+                const double c = (st == 3) ? 1.0 : 2.0;
+                P_U = P_U + c * kn_u;
+                P_V = P_V + c * kn_v;
+                P_W = P_W + c * kn_w;
+            }
+        }
+        AdvectX = didt * (P_U / 6.0);
+        AdvectY = didt * (P_V / 6.0);
+        AdvectZ = didt * (P_W / 6.0);
     }
 
     double TurbHx = 0.0, TurbHy = 0.0;
@@ -788,19 +1109,7 @@ __device__ void rp_update_one(const RpStepArgs& A, int64_t n, const W& w, const 
     TurbHy = TurbHy * pn;
 
     double TurbV = 0.0;
-    if (A.vturb_on && turbv_in) {                          // VTurb, 783 (split kernel)
-        TurbV = turbv_in[n];
-    } else if (A.vturb_on) {                               // VTurb, 783
-        if (!have_s1) {
-            rp_rho_cell(g, Xpar, Ypar, S1.rc, fl);
-            S1.tdepth = -1.0 * rp_bil(g.h, S1.rc);
-            S1.zb = rp_zeta_at<T>(g, S1.rc, g.sb);
-            S1.zc = rp_zeta_at<T>(g, S1.rc, g.sc);
-            S1.zf = rp_zeta_at<T>(g, S1.rc, g.sf);
-            S1.zeta = rp_polintd(A.pi, S1.zb, S1.zc, S1.zf);
-        }
-        TurbV = rp_vturb<T>(A, g, S1, Zpar, pid, fl, w);
-    }
+    if (A.vturb_on) TurbV = turbv[n];                      // VTurb, 783
     double ZBehav = 0.0;                                   // behave(), 800-804
     if (A.beh.behavior || A.beh.va || A.beh.wa) ZBehav = rp_behave<T>(A, n, g, Xpar, Ypar, Zpar, pid, fl);
 
