@@ -324,6 +324,17 @@ __device__ __forceinline__ double rp_div_rcp(double a, double b, const RpRcp& R)
     return fma(r1, R.y, q1);
 }
 
+// 1 / b to about an ulp, for the factors of the forms that need no bit of the
+// reference's (pivots, which depend on the spacing and p alone and are far from
+// the ends of the range): the IEEE operator costs some 40 instructions and a
+// branch, this six
+__device__ __forceinline__ double rp_rcp_ulp(double b) {
+    double s;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(s) : "d"(b));
+    s = fma(s, fma(-b, s, 1.0), s);
+    return fma(s, fma(-b, s, 1.0), s);
+}
+
 // RN(a / b) given y = RN(1 / b)
 __device__ __forceinline__ double rp_div_by(double a, double b, double y) {
     if (max(rp_exp_off_z(a), rp_exp_off(b)) >= kDivSpan) return a / b;

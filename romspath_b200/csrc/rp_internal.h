@@ -21,9 +21,10 @@ constexpr int kVturbSharedBlocks = 10;                 // the same where u is in
 #endif
 constexpr int kAdvectMinBlocks = RP_ADVECT_MIN_BLOCKS; // exact form: 128-thread blocks of the rest of the step
 #ifndef RP_MIXED_MIN_BLOCKS
-#define RP_MIXED_MIN_BLOCKS 8
+#define RP_MIXED_MIN_BLOCKS 4
 #endif
-constexpr int kMixedMinBlocks = RP_MIXED_MIN_BLOCKS;   // same, mixed-precision step
+constexpr int kMixedMinBlocks = RP_MIXED_MIN_BLOCKS;   // same, mixed-precision step with VTurb
+constexpr int kMixedAdvectBlocks = 8;                  // same, without VTurb
 #ifndef RP_MIXED_VT_BLOCKS
 #define RP_MIXED_VT_BLOCKS 2
 #endif

@@ -13,6 +13,14 @@
 namespace rp {
 
 // Fused form: one thread per particle for the whole step.
+//
+// Bound by the latency of the fit's workspace and of the column's gathers
+// (neither the issue slots, about half busy, nor DRAM at 40 %): four blocks of
+// 128 an SM, whose 128 registers hold a quad of rows and the next one's loads
+// without spilling and whose workspaces nearly fit in L2, are faster than eight
+// at 64 registers.  Per 12-step interval, eight, five and four blocks: 512x384x30
+// with 1,048,576 particles 18.8, 18.7 and 18.5 ms; 130x98x20 with 4,194,304 58.8,
+// 54.1 and 51.3 ms (23.0 and 62.8 ms one row at a time in eight blocks).
 // FEAT: built with the options beyond the passive step (diagnostics,
 // WETDRY, behave); the passive variant is chosen when they are all off.
 // BLK: threads per block (the register cap stays that of 128 x 8 resident
@@ -20,11 +28,11 @@ namespace rp {
 template <typename E, int NPMAX, bool FEAT, bool PREF = true, int BLK = kStepBlock>
 __global__ void __launch_bounds__(BLK, kMixedMinBlocks * kStepBlock / BLK)
     k_step_mixed(const __grid_constant__ RpStepArgs A) {
-    double buf[kMixedArrays * (NPMAX + 1)];
+    __align__(16) float buf[MSpline<NPMAX, PREF>::kWords];
     const MSpline<NPMAX, PREF> w{buf};
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < A.p.n; n += stride)
-        m_update_one<E, FEAT>(A, n, w, nullptr);
+        m_update_one<E, FEAT, true>(A, n, w, nullptr);
 }
 
 // Split form: VTurb alone at a resident-thread count whose spline
@@ -33,7 +41,7 @@ __global__ void __launch_bounds__(BLK, kMixedMinBlocks * kStepBlock / BLK)
 template <typename E, int NPMAX>
 __global__ void __launch_bounds__(kStepBlock, kMixedVtMinBlocks) k_vturb_mixed(const __grid_constant__ RpStepArgs A,
                                                                                float* __restrict__ turbv) {
-    double buf[kMixedArrays * (NPMAX + 1)];
+    __align__(16) float buf[MSpline<NPMAX>::kWords];
     const MSpline<NPMAX> w{buf};
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < A.p.n; n += stride)
@@ -61,13 +69,15 @@ __global__ void __launch_bounds__(kSmemBlock) k_vturb_smem(const __grid_constant
         m_vturb_one<E>(A, n, w, turbv);
 }
 
+// The step but for VTurb: the split forms' second kernel, and the whole step
+// with VTurb off (four stages of gathers: more threads hide more).
 template <typename E, bool FEAT>
-__global__ void __launch_bounds__(kStepBlock, kMixedMinBlocks) k_advect_mixed(const __grid_constant__ RpStepArgs A,
+__global__ void __launch_bounds__(kStepBlock, kMixedAdvectBlocks) k_advect_mixed(const __grid_constant__ RpStepArgs A,
                                                              const float* __restrict__ turbv) {
     const MSpline<1> none{nullptr};
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < A.p.n; n += stride)
-        m_update_one<E, FEAT>(A, n, none, turbv);
+        m_update_one<E, FEAT, false>(A, n, none, turbv);
 }
 
 // The diagnostics of the particles the step just advanced (their tdepth in
@@ -131,13 +141,19 @@ static cudaError_t launch_mixed_t(const RpStepArgs& A, float* turbv, int split, 
                                   int* nlaunch) {
     int64_t blocks = 0;
     cudaError_t e;
-    if (split == 2 && A.vturb_on) {
+    if (!A.vturb_on) {
+        if ((e = resident_grid(k_advect_mixed<E, FEAT>, A.p.n, num_sms, A.grid_cap, &blocks)) != cudaSuccess) return e;
+        k_advect_mixed<E, FEAT><<<(unsigned)blocks, kStepBlock, 0, s>>>(A, nullptr);
+        *nlaunch += 1;
+        return cudaGetLastError();
+    }
+    if (split == 2) {
         // the shared-memory column holds sw <= NPMAX/4 levels
         int swmax = 0;
         for (int k = 0; k < A.ngrid; k++) swmax = max(swmax, A.g[k].N + 1);
         if (swmax > NPMAX / 4) split = 1;
     }
-    if (split == 2 && A.vturb_on) {
+    if (split == 2) {
         const size_t smem = (size_t)SmemView<NPMAX>::kWords * kSmemBlock * sizeof(float);
         static bool attr_set = false;
         if (!attr_set) {
@@ -183,7 +199,7 @@ static cudaError_t launch_mixed_t(const RpStepArgs& A, float* turbv, int split, 
         *nlaunch += 1;
         return cudaGetLastError();
     }
-    if (split >= 3 || !split || !A.vturb_on) {
+    if (split >= 3 || !split) {
         if ((e = resident_grid(k_step_mixed<E, NPMAX, FEAT>, A.p.n, num_sms, A.grid_cap, &blocks)) != cudaSuccess)
             return e;
         k_step_mixed<E, NPMAX, FEAT><<<(unsigned)blocks, kStepBlock, 0, s>>>(A);

@@ -25,6 +25,7 @@
 #pragma once
 
 #include <cuda_fp16.h>
+#include <math_constants.h>
 
 #include "rp_step.cuh"
 
@@ -508,33 +509,25 @@ __device__ __forceinline__ void m_find_currents(const RpStepArgs& A, const RpGri
 // traffic is three arrays written forward and read backward plus u written
 // backward.
 
-// Workspace: the chol1d arrays (ratio1, ratio2 and u), then four FP32
-// arrays for the data (the column and the resampled values carry FP32
-// information only).  RP_MIXED_WS sets the chol1d arrays' storage: 0 all
-// FP64, 1 the factor ratios FP32 and u FP64, 2 all FP32 (the default; the
-// sweeps of m_chol1d compute in FP32 either way).  kMixedArrays (NPMAX+1)
-// doubles in all.
-#ifndef RP_MIXED_WS
-#define RP_MIXED_WS 2
-#endif
-#if RP_MIXED_WS == 0
-using MRatio = double;
-using MU = double;
-#elif RP_MIXED_WS == 1
-using MRatio = float;
-using MU = double;
-#else
-using MRatio = float;
-using MU = float;
-#endif
-constexpr int kMixedBytesPerPoint = 2 * (int)sizeof(MRatio) + (int)sizeof(MU) + 4 * 4;
-constexpr int kMixedArrays = (kMixedBytesPerPoint + 7) / 8;
+// Workspace: u, the factor ratios of the rows before the factor turns
+// stationary, the resampled data, and the column's pieces, all FP32 (the
+// sweeps of m_chol1d compute in FP32).  The sweeps take rows 2..5, 6..9, ...
+// together and move each quad as one 16-byte access: element i of u and the
+// ratios sits at position i + 2, that of y, resampled two points ahead of its
+// row, at position i.
+constexpr int m_row_words(int npmax) { return (npmax + 6) / 4 * 4; }   // positions 0 .. npmax + 2
 
-struct MFit;
+struct MFit {
+    int np, sw;
+    double z1, h, rh;              // first break, spacing, 1/h
+    double serr, dy2;
+};
 
-// The per-thread workspace in local memory (the fused step): every array
-// of the fit, the resampled data y stored by the first pass.  PREF: the
-// back substitution loads u four rows ahead (fewer stalls, more registers
+// The per-thread workspace in local memory (the fused step), the resampled
+// data y stored by the first pass (formed again from the column at each piece
+// instead, 512x384x30 with 1,048,576 particles: 19.9 ms an interval, 18.8 with
+// y stored).  Piece j of the column, [z(j), z(j+1)], is one quad (z(j+1), slope, intercept, -).  PREF: the
+// back substitution loads its next quad ahead (fewer stalls, more registers
 // live; which is faster depends on the workload).
 template <int NPMAX, bool PREF = true>
 struct MSpline {
@@ -542,27 +535,28 @@ struct MSpline {
     static constexpr int kColBatch = 2;
     static constexpr bool kLightCheck = false;
     static constexpr bool kPrefetch = PREF;
-    double* base;
-    __device__ __forceinline__ MU& u(int i) const { return reinterpret_cast<MU*>(base)[i]; }  // u(i)/v(i,1), then u(i)
-    __device__ __forceinline__ MRatio* rb() const {
-        return reinterpret_cast<MRatio*>(reinterpret_cast<char*>(base) + (NPMAX + 1) * sizeof(MU));
+    static constexpr int kRow = m_row_words(NPMAX);
+    static constexpr int kWords = 4 * kRow + 4 * (NPMAX + 1);
+    float* base;                   // kWords floats, 16-byte aligned
+    __device__ __forceinline__ float& u(int i) const { return base[i + 2]; }              // u(i)/v(i,1), then u(i)
+    __device__ __forceinline__ float& s1(int i) const { return base[kRow + i + 2]; }      // ratio1(i)
+    __device__ __forceinline__ float& s2(int i) const { return base[2 * kRow + i + 2]; }  // ratio2(i)
+    __device__ __forceinline__ float& y(int i) const { return base[3 * kRow + i]; }       // resampled data y(i)
+    // rows i .. i + 3: i = 2, 6, 10, ... (y: i = 4, 8, ...)
+    __device__ __forceinline__ float4 u4(int i) const { return *reinterpret_cast<const float4*>(&u(i)); }
+    __device__ __forceinline__ float4 s14(int i) const { return *reinterpret_cast<const float4*>(&s1(i)); }
+    __device__ __forceinline__ float4 s24(int i) const { return *reinterpret_cast<const float4*>(&s2(i)); }
+    __device__ __forceinline__ void set_u4(int i, const float4& v) const { *reinterpret_cast<float4*>(&u(i)) = v; }
+    __device__ __forceinline__ void set_s14(int i, const float4& v) const { *reinterpret_cast<float4*>(&s1(i)) = v; }
+    __device__ __forceinline__ void set_s24(int i, const float4& v) const { *reinterpret_cast<float4*>(&s2(i)) = v; }
+    __device__ __forceinline__ void set_y4(int i, const float4& v) const { *reinterpret_cast<float4*>(&y(i)) = v; }
+    __device__ __forceinline__ float yat(const MFit&, int i, int&) const { return y(i); }
+    __device__ __forceinline__ float4 seg(int j) const {
+        return *reinterpret_cast<const float4*>(base + 4 * kRow + 4 * j);
     }
-    __device__ __forceinline__ MRatio& s1(int i) const { return rb()[i]; }                   // ratio1(i)
-    __device__ __forceinline__ MRatio& s2(int i) const { return rb()[(NPMAX + 1) + i]; }     // ratio2(i)
-    __device__ __forceinline__ float* fb() const {
-        return reinterpret_cast<float*>(reinterpret_cast<char*>(base) + (NPMAX + 1) * (sizeof(MU) + 2 * sizeof(MRatio)));
+    __device__ __forceinline__ void set_seg(int j, float zn, float m, float b) const {
+        *reinterpret_cast<float4*>(base + 4 * kRow + 4 * j) = make_float4(zn, m, b, 0.f);
     }
-    __device__ __forceinline__ float& y(int i) const { return fb()[i]; }                     // resampled data y(i)
-    __device__ __forceinline__ float& cz(int k) const { return fb()[(NPMAX + 1) + k]; }      // column z(k)
-    __device__ __forceinline__ float& cm(int k) const { return fb()[2 * (NPMAX + 1) + k]; }  // slope on [z(k), z(k+1)]
-    __device__ __forceinline__ float& cb(int k) const { return fb()[3 * (NPMAX + 1) + k]; }  // intercept
-    __device__ __forceinline__ double yat(const MFit&, int i) const { return (double)y(i); }
-};
-
-struct MFit {
-    int np, sw;
-    double z1, h, rh;              // first break, spacing, 1/h
-    double serr, dy2;
 };
 
 // The workspace in shared memory (the split step's VTurb kernel): u, the
@@ -575,7 +569,6 @@ struct MFit {
 // sweep forms).
 template <int NPMAX, int KSM, int CMAX, int B>
 struct MSmemSpline {
-    static_assert(sizeof(MU) == 4 && sizeof(MRatio) == 4, "shared-memory workspace holds FP32 arrays");
     static constexpr bool kStoreY = false;
     static constexpr int kColBatch = 8;
     static constexpr bool kLightCheck = true;
@@ -591,81 +584,108 @@ struct MSmemSpline {
         return (i <= KSM + 1) ? sm[(NPMAX + KSM + i - 2) * B] : ovf[NPMAX + 1 + i];
     }
     __device__ __forceinline__ float& y(int) const { return ovf[0]; }        // never stored (kStoreY)
+    __device__ __forceinline__ void set_y4(int, const float4&) const {}
+    __device__ __forceinline__ float4 u4(int i) const { return make_float4(u(i), u(i + 1), u(i + 2), u(i + 3)); }
+    __device__ __forceinline__ float4 s14(int i) const { return make_float4(s1(i), s1(i + 1), s1(i + 2), s1(i + 3)); }
+    __device__ __forceinline__ float4 s24(int i) const { return make_float4(s2(i), s2(i + 1), s2(i + 2), s2(i + 3)); }
+    __device__ __forceinline__ void set_u4(int i, const float4& v) const {
+        u(i) = v.x;
+        u(i + 1) = v.y;
+        u(i + 2) = v.z;
+        u(i + 3) = v.w;
+    }
+    __device__ __forceinline__ void set_s14(int i, const float4& v) const {
+        s1(i) = v.x;
+        s1(i + 1) = v.y;
+        s1(i + 2) = v.z;
+        s1(i + 3) = v.w;
+    }
+    __device__ __forceinline__ void set_s24(int i, const float4& v) const {
+        s2(i) = v.x;
+        s2(i + 1) = v.y;
+        s2(i + 2) = v.z;
+        s2(i + 3) = v.w;
+    }
     __device__ __forceinline__ float& cz(int k) const { return sm[(NPMAX + 2 * KSM + k - 1) * B]; }
     __device__ __forceinline__ float& cm(int k) const { return sm[(NPMAX + 2 * KSM + CMAX + k - 1) * B]; }
     __device__ __forceinline__ float& cb(int k) const { return sm[(NPMAX + 2 * KSM + 2 * CMAX + k - 1) * B]; }
-    // resampled value y(i) at z1 + (i-1) h: the column piece j with
-    // cz(j) <= x (j in 1..sw-1; 1 below cz(2)), found by bisection
-    __device__ __forceinline__ double yat(const MFit& f, int i) const;
+    __device__ __forceinline__ float4 seg(int j) const { return make_float4(cz(j + 1), cm(j), cb(j), 0.f); }
+    __device__ __forceinline__ void set_seg(int j, float zn, float m, float b) const {
+        cz(j + 1) = zn;
+        cm(j) = m;
+        cb(j) = b;
+    }
+    __device__ __forceinline__ float yat(const MFit& f, int i, int& j) const;
 };
 
-// linint of the column at ascending points: the current piece j (slope,
-// intercept and upper end) is held in registers and advanced as needed
-template <class W>
+// linint of the column at ascending points in type R: the current piece
+// (slope, intercept and upper end) and the next one are held in registers,
+// so that an advance waits for no load: in a warp some lane advances at
+// nearly every point.  The last piece's upper end is NaN (m_vturb), which
+// ends the walk also at an infinite point (a frame whose zeta is).
+template <class W, typename R>
 struct MWalk {
     int j;
-    double zn, m, b;               // cz(j+1), cm(j), cb(j)
-    __device__ __forceinline__ void init(const W& w) {
-        j = 1;
-        zn = w.cz(2);
-        m = w.cm(1);
-        b = w.cb(1);
+    float4 nx;                     // piece j + 1
+    R zn, m, b;                    // piece j
+    __device__ __forceinline__ void take(const float4& v) {
+        zn = (R)v.x;
+        m = (R)v.y;
+        b = (R)v.z;
     }
-    __device__ __forceinline__ double at(const W& w, int sw, double x) {
-        while (j < sw - 1 && zn <= x) {
+    __device__ __forceinline__ void init(const W& w, int sw) {
+        j = 1;
+        take(w.seg(1));
+        nx = w.seg(min(2, sw - 1));
+    }
+    __device__ __forceinline__ R at(const W& w, int sw, R x) {
+        while (zn <= x) {
             j++;
-            zn = w.cz(j + 1);
-            m = w.cm(j);
-            b = w.cb(j);
+            take(nx);
+            nx = w.seg(min(j + 1, sw - 1));
         }
         return m * x + b;
     }
 };
 
-template <int NPMAX, int KSM, int CMAX, int B>
-__device__ __forceinline__ double MSmemSpline<NPMAX, KSM, CMAX, B>::yat(const MFit& f, int i) const {
-    const double x = (i == 1) ? f.z1 : f.z1 + (double)(i - 1) * f.h;
-    int lo = 1, hi = f.sw - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if ((double)cz(mid) <= x) lo = mid; else hi = mid - 1;
+// The resampled value y(i) at z1 + (i-1) h as the sweeps form it: linint's
+// piece j (j in 1..sw-1, the last whose lower end is at or below the point; 1
+// below z(2)), found by bisection the first time (j = 0) and from the previous
+// point's piece after that.
+template <class W>
+__device__ __forceinline__ float m_resampled(const W& w, const MFit& f, int i, int& j) {
+    const float x = fmaf((float)(i - 1), (float)f.h, (float)f.z1);
+    if (j == 0) {
+        int lo = 1, hi = f.sw - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (w.seg(mid - 1).x <= x) lo = mid; else hi = mid - 1;
+        }
+        j = lo;
     }
-    return (double)cm(lo) * x + (double)cb(lo);
+    while (j > 1 && !(w.seg(j - 1).x <= x)) j--;
+    float4 v = w.seg(j);
+    while (v.x <= x) v = w.seg(++j);
+    return fmaf(v.y, x, v.z);
+}
+template <int NPMAX, int KSM, int CMAX, int B>
+__device__ __forceinline__ float MSmemSpline<NPMAX, KSM, CMAX, B>::yat(const MFit& f, int i, int& j) const {
+    return m_resampled(*this, f, i, j);
 }
 
-// linint of the column at ascending points in FP32 (the column's breaks,
-// slopes and intercepts are stored in FP32)
-template <class W>
-struct MWalkF {
-    int j;
-    float zn, m, b;                // cz(j+1), cm(j), cb(j)
-    __device__ __forceinline__ void init(const W& w) {
-        j = 1;
-        zn = w.cz(2);
-        m = w.cm(1);
-        b = w.cb(1);
-    }
-    __device__ __forceinline__ float at(const W& w, int sw, float x) {
-        while (j < sw - 1 && zn <= x) {
-            j++;
-            zn = w.cz(j + 1);
-            m = w.cm(j);
-            b = w.cb(j);
-        }
-        return fmaf(m, x, b);
-    }
-};
-
 // One chol1d pass at p: factorise, solve for u, form qu = Q u; returns
-// sum_i qu(i)^2 dy^2 and, on request, utru = sum v4 (u(i-1)(u(i-1)+u(i)) + u(i)^2).
+// sum_i qu(i)^2 dy^2.  With store_y the resampled values y(i) are also kept
+// (for ppvalu).
 // The factor's rows before it turns stationary are formed in FP64 and
 // stored in FP32; the substitutions, qu and its sum run in FP32 (the data,
-// the factor ratios and u are FP32 values).  With store_y the resampled
-// values y(i) are also kept (for ppvalu); u is written back only with
-// store_u (a pass whose u may be the fit's).
+// the factor ratios and u are FP32 values).
+//
+// The sweeps take four rows at a time: a quad's values are one 16-byte
+// access of the workspace, and whether the factor still moves is asked once
+// a quad.  One row at a time cost 73 thread instructions a row for both
+// sweeps, 28 of them addresses, counters and compares.
 template <class W>
-__device__ double m_chol1d(const W& w, const MFit& f, double p, double* utru_out, bool store_y,
-                           bool store_u) {
+__device__ __forceinline__ double m_chol1d(const W& w, const MFit& f, double p, bool store_y) {
     store_y = store_y && W::kStoreY;
     const int np = f.np;
     const double r = f.serr * f.rh;
@@ -676,8 +696,8 @@ __device__ double m_chol1d(const W& w, const MFit& f, double p, double* utru_out
     const double F = six1mp * r2;
     const float hf = (float)f.h, rhf = (float)f.rh, z1f = (float)f.z1;
     // Q'y on the fly: qty(i) = (y(i+1) - 2 y(i) + y(i-1)) / h, y at z1 + (i-1) h
-    MWalkF<W> wk;
-    wk.init(w);
+    MWalk<W, float> wk;
+    wk.init(w, f.sw);
     float ym = wk.at(w, f.sw, z1f);
     float y0 = wk.at(w, f.sw, z1f + hf);
     float yp = wk.at(w, f.sw, fmaf(2.f, hf, z1f));
@@ -689,127 +709,158 @@ __device__ double m_chol1d(const W& w, const MFit& f, double p, double* utru_out
     double a1 = D, a2 = E, b1 = D;
     float uprev = 0.f, ucur = (yp - 2.f * y0 + ym) * rhf, r2prev = 0.f;
     // The bands are constant (uniform breaks), so the factor converges to
-    // a fixed point: once a row's ratios round to the previous row's in
-    // FP32, rows ks..np-3 reuse them (no division, no store); the last row
-    // (F = 0 there) is factorised from the held state.
-    int ks = np - 1;                                 // first reused row (np-1: none)
-    float hinv = 0.f, hr1 = 0.f, hr2 = 0.f;
-    float pr1 = 0.f, pr2 = 0.f;
-#pragma unroll 2
-    for (int i = 2; i <= np - 2; i++) {
-        float inv, ratio1, ratio2;
-        if (i < ks || i == np - 2) {
-            const double Fi = (i <= np - 3) ? F : 0.0;
-            const double invd = 1.0 / a1;            // one division per row
-            const double ratio1d = a2 * invd;
-            const double b1n = b1 - ratio1d * a2;
-            const double c2 = E - ratio1d * Fi;
-            const double ratio2d = Fi * invd;
-            const double c1 = D - ratio2d * Fi;
-            inv = (float)invd;
-            ratio1 = (float)ratio1d;
-            ratio2 = (float)ratio2d;
-            if (i > 2 && i < np - 2 && ratio1 == pr1 && ratio2 == pr2) {
-                ks = i;
-                hinv = inv;
-                hr1 = ratio1;
-                hr2 = ratio2;
-            } else {
-                w.s1(i) = ratio1;
-                w.s2(i) = ratio2;
-                a1 = b1n;
-                a2 = c2;
-                b1 = c1;
-            }
-            pr1 = ratio1;
-            pr2 = ratio2;
-        } else {
-            inv = hinv;
-            ratio1 = hr1;
-            ratio2 = hr2;
-        }
-        w.u(i) = ucur * inv;
+    // a fixed point: once the last two rows of a quad have the same ratios
+    // in FP32, rows ks..np-3 reuse them (no division, no store); the last
+    // row (F = 0 there) is factorised from the state held then.
+    int ks = np - 2;                                 // first reused row (np-2: none)
+    bool held = false;
+    float hinv = 0.f, h1 = 0.f, h2 = 0.f;
+    float xi = 3.f;                                  // point i + 1 (0-based), the next to be resampled
+    auto factor = [&](float& inv, float& ratio1, float& ratio2) {
+        const double invd = rp_rcp_ulp(a1);               // one reciprocal per row
+        const double ratio1d = a2 * invd, ratio2d = F * invd;
+        a1 = b1 - ratio1d * a2;
+        a2 = E - ratio1d * F;
+        b1 = D - ratio2d * F;
+        inv = (float)invd;
+        ratio1 = (float)ratio1d;
+        ratio2 = (float)ratio2d;
+    };
+    // row i's u(i)/v(i,1); advances the substitution to row i + 1
+    auto forward = [&](float inv, float ratio1, float ratio2) -> float {
+        const float ui = ucur * inv;
         ym = y0;
         y0 = yp;
-        yp = wk.at(w, f.sw, fmaf((float)(i + 1), hf, z1f));   // y(i+2) at z1 + (i+1) h
-        if (store_y) w.y(i + 2) = yp;
-        const float qn = (yp - 2.f * y0 + ym) * rhf;          // qty(i+1)
+        yp = wk.at(w, f.sw, fmaf(xi, hf, z1f));      // y(i+2) at z1 + (i+1) h
+        xi += 1.f;
+        const float qn = (yp - 2.f * y0 + ym) * rhf; // qty(i+1)
         const float unext = qn - ratio1 * ucur - r2prev * uprev;
         uprev = ucur;
         ucur = unext;
         r2prev = ratio2;
+        return ui;
+    };
+    int i = 2;
+#pragma unroll 1
+    for (; i + 3 <= np - 3; i += 4) {
+        float inv[4], q1[4], q2[4], uq[4], yq[4];
+        if (!held) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) factor(inv[k], q1[k], q2[k]);
+            w.set_s14(i, make_float4(q1[0], q1[1], q1[2], q1[3]));
+            w.set_s24(i, make_float4(q2[0], q2[1], q2[2], q2[3]));
+            if (q1[3] == q1[2] && q2[3] == q2[2]) {
+                held = true;
+                ks = i + 4;
+                hinv = inv[3];
+                h1 = q1[3];
+                h2 = q2[3];
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                inv[k] = hinv;
+                q1[k] = h1;
+                q2[k] = h2;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            uq[k] = forward(inv[k], q1[k], q2[k]);
+            yq[k] = yp;
+        }
+        w.set_u4(i, make_float4(uq[0], uq[1], uq[2], uq[3]));
+        if (store_y) w.set_y4(i + 2, make_float4(yq[0], yq[1], yq[2], yq[3]));
     }
+    const int it = i;                                // first row after the quads
+#pragma unroll 1
+    for (; i <= np - 3; i++) {
+        float inv = hinv, ratio1 = h1, ratio2 = h2;
+        if (!held) {
+            factor(inv, ratio1, ratio2);
+            w.s1(i) = ratio1;
+            w.s2(i) = ratio2;
+        }
+        w.u(i) = forward(inv, ratio1, ratio2);
+        if (store_y) w.y(i + 2) = yp;
+    }
+    // row np-2 (F = 0) and u(np-1)
+    const double invl = rp_rcp_ulp(a1);
+    const double ratiol = a2 * invl;
+    const float q1l = (float)ratiol;
+    const float ul = forward((float)invl, q1l, 0.f); // resamples y(np)
+    if (store_y) w.y(np) = yp;
+    const float uend = (float)((double)ucur / (b1 - ratiol * a2));
     // back substitution, descending, with qu and its sum of squares:
     // raw(k) = (u(k) - u(k-1))/h for 2 <= k <= np, raw(1) = raw(np+1) = 0,
     // qu(k) = raw(k+1) - raw(k)
-    const bool want_utru = utru_out != nullptr;
-    float up1 = 0.f;                                 // u(np)
-    float up2 = 0.f;                                 // u(np+1), unused
-    float rawp = 0.f;                                // raw(np+1)
-    float sum = 0.f, utru = 0.f;                     // sum of qu^2 (times dy2 at the end)
-    if (store_u) w.u(np) = 0.f;
-    {
-        const float ui = (float)((double)ucur / a1); // u(np-1)
-        if (store_u) w.u(np - 1) = ui;
-        const float raw = (up1 - ui) * rhf;          // raw(np)
-        const float fin = rawp - raw;                // qu(np)
-        sum = fmaf(fin, fin, sum);
-        if (want_utru) utru = utru + hf * (ui * (ui + up1) + up1 * up1);
-        rawp = raw;
-        up2 = up1;
-        up1 = ui;
-    }
-    const float h1 = hr1, h2 = hr2;                  // the held rows' ratios
-    // with W::kPrefetch, u(i) is loaded four rows ahead of its use (index 1
-    // stands in past the start; that value is never used)
-    float q0 = w.u(np - 2), q1 = w.u(max(np - 3, 1)), q2 = w.u(max(np - 4, 1)), q3 = w.u(max(np - 5, 1));
-#pragma unroll 2
-    for (int i = np - 2; i >= 2; i--) {
-        float uq;
-        if constexpr (W::kPrefetch) {
-            uq = q0;
-            q0 = q1;
-            q1 = q2;
-            q2 = q3;
-            q3 = w.u(max(i - 4, 1));
-        } else {
-            uq = w.u(i);
-        }
-        const bool held = (i >= ks && i <= np - 3);
-        float s1v = h1, s2v = h2;
-        if (!held) {
-            s1v = w.s1(i);
-            s2v = w.s2(i);
-        }
-        const float ui = uq - up1 * s1v - up2 * s2v;
-        if (store_u) w.u(i) = ui;
+    float up1 = 0.f, up2 = 0.f;                      // u(i+1), u(i+2)
+    float rawp = 0.f;                                // raw(i+2)
+    float sum = 0.f;                                 // sum of qu^2 (times dy2 at the end)
+    auto tally = [&](float ui) {
         const float raw = (up1 - ui) * rhf;          // raw(i+1)
         const float fin = rawp - raw;                // qu(i+1)
         sum = fmaf(fin, fin, sum);
-        if (want_utru) utru = utru + hf * (ui * (ui + up1) + up1 * up1);
         rawp = raw;
         up2 = up1;
         up1 = ui;
-    }
+    };
+    w.u(np) = 0.f;
+    w.u(np - 1) = uend;
+    tally(uend);
     {
-        const float raw = up1 * rhf;                 // raw(2), u(1) = 0
-        const float fin2 = rawp - raw;               // qu(2)
-        sum = sum + fin2 * fin2 + raw * raw;         // qu(1) = raw(2)
-        if (want_utru) utru = utru + hf * (up1 * up1);
+        const float ui = ul - up1 * q1l;             // u(np) = 0
+        w.u(np - 2) = ui;
+        tally(ui);
     }
-    if (store_u) w.u(1) = 0.f;
-    if (want_utru) *utru_out = (double)utru;
+#pragma unroll 1
+    for (i = np - 3; i >= it; i--) {
+        const float s1v = held ? h1 : w.s1(i), s2v = held ? h2 : w.s2(i);
+        const float ui = w.u(i) - up1 * s1v - up2 * s2v;
+        w.u(i) = ui;
+        tally(ui);
+    }
+    i = it - 4;
+    float4 un = w.u4(max(i, 2));
+#pragma unroll 1
+    for (; i >= 2; i -= 4) {
+        float4 s1q = make_float4(h1, h1, h1, h1), s2q = make_float4(h2, h2, h2, h2);
+        if (i < ks) {
+            s1q = w.s14(i);
+            s2q = w.s24(i);
+        }
+        float4 uq = W::kPrefetch ? un : w.u4(i);
+        if (W::kPrefetch) un = w.u4(max(i - 4, 2));
+        uq.w = uq.w - up1 * s1q.w - up2 * s2q.w;
+        tally(uq.w);
+        uq.z = uq.z - up1 * s1q.z - up2 * s2q.z;
+        tally(uq.z);
+        uq.y = uq.y - up1 * s1q.y - up2 * s2q.y;
+        tally(uq.y);
+        uq.x = uq.x - up1 * s1q.x - up2 * s2q.x;
+        tally(uq.x);
+        w.set_u4(i, uq);
+    }
+    tally(0.f);                                      // u(1) = 0: raw(2), qu(2)
+    sum = fmaf(rawp, rawp, sum);                     // qu(1) = raw(2)
+    w.u(1) = 0.f;
     return (double)sum * f.dy2;
 }
 
-// SF(q) = 36 sum qu^2 dy^2 / (1+q)^2 of one chol1d pass at p = q/(1+q)
+// utru = sum v4 (u(i-1)(u(i-1)+u(i)) + u(i)^2) of the pass just made
 template <class W>
-__device__ __forceinline__ double m_sf(const W& w, const MFit& f, double q, bool store_y,
-                                       bool store_u) {
-    return 36.0 * m_chol1d(w, f, q / (1.0 + q), nullptr, store_y, store_u) / ((1.0 + q) * (1.0 + q));
+__device__ __forceinline__ float m_utru(const W& w, const MFit& f) {
+    const float hf = (float)f.h;
+    float utru = 0.f, up1 = 0.f;
+    for (int i = f.np - 1; i >= 1; i--) {
+        const float ui = w.u(i);
+        utru = utru + hf * (ui * (ui + up1) + up1 * up1);
+        up1 = ui;
+    }
+    return utru;
 }
 
-// The same sum S(p) = sum qu^2 dy^2 = u'Tu (T = Q'D^2Q) from one forward
+// chol1d's sum S(p) = sum qu^2 dy^2 = u'Tu (T = Q'D^2Q) from one forward
 // sweep, with nothing stored and no back substitution.  With
 // M(p) = 6(1-p) T + p R the matrix of chol1d and b = Q'y, let
 // phi(p) = b'M^-1 b = sum_i w_i^2 / d_i over the forward-substituted values
@@ -832,8 +883,8 @@ __device__ double m_light_S(const W& w, const MFit& f, double p) {
     const double Dd = -36.0 * r2 + 4.0 * f.h;          // dD/dp, dE/dp, dF/dp
     const double Ed = 24.0 * r2 + f.h;
     const double Fd = -6.0 * r2;
-    MWalk<W> wk;
-    wk.init(w);
+    MWalk<W, double> wk;
+    wk.init(w, f.sw);
     double ym = wk.at(w, f.sw, f.z1);
     double y0 = wk.at(w, f.sw, f.z1 + f.h);
     double xn = f.z1 + 2.0 * f.h;
@@ -911,116 +962,98 @@ __device__ __forceinline__ bool m_stencil_moved(const RpStepArgs& A) { return A.
 template <class W>
 __device__ double m_smooth(const W& w, const MFit& f, double s, int max_iter, double& qstate,
                            double& gstate, float& q2state, uint32_t& fl, int& passes) {
-    // the first full pass of every path also stores y(i); the p = 0 pass
-    // does not store u and is repeated as a full pass when p = 0 is the fit
-    passes = 1;
-    if (s <= 0.0) {
-        m_chol1d(w, f, 1.0, nullptr, true, true);
-        return 1.0;
-    }
+    // one call site of chol1d: its passes follow one another in a loop
+    enum { kGuess, kGuessFit, kNewton, kCold, kSecant };
     const double ooss = 1.0 / sqrt(s);
     const double q_in = qstate;
-    double q = q_in;
-    const bool warm = q > 0.0;
-    bool ys = false;                                 // y(i) stored by a pass already
     const double q2 = (double)q2state;               // the q of the step before the previous one
-    q2state = (float)q_in;                           // the previous q, for the next step
-    if (warm) {
-        // first guess: this step's q extrapolated from the previous two
-        // steps' (geometric, the ratio held to [1/2, 2]); the column changes
-        // smoothly from step to step, so this guess usually meets the
-        // criterion at once, where the previous q alone rarely does
-        if (q2 > 0.0) q = q * fmin(fmax(q / q2, 0.5), 2.0);
-        // the check: a full pass that stores u (the guess is usually the
-        // fit), or where the view asks for it a light pass (one forward
-        // sweep, nothing stored) followed by a full pass when it converged
-        double sfq;
-        bool us = false;
-        if (W::kLightCheck) {
-            sfq = 36.0 * m_light_S(w, f, q / (1.0 + q)) / ((1.0 + q) * (1.0 + q));
+    const bool warm = q_in > 0.0 && !(s <= 0.0);
+    if (!(s <= 0.0)) q2state = (float)q_in;          // the previous q, for the next step
+    // first guess: this step's q extrapolated from the previous two
+    // steps' (geometric, the ratio held to [1/2, 2]); the column changes
+    // smoothly from step to step, so this guess usually meets the
+    // criterion at once, where the previous q alone rarely does
+    double q = 0.0;
+    if (warm) q = (q2 > 0.0) ? q_in * fmin(fmax(q_in / q2, 0.5), 2.0) : q_in;
+    double prevq = 0.0, prevsf = 0.0;
+    int stage = warm ? kGuess : kCold, it = 0;
+    bool ys = false;                                 // y(i) stored by a pass already
+    for (passes = 1;; passes++) {
+        const double p = (s <= 0.0) ? 1.0 : q / (1.0 + q);
+        double sum;
+        if (W::kLightCheck && stage == kGuess) {
+            // the check where the view asks for it: one forward sweep,
+            // nothing stored, followed by a full pass when it converged
+            sum = m_light_S(w, f, p);
         } else {
-            sfq = m_sf(w, f, q, true, true);
+            sum = m_chol1d(w, f, p, !ys);
             ys = true;
-            us = true;
         }
-        if (fabs(sfq - s) <= 0.01 * s) {
-            if (!us) {
-                m_chol1d(w, f, q / (1.0 + q), nullptr, !ys, true);
-                passes = 2;
+        if (s <= 0.0 || stage == kGuessFit) return p;
+        const double sfq = 36.0 * sum / ((1.0 + q) * (1.0 + q));
+        const bool met = fabs(sfq - s) <= 0.01 * s;
+        const double oosf = 1.0 / sqrt(sfq);
+        if (stage == kGuess) {
+            prevq = q;
+            prevsf = oosf;
+            if (met) {
+                // the history keeps the root estimate rather than the accepted
+                // q (any q inside the 1 % band is accepted; the extrapolation
+                // of such q's would carry the band's spread)
+                const double qr = (gstate > 0.0) ? q - (oosf - ooss) / gstate : q;
+                qstate = (qr > 0.0) ? qr : q;
+                if (!W::kLightCheck) return p;
+                stage = kGuessFit;
+                continue;
             }
-            // the history keeps the root estimate rather than the accepted
-            // q (any q inside the 1 % band is accepted; the extrapolation
-            // of such q's would carry the band's spread)
-            const double qr = (gstate > 0.0) ? q - (1.0 / sqrt(sfq) - ooss) / gstate : q;
-            qstate = (qr > 0.0) ? qr : q;
-            return q / (1.0 + q);
-        }
-        double prevq = q, prevsf = 1.0 / sqrt(sfq);
-        const double qn = (gstate > 0.0) ? q + (ooss - prevsf) / gstate : 0.0;
-        q = (qn > 0.0) ? qn : q * sqrt(sfq / s);
-        for (int it = 0; it < 6 && q > 0.0; it++) {
-            sfq = m_sf(w, f, q, !ys, true);
-            ys = true;
-            passes++;
-            const double oosf = 1.0 / sqrt(sfq);
+            const double qn = (gstate > 0.0) ? q + (ooss - prevsf) / gstate : 0.0;
+            q = (qn > 0.0) ? qn : q * sqrt(sfq / s);
+            stage = kNewton;
+        } else if (stage == kCold) {
+            // the reference's sequence: p = 0 first
+            if (!(s < sfq)) {
+                qstate = 0.0;
+                gstate = 0.0;
+                return 0.0;
+            }
+            q = -(oosf - ooss) * sfq / (6.0 * (double)m_utru(w, f) * oosf);
+            prevq = 0.0;
+            prevsf = oosf;
+            it = 0;
+            stage = kSecant;
+            continue;
+        } else {
+            it++;
             const double g = (oosf - prevsf) / (q - prevq);
-            if (fabs(sfq - s) <= 0.01 * s) {
+            if (met) {
                 const double qr = q - (oosf - ooss) / g;
                 qstate = (g > 0.0 && qr > 0.0) ? qr : q;
                 gstate = g;
-                return q / (1.0 + q);
+                return p;
             }
             const double change = (oosf - ooss) / g;
             prevq = q;
             q = q - change;
             prevsf = oosf;
+            if (stage == kSecant && it >= max_iter) {
+                fl |= RP_FL_SPLINE;
+                gstate = 0.0;
+                qstate = prevq;
+                return p;
+            }
+        }
+        if (stage == kNewton && !(it < 6 && q > 0.0)) {
+            q = 0.0;
+            stage = kCold;
         }
     }
-    // cold start: the reference's sequence
-    double utru = 0.0;
-    double sfq = 36.0 * m_chol1d(w, f, 0.0, &utru, !ys, false);
-    passes += warm ? 1 : 0;
-    if (!(s < sfq)) {
-        m_chol1d(w, f, 0.0, nullptr, false, true);
-        passes++;
-        qstate = 0.0;
-        gstate = 0.0;
-        return 0.0;
-    }
-    double oosf = 1.0 / sqrt(sfq);
-    q = -(oosf - ooss) * sfq / (6.0 * utru * oosf);
-    double prevq = 0.0, prevsf = oosf;
-    int it = 0;
-    for (;;) {
-        sfq = m_sf(w, f, q, false, true);
-        oosf = 1.0 / sqrt(sfq);
-        it++;
-        passes++;
-        const double g = (oosf - prevsf) / (q - prevq);
-        if (fabs(sfq - s) <= 0.01 * s) {
-            gstate = g;
-            const double qr = q - (oosf - ooss) / g;
-            qstate = (g > 0.0 && qr > 0.0) ? qr : q;
-            return q / (1.0 + q);
-        }
-        if (it >= max_iter) {
-            fl |= RP_FL_SPLINE;
-            gstate = 0.0;
-            break;
-        }
-        const double change = (oosf - ooss) / g;
-        prevq = q;
-        q = q - change;
-        prevsf = oosf;
-    }
-    qstate = q;
-    return q / (1.0 + q);
 }
 
 // One piece of the fit: the coefficients a(i,1..4) smooth's epilogue forms
 // (pppack.f90:5303-5316) for piece i, from u and y.
 struct MPiece {
     int i;                          // 0: none yet
+    int j;                          // the column's piece at break i (where y is not stored; 0: none yet)
     double xi, c1, c2, c3, c4;
 };
 
@@ -1034,8 +1067,10 @@ __device__ __forceinline__ void m_piece(const W& w, const MFit& f, double p, int
     const double raw1 = (u1 - u0) * f.rh;                            // raw(i+1)
     const double raw2 = (i + 2 <= np) ? (u2 - u1) * f.rh : 0.0;      // raw(i+2)
     const double K1 = 6.0 * (1.0 - p) * f.dy2;
-    const double a1i = w.yat(f, i) - K1 * (raw1 - raw0);
-    const double a1n = w.yat(f, i + 1) - K1 * (raw2 - raw1);
+    const double y0 = (double)w.yat(f, i, pc.j);
+    const double y1 = (double)w.yat(f, i + 1, pc.j);
+    const double a1i = y0 - K1 * (raw1 - raw0);
+    const double a1n = y1 - K1 * (raw2 - raw1);
     const double a3i = u0 * 6.0 * p;
     const double a3n = u1 * 6.0 * p;
     const double a4i = (a3n - a3i) * f.rh;
@@ -1106,7 +1141,7 @@ __device__ float m_vturb(const RpStepArgs& A, const RpGridDev& g, const MStage& 
     const float4* qs = reinterpret_cast<const float4*>(g.qs_aks);
     const MTime tk = m_time(A, g, 0);
     const bool all[4] = {true, true, true, true};
-    float zprev = 0.f, kprev = 0.f;
+    float z1 = 0.f, zprev = 0.f, kprev = 0.f;
     // levels in batches of kColBatch: the batch's 4 kColBatch corner loads
     // are issued before any is used, so their latencies overlap (a
     // workspace view for a kernel with registers to spare asks for more)
@@ -1129,17 +1164,17 @@ __device__ float m_vturb(const RpStepArgs& A, const RpGridDev& g, const MStage& 
             const float2 scs = __ldg(g.scs_w + k - 1);
             const float zk = (k == sw) ? S.zeta : m_zlev(g.vtransform, hc, h, den_r, scs.x, scs.y, S.zeta);
             const float kk = m_level_of<E>(v[b], sc[b], cwt, all, tk);   // getInterpAKs
-            w.cz(k) = zk;
             if (k >= 2) {
                 const float m = (kk - kprev) / (zk - zprev);
-                w.cm(k - 1) = m;
-                w.cb(k - 1) = kprev - m * zprev;
+                w.set_seg(k - 1, (k == sw) ? CUDART_NAN_F : zk, m, kprev - m * zprev);
+            } else {
+                z1 = zk;
             }
             zprev = zk;
             kprev = kk;
         }
     }
-    f.z1 = w.cz(1);
+    f.z1 = (double)z1;
     f.h = (zeta - f.z1) / (double)(f.np - 1);
     f.rh = 1.0 / f.h;
     int passes;
@@ -1148,7 +1183,7 @@ __device__ float m_vturb(const RpStepArgs& A, const RpGridDev& g, const MStage& 
     const double deltat = A.deltat;
     double ParZc = (double)Zpar;
     MPiece pc;
-    pc.i = 0;
+    pc.i = pc.j = 0;
     double dev_next = 0.0;
     for (int i = 1; i <= A.loop; i++) {
         double DEV;                                    // draw 1+i; pairs (2,3), (4,5), ...
@@ -1376,11 +1411,12 @@ __device__ void m_vturb_one(const RpStepArgs& A, int64_t n, const W& w, float* t
 }
 
 // One particle of update_particles in the mixed form.  With turbv_in
-// non-null the VTurb displacement comes from the split form's first kernel.
+// non-null the VTurb displacement comes from the split form's first kernel
+// (VT: the kernel forms it itself; without, it carries none of VTurb's code).
 // FEAT: the kernel variant with the options beyond the passive step (the
 // diagnostics, WETDRY, behave); the passive variant carries none of their
 // code.
-template <typename E, bool FEAT, class W>
+template <typename E, bool FEAT, bool VT, class W>
 __device__ void m_update_one(const RpStepArgs& A, int64_t n, const W& w, const float* turbv_in) {
     const RpParticlesDev& Pt = A.p;
     if (!rp_active(A, n)) return;
@@ -1435,7 +1471,7 @@ __device__ void m_update_one(const RpStepArgs& A, int64_t n, const W& w, const f
         AdvectZ = didt * (AdvectZ * (1.f / 6.f));
     }
     MStage S1;
-    if (A.vturb_on && !turbv_in) {
+    if (VT && A.vturb_on) {
         m_rho_cell(g, Xpar, Ypar, S1.rc, fl);
         m_stage_2d(m_time(A, g, 0), g, S1);
     }
@@ -1450,8 +1486,8 @@ __device__ void m_update_one(const RpStepArgs& A, int64_t n, const W& w, const f
     TurbHx *= pm;
     TurbHy *= pn;
     float TurbV = 0.f;
-    if (A.vturb_on && turbv_in) {
-        TurbV = turbv_in[n];
+    if (!VT) {
+        if (A.vturb_on) TurbV = turbv_in[n];
     } else if (A.vturb_on) {
         double q = Pt.qwarm[n], gs = Pt.gwarm[n];
         float q2 = Pt.qwarm2[n];
