@@ -11,6 +11,7 @@
 namespace rp {
 
 constexpr int kAdjBlock = 128;
+constexpr int kAdjVtBlock = 64;
 
 __device__ __forceinline__ void adj_load(const AdjStateDev& s, int64_t n, double& x, double& y, double& z,
                                          AdjAux& a) {
@@ -30,28 +31,81 @@ __device__ __forceinline__ void adj_store_aux(const AdjStateDev& s, int64_t n, c
     s.isin[n] = a.isin;
 }
 
-// one step of the model in doubles on state s; find: search p and record
-// it in prec[n], else use prec[n]
+// VTurb's displacements of a step in doubles (tv[n]); find: search p and
+// record it in prec[n], else use prec[n].
+//
+// Bound by the fit's chains of dependent FP64 operations (a pivot, its
+// reciprocal, the next pivot): 64-thread blocks, eight an SM, hold 65,536
+// particles in one wave; the search's seven or so passes store nothing.  On the
+// 130x98x20 grid with 65,536 particles a forward step (this kernel and the
+// rest) takes 0.40 ms, 1.5 in one kernel whose passes kept their factor and
+// divided three times a row.
 template <int NPMAX>
+__global__ void __launch_bounds__(kAdjVtBlock, 512 / kAdjVtBlock)
+    k_adj_vturb(const __grid_constant__ RpStepArgs A, const __grid_constant__ AdjFrames F, AdjStateDev s,
+                double* __restrict__ prec, int find, double kappa, double* __restrict__ tv) {
+    using W = BFit<NPMAX, false>;
+    double buf[W::kArrays * (NPMAX + 1)];
+    const W w{buf};
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < A.p.n; n += stride) {
+        double p = find ? 0.0 : prec[n], t = 0.0;
+        uint32_t fl = 0;
+        if (a_active(A, A.p.dob[n], s.status[n], s.isin[n]))
+            t = b_vturb(A, F, s.gid[n] - 1, s.x[n], s.y[n], s.z[n], kappa, A.p.pid[n], find != 0, p, fl, w);
+        if (find) prec[n] = p;
+        tv[n] = t;
+    }
+}
+
+// The same with its derivatives in the start's x, y, z and in kappa: tv[q n],
+// q = 0..4 (b_vturb_rev).  A reverse step (this kernel and k_adj_reverse) on
+// the workload above takes 0.9 ms, 1.9 with the fit carried in dual numbers.
+template <int NPMAX>
+__global__ void __launch_bounds__(kAdjVtBlock, 512 / kAdjVtBlock)
+    k_adj_vturb_rev(const __grid_constant__ RpStepArgs A, const __grid_constant__ AdjFrames F, AdjStateDev s,
+                    const double* __restrict__ prec, double kappa, double* __restrict__ tv) {
+    using W = BFit<NPMAX, true>;
+    double buf[W::kArrays * (NPMAX + 1)];
+    const W w{buf};
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < A.p.n; n += stride) {
+        double t[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        uint32_t fl = 0;
+        if (a_active(A, A.p.dob[n], s.status[n], s.isin[n]))
+            b_vturb_rev(A, F, s.gid[n] - 1, s.x[n], s.y[n], s.z[n], kappa, A.p.pid[n], prec[n], fl, w, t);
+#pragma unroll
+        for (int q = 0; q < 5; q++) tv[q * A.p.n + n] = t[q];
+    }
+}
+
+// one step of the model in doubles on state s; with VTurb on, tv holds
+// k_adj_vturb's displacements
 __global__ void __launch_bounds__(kAdjBlock) k_adj_step(const __grid_constant__ RpStepArgs A,
                                                          const __grid_constant__ AdjFrames F, AdjStateDev s,
-                                                         double* __restrict__ prec, int find, double kappa) {
-    double buf[kAdjArrays * (NPMAX + 1)];
-    const AFit<double, NPMAX> w{buf};
+                                                         const double* __restrict__ tv) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < A.p.n; n += stride) {
         double x, y, z;
         AdjAux a;
         adj_load(s, n, x, y, z, a);
-        double p = find ? 0.0 : prec[n];
         uint32_t fl = 0;
-        a_step<double, NPMAX>(A, F, A.p.dob[n], A.p.pid[n], x, y, z, a, kappa, find != 0, p, fl, w);
-        if (find) prec[n] = p;
+        a_step<double>(A, F, A.p.dob[n], A.p.pid[n], x, y, z, a, fl,
+                       [&](const AStage<double>&, bool, double) { return tv[n]; });
         s.x[n] = x;
         s.y[n] = y;
         s.z[n] = z;
         adj_store_aux(s, n, a);
     }
+}
+
+// VTurb in dual numbers within a step
+template <class D, int NPMAX>
+__device__ __forceinline__ D adj_vturb_dual(const RpStepArgs& A, const AdjFrames& F, int gid, const D& X, const D& Y,
+                                            AStage<D>& S1, bool have_s1, const D& Zpar, const D& K, uint32_t pid,
+                                            double p, uint32_t& fl, const AFit<D, NPMAX>& w) {
+    if (!have_s1) b_stage(A, F, gid - 1, X, Y, S1, fl);
+    return a_vturb(A, F, gid - 1, S1, Zpar, K, pid, p, w);
 }
 
 // one step in dual numbers carrying d/d(x0, y0, z0, kappa): tangent-linear
@@ -78,9 +132,12 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_tangent(const __grid_constant
             Z.d[q] = tn[8 + q];
         }
         K.d[3] = 1.0;
-        double p = prec[n];
+        const D X0 = X, Y0 = Y;
+        const int gid = a.gid;
         uint32_t fl = 0;
-        a_step<D, NPMAX>(A, F, A.p.dob[n], A.p.pid[n], X, Y, Z, a, K, false, p, fl, w);
+        a_step<D>(A, F, A.p.dob[n], A.p.pid[n], X, Y, Z, a, fl, [&](AStage<D>& S1, bool have_s1, const D& Zpar) {
+            return adj_vturb_dual<D, NPMAX>(A, F, gid, X0, Y0, S1, have_s1, Zpar, K, A.p.pid[n], prec[n], fl, w);
+        });
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             tn[q] = X.d[q];
@@ -95,14 +152,48 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_tangent(const __grid_constant
 }
 
 // one reverse step: from the step's starting state s (read only), the
-// step's Jacobian by dual numbers seeded on (x, y, z, kappa); then
-// lambda <- J^T lambda for (x, y, z) and kbar += lambda . d(x,y,z)/dkappa
-template <int NPMAX>
+// step's Jacobian by dual numbers seeded on (x, y, z), VTurb's row of it from
+// tv (k_adj_vturb_rev); then lambda <- J^T lambda for (x, y, z) and
+// kbar += lambda . d(x,y,z)/dkappa (kappa enters z alone, through VTurb)
 __global__ void __launch_bounds__(kAdjBlock) k_adj_reverse(const __grid_constant__ RpStepArgs A,
                                                             const __grid_constant__ AdjFrames F, AdjStateDev s,
-                                                            const double* __restrict__ prec, double kappa,
-                                                            double* __restrict__ lx, double* __restrict__ ly,
-                                                            double* __restrict__ lz, double* __restrict__ kbar) {
+                                                            const double* __restrict__ tv, double* __restrict__ lx,
+                                                            double* __restrict__ ly, double* __restrict__ lz,
+                                                            double* __restrict__ kbar) {
+    using D = Dual<3>;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < A.p.n; n += stride) {
+        double x, y, z;
+        AdjAux a;
+        adj_load(s, n, x, y, z, a);
+        D X(x), Y(y), Z(z);
+        X.d[0] = 1.0;
+        Y.d[1] = 1.0;
+        Z.d[2] = 1.0;
+        uint32_t fl = 0;
+        const int vsign = a_step<D>(A, F, A.p.dob[n], A.p.pid[n], X, Y, Z, a, fl,
+                                    [&](const AStage<D>&, bool, const D&) {
+                                        D t(tv[n]);
+#pragma unroll
+                                        for (int q = 0; q < 3; q++) t.d[q] = tv[(q + 1) * A.p.n + n];
+                                        return t;
+                                    });
+        const double bx = lx[n], by = ly[n], bz = lz[n];
+        lx[n] = bx * X.d[0] + by * Y.d[0] + bz * Z.d[0];
+        ly[n] = bx * X.d[1] + by * Y.d[1] + bz * Z.d[1];
+        lz[n] = bx * X.d[2] + by * Y.d[2] + bz * Z.d[2];
+        if (A.vturb_on && vsign) kbar[n] += bz * ((double)vsign * tv[4 * A.p.n + n]);
+    }
+}
+
+// the same with the whole step in dual numbers seeded on (x, y, z, kappa), for
+// runs with more sub-steps a step than k_adj_vturb_rev keeps
+template <int NPMAX>
+__global__ void __launch_bounds__(kAdjBlock) k_adj_reverse_dual(const __grid_constant__ RpStepArgs A,
+                                                                 const __grid_constant__ AdjFrames F, AdjStateDev s,
+                                                                 const double* __restrict__ prec, double kappa,
+                                                                 double* __restrict__ lx, double* __restrict__ ly,
+                                                                 double* __restrict__ lz, double* __restrict__ kbar) {
     using D = Dual<4>;
     D buf[kAdjArrays * (NPMAX + 1)];
     const AFit<D, NPMAX> w{buf};
@@ -116,9 +207,12 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_reverse(const __grid_constant
         Y.d[1] = 1.0;
         Z.d[2] = 1.0;
         K.d[3] = 1.0;
-        double p = prec[n];
+        const D X0 = X, Y0 = Y;
+        const int gid = a.gid;
         uint32_t fl = 0;
-        a_step<D, NPMAX>(A, F, A.p.dob[n], A.p.pid[n], X, Y, Z, a, K, false, p, fl, w);
+        a_step<D>(A, F, A.p.dob[n], A.p.pid[n], X, Y, Z, a, fl, [&](AStage<D>& S1, bool have_s1, const D& Zpar) {
+            return adj_vturb_dual<D, NPMAX>(A, F, gid, X0, Y0, S1, have_s1, Zpar, K, A.p.pid[n], prec[n], fl, w);
+        });
         const double bx = lx[n], by = ly[n], bz = lz[n];
         lx[n] = bx * X.d[0] + by * Y.d[0] + bz * Z.d[0];
         ly[n] = bx * X.d[1] + by * Y.d[1] + bz * Z.d[1];
@@ -128,39 +222,48 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_reverse(const __grid_constant
 }
 
 template <class K>
-static int64_t adj_grid(K kernel, int64_t n, int num_sms) {
+static unsigned adj_grid(K kernel, int64_t n, int num_sms, int block) {
     int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kAdjBlock, 0) != cudaSuccess || occ < 1) occ = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, block, 0) != cudaSuccess || occ < 1) occ = 1;
     int64_t b = (int64_t)num_sms * occ;
-    const int64_t need = (n + kAdjBlock - 1) / kAdjBlock;
+    const int64_t need = (n + block - 1) / block;
     if (need < b) b = need;
-    return b < 1 ? 1 : b;
+    return (unsigned)(b < 1 ? 1 : b);
 }
 
 template <int NPMAX>
 static cudaError_t adj_launch_t(int kind, const RpStepArgs& A, const AdjFrames& F, const AdjStateDev& s,
-                                double* prec, int find, double kappa, double* t, double* lx, double* ly, double* lz,
-                                double* kbar, cudaStream_t st, int num_sms) {
+                                double* prec, int find, double kappa, double* tv, double* t, double* lx, double* ly,
+                                double* lz, double* kbar, cudaStream_t st, int num_sms) {
+    const int64_t n = A.p.n;
     if (kind == 0) {
-        k_adj_step<NPMAX><<<(unsigned)adj_grid(k_adj_step<NPMAX>, A.p.n, num_sms), kAdjBlock, 0, st>>>(A, F, s, prec,
-                                                                                                      find, kappa);
+        if (A.vturb_on)
+            k_adj_vturb<NPMAX><<<adj_grid(k_adj_vturb<NPMAX>, n, num_sms, kAdjVtBlock), kAdjVtBlock, 0, st>>>(
+                A, F, s, prec, find, kappa, tv);
+        k_adj_step<<<adj_grid(k_adj_step, n, num_sms, kAdjBlock), kAdjBlock, 0, st>>>(A, F, s, tv);
     } else if (kind == 1) {
-        k_adj_tangent<NPMAX><<<(unsigned)adj_grid(k_adj_tangent<NPMAX>, A.p.n, num_sms), kAdjBlock, 0, st>>>(
+        k_adj_tangent<NPMAX><<<adj_grid(k_adj_tangent<NPMAX>, n, num_sms, kAdjBlock), kAdjBlock, 0, st>>>(
             A, F, s, t, prec, kappa);
-    } else {
-        k_adj_reverse<NPMAX><<<(unsigned)adj_grid(k_adj_reverse<NPMAX>, A.p.n, num_sms), kAdjBlock, 0, st>>>(
+    } else if (A.vturb_on && A.loop > NPMAX) {
+        k_adj_reverse_dual<NPMAX><<<adj_grid(k_adj_reverse_dual<NPMAX>, n, num_sms, kAdjBlock), kAdjBlock, 0, st>>>(
             A, F, s, prec, kappa, lx, ly, lz, kbar);
+    } else {
+        if (A.vturb_on)
+            k_adj_vturb_rev<NPMAX><<<adj_grid(k_adj_vturb_rev<NPMAX>, n, num_sms, kAdjVtBlock), kAdjVtBlock, 0,
+                                     st>>>(A, F, s, prec, kappa, tv);
+        k_adj_reverse<<<adj_grid(k_adj_reverse, n, num_sms, kAdjBlock), kAdjBlock, 0, st>>>(A, F, s, tv, lx, ly, lz,
+                                                                                            kbar);
     }
     return cudaGetLastError();
 }
 
 cudaError_t launch_adj(int kind, const RpStepArgs& A, const AdjFrames& F, const AdjStateDev& s, double* prec, int find,
-                       double kappa, double* t, double* lx, double* ly, double* lz, double* kbar, int npmax,
-                       cudaStream_t st, int num_sms) {
+                       double kappa, double* tv, double* t, double* lx, double* ly, double* lz, double* kbar,
+                       int npmax, cudaStream_t st, int num_sms) {
     if (A.p.n <= 0) return cudaSuccess;
-    if (npmax <= 88) return adj_launch_t<88>(kind, A, F, s, prec, find, kappa, t, lx, ly, lz, kbar, st, num_sms);
-    if (npmax <= 128) return adj_launch_t<128>(kind, A, F, s, prec, find, kappa, t, lx, ly, lz, kbar, st, num_sms);
-    return adj_launch_t<144>(kind, A, F, s, prec, find, kappa, t, lx, ly, lz, kbar, st, num_sms);
+    if (npmax <= 88) return adj_launch_t<88>(kind, A, F, s, prec, find, kappa, tv, t, lx, ly, lz, kbar, st, num_sms);
+    if (npmax <= 128) return adj_launch_t<128>(kind, A, F, s, prec, find, kappa, tv, t, lx, ly, lz, kbar, st, num_sms);
+    return adj_launch_t<144>(kind, A, F, s, prec, find, kappa, tv, t, lx, ly, lz, kbar, st, num_sms);
 }
 
 // Fortran-ordered field (+ Stokes term, summed in FP64) -> [j][i][k] FP64

@@ -423,9 +423,9 @@ __device__ __forceinline__ S a_linint(const AFit<S, NPMAX>& w, int sw, const S& 
 }
 
 // chol1d (pppack.f90:1428-1566) on uniform breaks at a given p (the bands of
-// the mixed form's m_chol1d); returns sum qu^2 dy^2.  Leaves u(1..np).
+// the mixed form's m_chol1d).  Leaves u(1..np).
 template <class S, int NPMAX>
-__device__ S a_chol1d(const AFit<S, NPMAX>& w, int np, const S& hb, double p, double serr) {
+__device__ void a_chol1d(const AFit<S, NPMAX>& w, int np, const S& hb, double p, double serr) {
     const S r = serr / hb;
     const S r2 = r * r;
     const double six1mp = 6.0 * (1.0 - p);
@@ -454,51 +454,10 @@ __device__ S a_chol1d(const AFit<S, NPMAX>& w, int np, const S& hb, double p, do
         a2 = c2;
         b1 = c1;
     }
-    const double dy2 = serr * serr;
     w.u(np) = S(0.0);
     w.u(np - 1) = ucur / a1;
     for (int i = np - 2; i >= 2; i--) w.u(i) = w.u(i) - w.u(i + 1) * w.s1(i) - w.u(i + 2) * w.s2(i);
     w.u(1) = S(0.0);
-    S prev(0.0), sum(0.0);
-    for (int i = 2; i <= np; i++) {
-        const S raw = (w.u(i) - w.u(i - 1)) * rh;
-        const S fin = raw - prev;
-        sum = sum + fin * fin * dy2;
-        prev = raw;
-    }
-    sum = sum + prev * prev * dy2;
-    return sum;
-}
-
-// smooth()'s secant search for p (pppack.f90:5108-5317, reference cold
-// start) on uniform breaks; values only (double).
-template <int NPMAX>
-__device__ double a_find_p(const AFit<double, NPMAX>& w, int np, double hb, double serr, double s, int max_iter,
-                           uint32_t& fl) {
-    if (s <= 0.0) return 1.0;
-    // utru needs u at p = 0
-    double sfq = 36.0 * a_chol1d(w, np, hb, 0.0, serr);
-    double utru = 0.0;
-    for (int i = 2; i <= np; i++) {
-        const double ul = w.u(i - 1), ui = w.u(i);
-        utru = utru + hb * (ul * (ul + ui) + ui * ui);
-    }
-    if (!(s < sfq)) return 0.0;
-    const double ooss = 1.0 / sqrt(s);
-    double oosf = 1.0 / sqrt(sfq);
-    double q = -(oosf - ooss) * sfq / (6.0 * utru * oosf);
-    double prevq = 0.0, prevsf = oosf;
-    for (int it = 1;; it++) {
-        sfq = 36.0 * a_chol1d(w, np, hb, q / (1.0 + q), serr) / ((1.0 + q) * (1.0 + q));
-        if (fabs(sfq - s) <= 0.01 * s) break;
-        if (it >= max_iter) { fl |= RP_FL_SPLINE; break; }
-        oosf = 1.0 / sqrt(sfq);
-        const double change = (q - prevq) / (oosf - prevsf) * (oosf - ooss);
-        prevq = q;
-        q = q - change;
-        prevsf = oosf;
-    }
-    return q / (1.0 + q);
 }
 
 // ppvalu (pppack.f90:4246-4362) of the fit, piece formed as smooth's
@@ -529,11 +488,10 @@ __device__ __forceinline__ S a_ppvalu(const AFit<S, NPMAX>& w, int np, const S& 
 }
 
 // VTurb (ver_turb_module.f90:31-329) with the diffusivity data scaled by
-// kappa.  With find set, p is searched (values only) and returned in p;
-// otherwise p is the given (recorded) value.
+// kappa, at the recorded smoothing parameter p, in any arithmetic S.
 template <class S, int NPMAX>
 __device__ S a_vturb(const RpStepArgs& A, const AdjFrames& F, int gi, const AStage<S>& St, const S& Zpar,
-                     const S& kappa, uint32_t pid, bool find, double& p, uint32_t& fl, const AFit<S, NPMAX>& w) {
+                     const S& kappa, uint32_t pid, double p, const AFit<S, NPMAX>& w) {
     const RpGridDev& g = A.g[gi];
     const int sw = g.N + 1;
     const int np = (int)((double)sw * A.sub);
@@ -558,11 +516,6 @@ __device__ S a_vturb(const RpStepArgs& A, const AdjFrames& F, int gi, const ASta
     w.y(1) = w.kh(1);
     w.y(np) = w.kh(sw);
     for (int i = 2; i <= np - 1; i++) w.y(i) = a_linint(w, sw, z1 + (double)(i - 1) * hb);
-    if (find) {
-        if constexpr (sizeof(S) == sizeof(double)) {
-            p = a_find_p(w, np, aval(hb), A.serr, A.smth, A.spline_max_iter, fl);
-        }
-    }
     a_chol1d(w, np, hb, p, A.serr);
     // random displacement sub-steps (ver_turb_module.f90:231-293)
     const double deltat = A.deltat;
@@ -589,6 +542,610 @@ __device__ S a_vturb(const RpStepArgs& A, const AdjFrames& F, int gi, const ASta
     return ParZc - Zpar;
 }
 
+// ------------------------------------- VTurb in doubles, and its reverse
+//
+// The forward and replayed steps' VTurb (k_adj_vturb) and the reverse step's
+// (k_adj_vturb_rev), each a kernel of its own.  The reverse differentiates the
+// displacement by hand: through the sub-steps backwards, one more solve with
+// the fit's own factor (its matrix is symmetric), the bands, the resampling
+// and the column.  Carried through the fit as dual numbers of four directions
+// instead, every array holds five doubles a point (31 KB a thread).
+//
+// Arrays of one fit (1-based element i), NPMAX + 1 doubles each.  REV: the
+// reverse's arrays too.
+template <int NPMAX, bool REV>
+struct BFit {
+    static constexpr int kArrays = REV ? 11 : 6;
+    double* base;                  // kArrays (NPMAX + 1) doubles
+    __device__ __forceinline__ double& at(int a, int i) const { return base[a * (NPMAX + 1) + i]; }
+    __device__ __forceinline__ double& zc(int k) const { return at(0, k); }    // column z(k), K(k)
+    __device__ __forceinline__ double& kh(int k) const { return at(1, k); }
+    __device__ __forceinline__ double& y(int i) const { return at(2, i); }     // resampled data
+    __device__ __forceinline__ double& u(int i) const { return at(3, i); }
+    __device__ __forceinline__ double& s1(int i) const { return at(4, i); }    // the factor's ratios
+    __device__ __forceinline__ double& s2(int i) const { return at(5, i); }
+    __device__ __forceinline__ double& inv(int i) const { return at(6, i); }   // 1 / pivot
+    __device__ __forceinline__ double& ub(int i) const { return at(7, i); }    // adjoints of u, then M^-1 of them
+    __device__ __forceinline__ double& yb(int i) const { return at(8, i); }    // adjoints of y
+    __device__ __forceinline__ double& zt(int i) const { return at(9, i); }    // sub-step i's start and deviate
+    __device__ __forceinline__ double& dev(int i) const { return at(10, i); }
+    // adjoints of the column, over the factor once it has been used
+    __device__ __forceinline__ double& zcb(int k) const { return s1(k); }
+    __device__ __forceinline__ double& khb(int k) const { return s2(k); }
+};
+
+// What the passes of a fit share
+struct BPar {
+    int np, sw;
+    double z1, hb, rh, serr, r2;
+    // chol1d's bands on uniform breaks
+    __device__ __forceinline__ void bands(double p, double& D, double& E, double& F) const {
+        const double six1mp = 6.0 * (1.0 - p);
+        D = six1mp * (6.0 * r2) + 4.0 * p * hb;
+        E = six1mp * (-4.0 * r2) + p * hb;
+        F = six1mp * r2;
+    }
+};
+
+// the column's level k: z(k) of the three slots' zeta, K(k) before kappa
+template <class S>
+__device__ __forceinline__ void b_level(const RpStepArgs& A, const AdjFrames& F, int gi, const AStage<S>& St, int k,
+                                        S& z, S& K) {
+    const RpGridDev& g = A.g[gi];
+    const int sw = g.N + 1;
+    const S h = -St.tdepth;
+    const S* cw = St.rc.wet4 ? St.rc.cb : St.rc.ci;
+    const double s = __ldg(g.sw + k - 1), cs = __ldg(g.csw + k - 1);
+    S K3[3];
+#pragma unroll
+    for (int t = 0; t < 3; t++) {
+        const double* a = F.f[gi][4][t] + k - 1;
+        K3[t] = cw[0] * __ldg(a + St.rc.o[0] * sw) + cw[1] * __ldg(a + St.rc.o[1] * sw) +
+                cw[2] * __ldg(a + St.rc.o[2] * sw) + cw[3] * __ldg(a + St.rc.o[3] * sw);
+    }
+    K = a_polint(A.pi, K3[0], K3[1], K3[2]);
+    if (g.vtransform == 2) {                     // the slots share the stretching
+        const S Sk = (g.hc * s + h * cs) / (g.hc + h);
+        z = a_polint(A.pi, St.zb + (St.zb + h) * Sk, St.zc + (St.zc + h) * Sk, St.zf + (St.zf + h) * Sk);
+    } else {
+        z = a_polint(A.pi, a_zlev(g.vtransform, g.hc, s, cs, St.zb, h), a_zlev(g.vtransform, g.hc, s, cs, St.zc, h),
+                     a_zlev(g.vtransform, g.hc, s, cs, St.zf, h));
+    }
+}
+
+// linint's bracket of x in the column: from j up on ascending levels and
+// points, else by its bisection
+template <class W>
+__device__ __forceinline__ int b_bracket(const W& w, int sw, bool asc, int j, double x) {
+    if (asc) {
+        while (j < sw - 1 && !(w.zc(j + 1) > x)) j++;
+        return j;
+    }
+    int lo = 1, hi = sw;
+    while (hi - lo > 1) {
+        const int k = (hi + lo) / 2;
+        if (w.zc(k) > x) hi = k; else lo = k;
+    }
+    return lo;
+}
+
+// column and resampled data (ver_turb_module.f90:100-136)
+template <class W>
+__device__ __forceinline__ void b_column(const RpStepArgs& A, const AdjFrames& F, int gi, const AStage<double>& St,
+                                         double kappa, const W& w, BPar& B, bool& asc) {
+    const int sw = A.g[gi].N + 1, np = (int)((double)sw * A.sub);
+    asc = true;
+    double zp = 0.0;
+#pragma unroll 2
+    for (int k = 1; k <= sw; k++) {
+        double z, K;
+        b_level(A, F, gi, St, k, z, K);
+        w.zc(k) = z;
+        w.kh(k) = kappa * K;
+        asc = asc && (k == 1 || z > zp);
+        zp = z;
+    }
+    B.sw = sw;
+    B.np = np;
+    B.z1 = w.zc(1);
+    B.hb = (zp - B.z1) / (double)(np - 1);
+    asc = asc && B.hb > 0.0;
+    B.rh = 1.0 / B.hb;
+    B.serr = A.serr;
+    const double r = A.serr / B.hb;
+    B.r2 = r * r;
+    w.y(1) = w.kh(1);
+    w.y(np) = w.kh(sw);
+    int j = 0;
+    double m = 0.0, b = 0.0;
+    for (int i = 2; i <= np - 1; i++) {
+        const double x = B.z1 + (double)(i - 1) * B.hb;
+        const int jn = b_bracket(w, sw, asc, max(j, 1), x);
+        if (jn != j) {
+            j = jn;
+            m = (w.kh(j) - w.kh(j + 1)) / (w.zc(j) - w.zc(j + 1));
+            b = w.kh(j) - m * w.zc(j);
+        }
+        w.y(i) = m * x + b;
+    }
+}
+
+// chol1d's sum S(p) = sum qu^2 dy^2 and smooth's utru (which the search needs
+// at p = 0) from one forward sweep, with nothing stored and no back
+// substitution.  With M(p) = 6(1-p) T + p R the matrix of chol1d and b = Q'y,
+// phi(p) = b'M^-1 b = sum_i w_i^2 / d_i over the forward-substituted values w
+// and the pivots d; u'Mu = phi and dphi/dp = -u'M'u = 6 u'Tu - u'Ru, so that
+//   S = u'Tu = (phi + p phi') / 6,   at p = 0:  utru = u'Ru / 2 = (phi - phi') / 2,
+// and phi' is carried through the sweep as derivatives in p of the factor and
+// of w.  A row is one chain (pivot, reciprocal, ratio, pivot).
+template <class W>
+__device__ __forceinline__ void b_light(const W& w, const BPar& B, double p, double& sum, double& utru) {
+    const int np = B.np;
+    double D, E, F;
+    B.bands(p, D, E, F);
+    const double Dd = -36.0 * B.r2 + 4.0 * B.hb, Ed = 24.0 * B.r2 + B.hb, Fd = -6.0 * B.r2;
+    double a1 = D, a2 = E, b1 = D, a1d = Dd, a2d = Ed, b1d = Dd;
+    double y0 = w.y(2), yp = w.y(3);
+    double wc = (yp - 2.0 * y0 + w.y(1)) * B.rh, wcd = 0.0, wp = 0.0, wpd = 0.0;   // w(i), w(i-1) and d/dp
+    double r2p = 0.0, r2pd = 0.0;                                                  // ratio2(i-1)
+    double phi = 0.0, phid = 0.0;
+    auto row = [&](double yn, double Fi, double Fid) {
+        const double inv = rp_rcp_ulp(a1);
+        const double invd = -(a1d * inv) * inv;
+        const double wi = wc * inv;
+        phi = fma(wc, wi, phi);
+        phid = fma(2.0 * wcd, wi, fma(wc * wc, invd, phid));
+        const double q1 = a2 * inv, q1d = fma(a2d, inv, a2 * invd);
+        const double q2 = Fi * inv, q2d = fma(Fid, inv, Fi * invd);
+        const double a1n = fma(-q1, a2, b1);
+        const double a1dn = fma(-q1d, a2, fma(-q1, a2d, b1d));
+        a2 = fma(-q1, Fi, E);
+        a2d = fma(-q1d, Fi, fma(-q1, Fid, Ed));
+        b1 = fma(-q2, Fi, D);
+        b1d = fma(-q2d, Fi, fma(-q2, Fid, Dd));
+        a1 = a1n;
+        a1d = a1dn;
+        const double qn = (yn - 2.0 * yp + y0) * B.rh;                             // qty(i+1)
+        y0 = yp;
+        yp = yn;
+        const double wn = fma(-r2p, wp, fma(-q1, wc, qn));
+        const double wnd = -fma(q1d, wc, fma(q1, wcd, fma(r2pd, wp, r2p * wpd)));
+        wp = wc;
+        wpd = wcd;
+        wc = wn;
+        wcd = wnd;
+        r2p = q2;
+        r2pd = q2d;
+    };
+    int i = 2;
+#pragma unroll 1
+    for (; i + 3 <= np - 3; i += 4) {            // the rows' data read together
+        const double ya = w.y(i + 2), yb = w.y(i + 3), yc = w.y(i + 4), yd = w.y(i + 5);
+        row(ya, F, Fd);
+        row(yb, F, Fd);
+        row(yc, F, Fd);
+        row(yd, F, Fd);
+    }
+#pragma unroll 1
+    for (; i <= np - 2; i++) row(w.y(i + 2), i <= np - 3 ? F : 0.0, i <= np - 3 ? Fd : 0.0);
+    {                                                                              // row np-1
+        const double inv = rp_rcp_ulp(a1);
+        const double invd = -(a1d * inv) * inv;
+        const double wi = wc * inv;
+        phi = fma(wc, wi, phi);
+        phid = fma(2.0 * wcd, wi, fma(wc * wc, invd, phid));
+    }
+    sum = fma(p, phid, phi) * (1.0 / 6.0);
+    utru = 0.5 * (phi - phid);
+}
+
+// smooth()'s secant search for p (pppack.f90:5108-5317, reference cold
+// start) on uniform breaks
+template <class W>
+__device__ __forceinline__ double b_find_p(const W& w, const BPar& B, double s, int max_iter, uint32_t& fl) {
+    if (s <= 0.0) return 1.0;
+    const double ooss = 1.0 / sqrt(s);
+    double q = 0.0, prevq = 0.0, prevsf = 0.0;
+#pragma unroll 1
+    for (int it = 0;; it++) {
+        const double p = q / (1.0 + q);
+        double sum, utru;
+        b_light(w, B, p, sum, utru);
+        const double sfq = 36.0 * sum / ((1.0 + q) * (1.0 + q));
+        const double oosf = 1.0 / sqrt(sfq);
+        if (it == 0) {
+            if (!(s < sfq)) return 0.0;
+            q = -(oosf - ooss) * sfq / (6.0 * utru * oosf);
+        } else {
+            if (fabs(sfq - s) <= 0.01 * s) return p;
+            if (it >= max_iter) {
+                fl |= RP_FL_SPLINE;
+                return p;
+            }
+            const double change = (q - prevq) / (oosf - prevsf) * (oosf - ooss);
+            prevq = q;
+            q = q - change;
+        }
+        prevsf = oosf;
+    }
+}
+
+// chol1d (pppack.f90:1428-1566) at p; leaves u(1..np), the ratios and, REV,
+// the pivots' reciprocals
+template <bool REV, class W>
+__device__ __forceinline__ void b_solve(const W& w, const BPar& B, double p) {
+    const int np = B.np;
+    double D, E, F;
+    B.bands(p, D, E, F);
+    double a1 = D, a2 = E, b1 = D;
+    double y0 = w.y(2), yp = w.y(3);
+    double uc = (yp - 2.0 * y0 + w.y(1)) * B.rh, up = 0.0, r2p = 0.0;
+    auto row = [&](int i, double yn, double Fi) {
+        const double inv = rp_rcp_ulp(a1);
+        const double q1 = a2 * inv, q2 = Fi * inv;
+        w.s1(i) = q1;
+        w.s2(i) = q2;
+        w.u(i) = uc * inv;
+        if (REV) w.inv(i) = inv;
+        a1 = fma(-q1, a2, b1);
+        a2 = fma(-q1, Fi, E);
+        b1 = fma(-q2, Fi, D);
+        const double qn = (yn - 2.0 * yp + y0) * B.rh;
+        y0 = yp;
+        yp = yn;
+        const double un = fma(-r2p, up, fma(-q1, uc, qn));
+        up = uc;
+        uc = un;
+        r2p = q2;
+    };
+    int i = 2;
+#pragma unroll 1
+    for (; i + 3 <= np - 3; i += 4) {
+        const double ya = w.y(i + 2), yb = w.y(i + 3), yc = w.y(i + 4), yd = w.y(i + 5);
+        row(i, ya, F);
+        row(i + 1, yb, F);
+        row(i + 2, yc, F);
+        row(i + 3, yd, F);
+    }
+#pragma unroll 1
+    for (; i <= np - 2; i++) row(i, w.y(i + 2), i <= np - 3 ? F : 0.0);
+    const double inv = rp_rcp_ulp(a1);
+    if (REV) w.inv(np - 1) = inv;
+    double u2 = 0.0, u1 = uc * inv;              // u(i+2), u(i+1)
+    w.u(np) = 0.0;
+    w.u(np - 1) = u1;
+    w.u(1) = 0.0;
+    i = np - 2;
+#pragma unroll 1
+    for (; i - 3 >= 2; i -= 4) {                 // four rows' values read together
+        double v[4], q1[4], q2[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            v[k] = w.u(i - k);
+            q1[k] = w.s1(i - k);
+            q2[k] = w.s2(i - k);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const double ui = fma(-u1, q1[k], fma(-u2, q2[k], v[k]));
+            w.u(i - k) = ui;
+            u2 = u1;
+            u1 = ui;
+        }
+    }
+    for (; i >= 2; i--) {
+        const double ui = fma(-u1, w.s1(i), fma(-u2, w.s2(i), w.u(i)));
+        w.u(i) = ui;
+        u2 = u1;
+        u1 = ui;
+    }
+}
+
+// ppvalu's piece at x (a_ppvalu's terms)
+struct BPiece {
+    int i;
+    double hx, c1, c2, c3, c4, a1n, a3n, d0, d1, d2;   // d: u(i)-u(i-1), u(i+1)-u(i), u(i+2)-u(i+1)
+};
+template <class W>
+__device__ __forceinline__ BPiece b_piece(const W& w, const BPar& B, double p, double x) {
+    BPiece c;
+    const int np = B.np;
+    const double t = floor((x - B.z1) * B.rh);
+    const int i = (t >= 0.0 && t < (double)(np - 1)) ? (int)t + 1 : ((t >= (double)(np - 1)) ? np - 1 : 1);
+    const double u0 = w.u(i), u1 = w.u(i + 1);
+    c.i = i;
+    c.d0 = (i >= 2) ? u0 - w.u(i - 1) : 0.0;
+    c.d1 = u1 - u0;
+    c.d2 = (i + 2 <= np) ? w.u(i + 2) - u1 : 0.0;
+    const double K1 = 6.0 * (1.0 - p) * B.serr * B.serr;
+    c.c1 = w.y(i) - K1 * ((c.d1 - c.d0) * B.rh);
+    c.a1n = w.y(i + 1) - K1 * ((c.d2 - c.d1) * B.rh);
+    c.c3 = u0 * (6.0 * p);
+    c.a3n = u1 * (6.0 * p);
+    c.c4 = (c.a3n - c.c3) * B.rh;
+    c.c2 = (c.a1n - c.c1) * B.rh - (c.c3 + c.c4 * (1.0 / 3.0) * B.hb) * 0.5 * B.hb;
+    c.hx = x - (B.z1 + (double)(i - 1) * B.hb);
+    return c;
+}
+__device__ __forceinline__ double b_value(const BPiece& c) {
+    return ((c.c4 * (1.0 / 3.0) * c.hx + c.c3) * 0.5 * c.hx + c.c2) * c.hx + c.c1;
+}
+__device__ __forceinline__ double b_slope(const BPiece& c) { return (c.c4 * 0.5 * c.hx + c.c3) * c.hx + c.c2; }
+
+// adjoint g of the piece's value (DERIV: of its slope) to x (returned), u, y,
+// the spacing and the first break
+template <bool DERIV, class W>
+__device__ __forceinline__ double b_piece_rev(const W& w, const BPar& B, double p, const BPiece& c, double g,
+                                              double& hbb, double& z1b) {
+    const int np = B.np, i = c.i;
+    const double hx = c.hx, hb = B.hb, rh = B.rh;
+    const double xb = g * (DERIV ? c.c4 * hx + c.c3 : b_slope(c));
+    double a1b = DERIV ? 0.0 : g, a2b = DERIV ? g : g * hx;
+    double a3b = DERIV ? g * hx : g * 0.5 * hx * hx;
+    double a4b = DERIV ? g * 0.5 * hx * hx : g * (1.0 / 6.0) * hx * hx * hx;
+    double rhb = a2b * (c.a1n - c.c1);
+    double a1nb = a2b * rh;
+    a1b -= a2b * rh;
+    hbb -= a2b * (0.5 * c.c3 + c.c4 * hb * (1.0 / 3.0));
+    a3b -= 0.5 * hb * a2b;
+    a4b -= hb * hb * (1.0 / 6.0) * a2b;
+    const double a3nb = a4b * rh;
+    a3b -= a4b * rh;
+    rhb += a4b * (c.a3n - c.c3);
+    const double K1 = 6.0 * (1.0 - p) * B.serr * B.serr;
+    const double r0b = K1 * a1b, r1b = K1 * (a1nb - a1b), r2b = -K1 * a1nb;       // of raw(i), raw(i+1), raw(i+2)
+    rhb += r0b * c.d0 + r1b * c.d1 + r2b * c.d2;
+    if (i >= 2) w.ub(i - 1) -= r0b * rh;
+    w.ub(i) += ((i >= 2 ? r0b : 0.0) - r1b) * rh + 6.0 * p * a3b;
+    w.ub(i + 1) += (r1b - (i + 2 <= np ? r2b : 0.0)) * rh + 6.0 * p * a3nb;
+    if (i + 2 <= np) w.ub(i + 2) += r2b * rh;
+    w.yb(i) += a1b;
+    w.yb(i + 1) += a1nb;
+    hbb -= rhb * rh * rh + xb * (double)(i - 1);
+    z1b -= xb;
+    return xb;
+}
+
+// One sub-step of the random walk (ver_turb_module.f90:231-293) from z
+struct BSub {
+    bool in1, in2, bot, top;       // slope taken; diffusivity taken from the fit; reflected
+    double kz, z3, sd, z;          // slope times deltat, z3, sqrt(2 K deltat), the new position
+    BPiece c1, c2;
+};
+template <class W>
+__device__ __forceinline__ BSub b_sub(const W& w, const BPar& B, const RpStepArgs& A, double p, double tdepth,
+                                      double zeta, double z, double dev) {
+    BSub s;
+    s.in1 = !(z <= tdepth || z >= zeta);
+    double kp = 0.0;
+    if (s.in1) {
+        s.c1 = b_piece(w, B, p, z);
+        kp = b_slope(s.c1);
+    }
+    s.kz = kp * A.deltat;
+    s.z3 = z + 0.5 * s.kz;
+    s.in2 = !(s.z3 < tdepth || s.z3 > zeta);
+    double K = A.aksback;
+    if (s.in2) {
+        s.c2 = b_piece(w, B, p, s.z3);
+        K = b_value(s.c2);
+        if (K < A.aksback) {
+            K = A.aksback;
+            s.in2 = false;
+        }
+    }
+    s.sd = sqrt(2.0 * K * A.deltat);
+    double n = z + (s.kz + dev * s.sd);
+    s.bot = n <= tdepth && n - tdepth < 0.0;
+    if (n <= tdepth) n = tdepth + fabs(n - tdepth);
+    s.top = n >= zeta;
+    if (s.top) n = zeta - fabs(n - zeta);
+    s.z = n;
+    return s;
+}
+
+// RK stage 1's 2-D quantities and the z clamp find_currents applies there
+// (advection_module.f90:171-183)
+template <class S>
+__device__ __forceinline__ void b_stage(const RpStepArgs& A, const AdjFrames& F, int gi, const S& X, const S& Y,
+                                        AStage<S>& St, uint32_t& fl) {
+    a_rho_cell(A.g[gi], X, Y, St.rc, fl);
+    a_stage_2d(A, F, gi, A.g[gi], St);
+}
+
+// VTurb's displacement; find: p is searched and returned, else given
+template <class W>
+__device__ __forceinline__ double b_vturb(const RpStepArgs& A, const AdjFrames& F, int gi, double X, double Y,
+                                          double Z, double kappa, uint32_t pid, bool find, double& p, uint32_t& fl,
+                                          const W& w) {
+    AStage<double> St;
+    b_stage(A, F, gi, X, Y, St, fl);
+    if (A.scheme == 1) {
+        if (Z < St.tdepth) Z = St.tdepth + RP_F_0P001;
+        if (Z > St.zeta) Z = St.zeta - RP_F_0P001;
+    }
+    BPar B;
+    bool asc;
+    b_column(A, F, gi, St, kappa, w, B, asc);
+    if (find) p = b_find_p(w, B, A.smth, A.spline_max_iter, fl);
+    b_solve<false>(w, B, p);
+    double z = Z, dev, dev_next = 0.0;
+#pragma unroll 1
+    for (int i = 1; i <= A.loop; i++) {
+        if (i & 1) rp_normal2(A, pid, (uint32_t)(1 + i), i < A.loop, dev, dev_next);
+        else dev = dev_next;
+        z = b_sub(w, B, A, p, St.tdepth, St.zeta, z, dev).z;
+    }
+    return z - Z;
+}
+
+// VTurb's displacement t[0] and its derivatives t[1..4] in the start's x, y, z
+// and in kappa, at the recorded p; A.loop <= NPMAX
+template <class W>
+__device__ __forceinline__ void b_vturb_rev(const RpStepArgs& A, const AdjFrames& F, int gi, double X, double Y,
+                                            double Z, double kappa, uint32_t pid, double p, uint32_t& fl, const W& w,
+                                            double t[5]) {
+    BPar B;
+    bool asc;
+    int clamp = 0;                 // stage 1's z: 1 put on the bottom, 2 under the surface
+    double hbb = 0.0, z1b = 0.0, tdb = 0.0, zeb = 0.0;   // adjoints of hb, z1, tdepth, zeta
+    double zb = 1.0;                                     // of the position
+    {
+        AStage<double> St;
+        b_stage(A, F, gi, X, Y, St, fl);
+        if (A.scheme == 1) {
+            if (Z < St.tdepth) {
+                Z = St.tdepth + RP_F_0P001;
+                clamp = 1;
+            }
+            if (Z > St.zeta) {
+                Z = St.zeta - RP_F_0P001;
+                clamp = 2;
+            }
+        }
+        b_column(A, F, gi, St, kappa, w, B, asc);
+        b_solve<true>(w, B, p);
+        for (int i = 1; i <= B.np; i++) {
+            w.ub(i) = 0.0;
+            w.yb(i) = 0.0;
+        }
+        double z = Z, dev = 0.0, dev_next = 0.0;
+#pragma unroll 1
+        for (int i = 1; i <= A.loop; i++) {
+            if (i & 1) rp_normal2(A, pid, (uint32_t)(1 + i), i < A.loop, dev, dev_next);
+            else dev = dev_next;
+            w.zt(i) = z;
+            w.dev(i) = dev;
+            z = b_sub(w, B, A, p, St.tdepth, St.zeta, z, dev).z;
+        }
+        t[0] = z - Z;
+#pragma unroll 1
+        for (int i = A.loop; i >= 1; i--) {
+            const double zi = w.zt(i), d = w.dev(i);
+            const BSub s = b_sub(w, B, A, p, St.tdepth, St.zeta, zi, d);
+            if (s.top) {
+                zeb += 2.0 * zb;
+                zb = -zb;
+            }
+            if (s.bot) {
+                tdb += 2.0 * zb;
+                zb = -zb;
+            }
+            double kzb = zb;
+            if (s.in2) {
+                const double Kb = zb * d * ((s.sd > 0.0) ? 0.5 / s.sd : 0.0) * 2.0 * A.deltat;
+                const double z3b = b_piece_rev<false>(w, B, p, s.c2, Kb, hbb, z1b);
+                zb += z3b;
+                kzb += 0.5 * z3b;
+            }
+            if (s.in1) zb += b_piece_rev<true>(w, B, p, s.c1, kzb * A.deltat, hbb, z1b);
+        }
+    }
+    const int np = B.np, sw = B.sw;
+    // lambda = M^-1 ub by the fit's factor; u(1) = u(np) = 0
+    {
+        double w1 = 0.0, w2 = 0.0, q1 = 0.0, q2 = 0.0, q2p = 0.0;   // w(i-1), w(i-2), ratio1(i-1), ratio2(i-1), (i-2)
+        for (int i = 2; i <= np - 1; i++) {
+            const double wi = fma(-q2p, w2, fma(-q1, w1, w.ub(i)));
+            w.ub(i) = wi * w.inv(i);
+            w2 = w1;
+            w1 = wi;
+            q2p = q2;
+            if (i <= np - 2) {
+                q1 = w.s1(i);
+                q2 = w.s2(i);
+            }
+        }
+        double l2 = 0.0, l1 = w.ub(np - 1);
+        for (int i = np - 2; i >= 2; i--) {
+            const double li = fma(-l1, w.s1(i), fma(-l2, w.s2(i), w.ub(i)));
+            w.ub(i) = li;
+            l2 = l1;
+            l1 = li;
+        }
+        w.ub(1) = 0.0;
+        w.ub(np) = 0.0;
+    }
+    // bands and right-hand side in hb, then the data: b(i) = (y(i+1) - 2 y(i) + y(i-1)) / hb
+    {
+        const double six1mp = 6.0 * (1.0 - p), dr2 = -2.0 * B.r2 * B.rh;
+        const double Dh = six1mp * 6.0 * dr2 + 4.0 * p, Eh = six1mp * -4.0 * dr2 + p, Fh = six1mp * dr2;
+        double sD = 0.0, sE = 0.0, sF = 0.0, sB = 0.0;
+        double lm2 = 0.0, lm1 = 0.0, um2 = 0.0, um1 = 0.0;
+        for (int i = 2; i <= np - 1; i++) {
+            const double l = w.ub(i), u = w.u(i);
+            sD = fma(l, u, sD);
+            sE = fma(l, um1, fma(lm1, u, sE));
+            sF = fma(l, um2, fma(lm2, u, sF));
+            sB = fma(l, (w.y(i + 1) - 2.0 * w.y(i) + w.y(i - 1)) * B.rh, sB);
+            lm2 = lm1;
+            lm1 = l;
+            um2 = um1;
+            um1 = u;
+        }
+        hbb -= Dh * sD + Eh * sE + Fh * sF + sB * B.rh;
+        for (int i = 1; i <= np; i++) {
+            const double lp = (i < np) ? w.ub(i + 1) : 0.0, lm = (i > 1) ? w.ub(i - 1) : 0.0;
+            w.yb(i) += (lp - 2.0 * w.ub(i) + lm) * B.rh;
+        }
+    }
+    // the resampling: y(i) = K(j) + m (x - z(j)), x = z1 + (i-1) hb
+    for (int k = 1; k <= sw; k++) {
+        w.zcb(k) = 0.0;
+        w.khb(k) = 0.0;
+    }
+    w.khb(1) += w.yb(1);
+    w.khb(sw) += w.yb(np);
+    {
+        int j = 0;
+        double m = 0.0, rz = 0.0, z0 = 0.0;
+        for (int i = 2; i <= np - 1; i++) {
+            const double x = B.z1 + (double)(i - 1) * B.hb, g = w.yb(i);
+            const int jn = b_bracket(w, sw, asc, max(j, 1), x);
+            if (jn != j) {
+                j = jn;
+                z0 = w.zc(j);
+                rz = 1.0 / (z0 - w.zc(j + 1));
+                m = (w.kh(j) - w.kh(j + 1)) * rz;
+            }
+            const double gm = g * m, mb = g * (x - z0) * rz;
+            z1b += gm;
+            hbb += (double)(i - 1) * gm;
+            w.khb(j) += g + mb;
+            w.khb(j + 1) -= mb;
+            w.zcb(j) -= gm + mb * m;
+            w.zcb(j + 1) += mb * m;
+        }
+    }
+    const double hr = hbb / (double)(np - 1);
+    w.zcb(sw) += hr;
+    w.zcb(1) += z1b - hr;
+    // the column and the 2-D quantities in x and y, and K in kappa
+    Dual<2> DX(X), DY(Y);
+    DX.d[0] = 1.0;
+    DY.d[1] = 1.0;
+    AStage<Dual<2>> St;
+    b_stage(A, F, gi, DX, DY, St, fl);
+    // Z of the clamp: t = z - Z
+    const double Zb = zb - 1.0;
+    if (clamp == 1) tdb += Zb;
+    if (clamp == 2) zeb += Zb;
+    double gx = tdb * St.tdepth.d[0] + zeb * St.zeta.d[0], gy = tdb * St.tdepth.d[1] + zeb * St.zeta.d[1], gk = 0.0;
+#pragma unroll 1
+    for (int k = 1; k <= sw; k++) {
+        Dual<2> z, K;
+        b_level(A, F, gi, St, k, z, K);
+        const double zk = w.zcb(k), kk = w.khb(k);
+        gx += zk * z.d[0] + kk * (kappa * K.d[0]);
+        gy += zk * z.d[1] + kk * (kappa * K.d[1]);
+        gk += kk * K.v;
+    }
+    t[1] = gx;
+    t[2] = gy;
+    t[3] = (clamp == 0) ? Zb : 0.0;
+    t[4] = gk;
+}
+
 // ----------------------------------------------------------- one step
 
 // The state a step carries besides (x, y, z).
@@ -598,13 +1155,20 @@ struct AdjAux {
     int8_t isin;
 };
 
+// Skip tests of update_particles (ROMSPath.f90:672-690)
+__device__ __forceinline__ bool a_active(const RpStepArgs& A, double dob, double status, int8_t isin) {
+    return !(A.ix[2] <= dob || status == 9.0 || (A.oob && !isin));
+}
+
 // One particle-step of the model (ROMSPath.f90:672-892) from (X, Y, Z) with
-// auxiliary state `a`; updates X, Y, Z, a.  find: search p and return it;
-// else use p.
-template <class S, int NPMAX>
-__device__ void a_step(const RpStepArgs& A, const AdjFrames& F, double dob, uint32_t pid, S& X, S& Y, S& Z, AdjAux& a,
-                       const S& kappa, bool find, double& p, uint32_t& fl, const AFit<S, NPMAX>& w) {
-    if (A.ix[2] <= dob || a.status == 9.0 || (A.oob && !a.isin)) return;      // ROMSPath.f90:672-690
+// auxiliary state `a`; updates X, Y, Z, a.  vturb(St, have_s1, Zpar) is VTurb's
+// displacement (S1: RK stage 1's quantities where have_s1), called with VTurb
+// on.  Returns the sign the new Z carries VTurb's displacement with (0: not at
+// all).
+template <class S, class V>
+__device__ __forceinline__ int a_step(const RpStepArgs& A, const AdjFrames& F, double dob, uint32_t pid, S& X, S& Y,
+                                      S& Z, AdjAux& a, uint32_t& fl, V&& vturb) {
+    if (!a_active(A, dob, a.status, a.isin)) return 0;
     a.age = a.age + (double)(float)A.idt;
     int gid = a.gid;
     const int gi = gid - 1;
@@ -657,13 +1221,7 @@ __device__ void a_step(const RpStepArgs& A, const AdjFrames& F, double dob, uint
         TurbHy = rp_normal(A, pid, 1u) * sc * pn;
     }
     S TurbV(0.0);
-    if (A.vturb_on) {
-        if (!have_s1) {
-            a_rho_cell(g, Xpar, Ypar, S1.rc, fl);
-            a_stage_2d(A, F, gi, g, S1);
-        }
-        TurbV = a_vturb(A, F, gi, S1, Zpar, kappa, pid, find, p, fl, w);
-    }
+    if (A.vturb_on) TurbV = vturb(S1, have_s1, Zpar);
     // new position and hand-off (ROMSPath.f90:821-836)
     const S newX = X + AdvectX + TurbHx;
     const S newY = Y + AdvectY + TurbHy;
@@ -692,11 +1250,13 @@ __device__ void a_step(const RpStepArgs& A, const AdjFrames& F, double dob, uint
     } else {
         newZ = tdepth + A.vertdist;
     }
+    int vsign = 0;
     if (ingrid) {                                         // 874-892
         a.isin = 1;
         X = tX;
         Y = tY;
         Z = newZ;
+        if (A.nsb == 0) vsign = (hbot != htop) ? -1 : 1;
         double st = 1.0;
         if (htop) st = RP_F_1P1;
         if (hbot) st = RP_F_1P2;
@@ -710,4 +1270,5 @@ __device__ void a_step(const RpStepArgs& A, const AdjFrames& F, double dob, uint
         a.isin = 1;
         a.status = -9.0;
     }
+    return vsign;
 }

@@ -128,7 +128,7 @@ struct rp_ctx {
         double* prec = nullptr;                // recorded p: nsteps x n
         double* seg = nullptr;                 // one segment of step-start states: ckpt blocks
         double* work = nullptr;                // working state block
-        double *lx = nullptr, *ly = nullptr, *lz = nullptr, *kbar = nullptr, *tan = nullptr;
+        double *lx = nullptr, *ly = nullptr, *lz = nullptr, *kbar = nullptr, *tan = nullptr, *tv = nullptr;
         size_t cap_steps = 0;
     } adj;
     int64_t launches = 0;
@@ -346,7 +346,7 @@ void free_ctx(rp_ctx* c) {
                     c->dstage[0], c->dstage[1], c->x32, c->y32, c->z32, c->cx, c->cy, c->cz, c->qwarm, c->gwarm, c->qwarm2,
                     c->ftmp, c->qmax, c->sb.keys, c->sb.hist, c->sb.sums, c->sb.perm, c->sb.gbase,
                     c->adj.ck, c->adj.prec, c->adj.seg, c->adj.work, c->adj.lx, c->adj.ly, c->adj.lz,
-                    c->adj.kbar, c->adj.tan, c->d_salt, c->d_temp, c->d_mean_salt, c->d_mean_temp,
+                    c->adj.kbar, c->adj.tan, c->adj.tv, c->d_salt, c->d_temp, c->d_mean_salt, c->d_mean_temp,
                     c->d_hob, c->d_bustr, c->d_bvstr, c->outbuf, c->wd_stage, c->b_acc, c->b_vort,
                     c->b_behavew, c->b_ssf, c->d_spl};
     for (int g = 0; g < RP_MAXNGRID; g++)
@@ -549,8 +549,9 @@ int sort_buffers(rp_ctx* ctx) {
 
 // An adjoint state block: x, y, z, age, status (doubles), gid (int32),
 // isin (int8) for n particles, laid out in one allocation of
-// adj_block_bytes(n).
-size_t adj_block_bytes(int64_t n) { return (size_t)n * (5 * 8 + 4 + 1) + 64; }
+// adj_block_bytes(n), a multiple of the columns' alignment so that blocks can
+// follow one another for any n.
+size_t adj_block_bytes(int64_t n) { return ((size_t)n * (5 * 8 + 4 + 1) + 255) / 256 * 256; }
 
 rp::AdjStateDev adj_view(void* base, int64_t n) {
     rp::AdjStateDev s;
@@ -1565,13 +1566,13 @@ int rp_forward(rp_ctx* ctx, int32_t nsteps, const rp_adj_step* steps, double kap
     const int nseg = (nsteps + checkpoint_every - 1) / checkpoint_every;
     const size_t blk = adj_block_bytes(n);
     // (re)allocate for this run
-    double* bufs[] = {J.ck, J.prec, J.seg, J.work, J.lx, J.ly, J.lz, J.kbar, J.tan};
+    double* bufs[] = {J.ck, J.prec, J.seg, J.work, J.lx, J.ly, J.lz, J.kbar, J.tan, J.tv};
     for (double* b : bufs) if (b) cudaFree(b);
-    J.ck = J.prec = J.seg = J.work = J.lx = J.ly = J.lz = J.kbar = J.tan = nullptr;
+    J.ck = J.prec = J.seg = J.work = J.lx = J.ly = J.lz = J.kbar = J.tan = J.tv = nullptr;
     if (dalloc(&J.ck, blk * (size_t)(nseg + 1)) || dalloc(&J.prec, (size_t)nsteps * n * 8) ||
         dalloc(&J.seg, blk * (size_t)checkpoint_every) || dalloc(&J.work, blk) || dalloc(&J.lx, (size_t)n * 8) ||
         dalloc(&J.ly, (size_t)n * 8) || dalloc(&J.lz, (size_t)n * 8) || dalloc(&J.kbar, (size_t)n * 8) ||
-        dalloc(&J.tan, (size_t)n * 12 * 8))
+        dalloc(&J.tan, (size_t)n * 12 * 8) || dalloc(&J.tv, (size_t)n * 5 * 8))
         return fail(ctx, RP_ERR_NOMEM, "rp_forward: checkpoint / record allocation");
     J.steps.assign(steps, steps + nsteps);
     J.ckpt = checkpoint_every;
@@ -1585,7 +1586,7 @@ int rp_forward(rp_ctx* ctx, int32_t nsteps, const rp_adj_step* steps, double kap
         RpStepArgs A;
         AdjFrames F;
         adj_args(ctx, J.steps[k], A, F, n);
-        CK(rp::launch_adj(0, A, F, cur, J.prec + (size_t)k * n, 1, kappa, nullptr, nullptr, nullptr, nullptr, nullptr,
+        CK(rp::launch_adj(0, A, F, cur, J.prec + (size_t)k * n, 1, kappa, J.tv, nullptr, nullptr, nullptr, nullptr, nullptr,
                           ctx->npmax, s, ctx->num_sms));
         ctx->launches++;
     }
@@ -1621,8 +1622,8 @@ int rp_backward(rp_ctx* ctx, const double* dL_dx, const double* dL_dy, const dou
                 RpStepArgs A;
                 AdjFrames F;
                 adj_args(ctx, J.steps[k], A, F, n);
-                CK(rp::launch_adj(0, A, F, work, J.prec + (size_t)k * n, 0, J.kappa, nullptr, nullptr, nullptr, nullptr,
-                                  nullptr, ctx->npmax, s, ctx->num_sms));
+                CK(rp::launch_adj(0, A, F, work, J.prec + (size_t)k * n, 0, J.kappa, J.tv, nullptr, nullptr, nullptr,
+                                  nullptr, nullptr, ctx->npmax, s, ctx->num_sms));
                 ctx->launches++;
             }
         }
@@ -1632,7 +1633,7 @@ int rp_backward(rp_ctx* ctx, const double* dL_dx, const double* dL_dy, const dou
             AdjFrames F;
             adj_args(ctx, J.steps[k], A, F, n);
             CK(rp::launch_adj(2, A, F, adj_view((char*)J.seg + blk * (size_t)(k - k0), n), J.prec + (size_t)k * n, 0,
-                              J.kappa, nullptr, J.lx, J.ly, J.lz, J.kbar, ctx->npmax, s, ctx->num_sms));
+                              J.kappa, J.tv, nullptr, J.lx, J.ly, J.lz, J.kbar, ctx->npmax, s, ctx->num_sms));
             ctx->launches++;
         }
     }
@@ -1668,7 +1669,7 @@ int rp_adj_replay(rp_ctx* ctx, const double* x0, const double* y0, const double*
         RpStepArgs A;
         AdjFrames F;
         adj_args(ctx, J.steps[k], A, F, n);
-        CK(rp::launch_adj(0, A, F, work, J.prec + k * n, 0, kappa, nullptr, nullptr, nullptr, nullptr, nullptr,
+        CK(rp::launch_adj(0, A, F, work, J.prec + k * n, 0, kappa, J.tv, nullptr, nullptr, nullptr, nullptr, nullptr,
                           ctx->npmax, s, ctx->num_sms));
         ctx->launches++;
     }
@@ -1692,7 +1693,7 @@ int rp_tangent(rp_ctx* ctx, double kappa, double* jac) {
         RpStepArgs A;
         AdjFrames F;
         adj_args(ctx, J.steps[k], A, F, n);
-        CK(rp::launch_adj(1, A, F, work, J.prec + k * n, 0, kappa, J.tan, nullptr, nullptr, nullptr, nullptr,
+        CK(rp::launch_adj(1, A, F, work, J.prec + k * n, 0, kappa, J.tv, J.tan, nullptr, nullptr, nullptr, nullptr,
                           ctx->npmax, s, ctx->num_sms));
         ctx->launches++;
     }
