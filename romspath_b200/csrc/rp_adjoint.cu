@@ -12,6 +12,9 @@ namespace rp {
 
 constexpr int kAdjBlock = 128;
 constexpr int kAdjVtBlock = 64;
+constexpr int kAdjStepBlocks = 4;      // blocks of the steps in doubles and in dual numbers an SM
+constexpr int kAdjReverseBlocks = 3;
+
 
 __device__ __forceinline__ void adj_load(const AdjStateDev& s, int64_t n, double& x, double& y, double& z,
                                          AdjAux& a) {
@@ -38,7 +41,7 @@ __device__ __forceinline__ void adj_store_aux(const AdjStateDev& s, int64_t n, c
 // reciprocal, the next pivot): 64-thread blocks, eight an SM, hold 65,536
 // particles in one wave; the search's seven or so passes store nothing.  On the
 // 130x98x20 grid with 65,536 particles a forward step (this kernel and the
-// rest) takes 0.40 ms, 1.5 in one kernel whose passes kept their factor and
+// rest) takes 0.29 ms, 1.5 in one kernel whose passes kept their factor and
 // divided three times a row.
 template <int NPMAX>
 __global__ void __launch_bounds__(kAdjVtBlock, 512 / kAdjVtBlock)
@@ -48,7 +51,8 @@ __global__ void __launch_bounds__(kAdjVtBlock, 512 / kAdjVtBlock)
     double buf[W::kArrays * (NPMAX + 1)];
     const W w{buf};
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < A.p.n; n += stride) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < A.p.n; i += stride) {
+        const int64_t n = s.order ? s.order[i] : i;
         double p = find ? 0.0 : prec[n], t = 0.0;
         uint32_t fl = 0;
         if (a_active(A, A.p.dob[n], s.status[n], s.isin[n]))
@@ -60,7 +64,7 @@ __global__ void __launch_bounds__(kAdjVtBlock, 512 / kAdjVtBlock)
 
 // The same with its derivatives in the start's x, y, z and in kappa: tv[q n],
 // q = 0..4 (b_vturb_rev).  A reverse step (this kernel and k_adj_reverse) on
-// the workload above takes 0.9 ms, 1.9 with the fit carried in dual numbers.
+// the workload above takes 0.62 ms, 1.9 with the fit carried in dual numbers.
 template <int NPMAX>
 __global__ void __launch_bounds__(kAdjVtBlock, 512 / kAdjVtBlock)
     k_adj_vturb_rev(const __grid_constant__ RpStepArgs A, const __grid_constant__ AdjFrames F, AdjStateDev s,
@@ -69,7 +73,8 @@ __global__ void __launch_bounds__(kAdjVtBlock, 512 / kAdjVtBlock)
     double buf[W::kArrays * (NPMAX + 1)];
     const W w{buf};
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < A.p.n; n += stride) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < A.p.n; i += stride) {
+        const int64_t n = s.order ? s.order[i] : i;
         double t[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
         uint32_t fl = 0;
         if (a_active(A, A.p.dob[n], s.status[n], s.isin[n]))
@@ -80,12 +85,15 @@ __global__ void __launch_bounds__(kAdjVtBlock, 512 / kAdjVtBlock)
 }
 
 // one step of the model in doubles on state s; with VTurb on, tv holds
-// k_adj_vturb's displacements
-__global__ void __launch_bounds__(kAdjBlock) k_adj_step(const __grid_constant__ RpStepArgs A,
+// k_adj_vturb's displacements.  Four stages of gathers; 65,536 particles 64 us
+// at four blocks an SM (one wave) with levels bisected and particles taken by
+// cell, 131 us at three, walked, as they lay.
+__global__ void __launch_bounds__(kAdjBlock, kAdjStepBlocks) k_adj_step(const __grid_constant__ RpStepArgs A,
                                                          const __grid_constant__ AdjFrames F, AdjStateDev s,
                                                          const double* __restrict__ tv) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < A.p.n; n += stride) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < A.p.n; i += stride) {
+        const int64_t n = s.order ? s.order[i] : i;
         double x, y, z;
         AdjAux a;
         adj_load(s, n, x, y, z, a);
@@ -119,7 +127,8 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_tangent(const __grid_constant
     D buf[kAdjArrays * (NPMAX + 1)];
     const AFit<D, NPMAX> w{buf};
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < A.p.n; n += stride) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < A.p.n; i += stride) {
+        const int64_t n = s.order ? s.order[i] : i;
         double x, y, z;
         AdjAux a;
         adj_load(s, n, x, y, z, a);
@@ -155,14 +164,15 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_tangent(const __grid_constant
 // step's Jacobian by dual numbers seeded on (x, y, z), VTurb's row of it from
 // tv (k_adj_vturb_rev); then lambda <- J^T lambda for (x, y, z) and
 // kbar += lambda . d(x,y,z)/dkappa (kappa enters z alone, through VTurb)
-__global__ void __launch_bounds__(kAdjBlock) k_adj_reverse(const __grid_constant__ RpStepArgs A,
+__global__ void __launch_bounds__(kAdjBlock, kAdjReverseBlocks) k_adj_reverse(const __grid_constant__ RpStepArgs A,
                                                             const __grid_constant__ AdjFrames F, AdjStateDev s,
                                                             const double* __restrict__ tv, double* __restrict__ lx,
                                                             double* __restrict__ ly, double* __restrict__ lz,
                                                             double* __restrict__ kbar) {
     using D = Dual<3>;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < A.p.n; n += stride) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < A.p.n; i += stride) {
+        const int64_t n = s.order ? s.order[i] : i;
         double x, y, z;
         AdjAux a;
         adj_load(s, n, x, y, z, a);
@@ -198,7 +208,8 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_reverse_dual(const __grid_con
     D buf[kAdjArrays * (NPMAX + 1)];
     const AFit<D, NPMAX> w{buf};
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < A.p.n; n += stride) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < A.p.n; i += stride) {
+        const int64_t n = s.order ? s.order[i] : i;
         double x, y, z;
         AdjAux a;
         adj_load(s, n, x, y, z, a);

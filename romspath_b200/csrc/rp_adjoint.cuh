@@ -340,6 +340,66 @@ __device__ __forceinline__ S a_col(const double* f, const int64_t o[4], const S 
     return L.z1 * pb + L.z2 * pt;
 }
 
+// The level at index k (1-based) as the picks above compare it, without
+// derivatives and with 1 / (hc + h) formed once
+struct ALevels {
+    double hc, h, rden, zeta;
+    __device__ __forceinline__ double at(const double* s, const double* cs, int k) const {
+        return zeta + (zeta + h) * ((hc * __ldg(s + k - 1) + h * __ldg(cs + k - 1)) * rden);
+    }
+};
+
+// The first of nz ascending levels above zpar (nz + 1: none), by bisection
+__device__ __forceinline__ int a_above(const ALevels& v, const double* s, const double* cs, int nz, double zpar) {
+    int lo = 0, hi = nz + 1;
+#pragma unroll 1
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (v.at(s, cs, mid) > zpar) hi = mid; else lo = mid;
+    }
+    return hi;
+}
+
+template <class S>
+__device__ __forceinline__ void a_bracket(const RpGridDev& g, const double* s, const double* cs, int nz, int i,
+                                          const S& zeta, const S& h, const S& zpar, APick<S>& L) {
+    if (i > nz || i == 1) {
+        L.ibot = L.itop = (i == 1) ? 1 : nz;
+        L.z1 = S(0.5);
+        L.z2 = S(0.5);
+        return;
+    }
+    const S z1 = a_zlev(2, g.hc, __ldg(s + i - 2), __ldg(cs + i - 2), zeta, h);
+    const S z2 = a_zlev(2, g.hc, __ldg(s + i - 1), __ldg(cs + i - 1), zeta, h);
+    const S Z = (zpar - z1) / (z2 - z1);
+    L.ibot = i - 1;
+    L.itop = i;
+    L.z1 = 1.0 - Z;
+    L.z2 = Z;
+}
+
+// Both brackets of getInterp3D.  Where the levels ascend (as in rp_walk2) by
+// bisection on their values: walked level by level with a division each, the
+// two walks were most of a stage.
+template <class S>
+__device__ __forceinline__ void a_walk2(const RpGridDev& g, const S& zeta, const S& depth, const S& zpar, APick<S>& Lr,
+                                        APick<S>& Lw, uint32_t& fl) {
+    const S h = -depth;
+    const double hv = aval(h), zv = aval(zeta), pv = aval(zpar);
+    if (!(g.asc && hv > 0.0 && hv < 1e30 && zv + hv > 0.0 && zv < 1e30 && pv == pv)) {
+        a_walk(g, false, zeta, depth, zpar, Lr, fl);
+        a_walk(g, true, zeta, depth, zpar, Lw, fl);
+        return;
+    }
+    const ALevels v{g.hc, hv, 1.0 / (g.hc + hv), zv};
+    const int N = g.N;
+    a_bracket(g, g.sr, g.csr, N, a_above(v, g.sr, g.csr, N, pv), zeta, h, zpar, Lr);
+    const int iw = a_above(v, g.sw, g.csw, N + 1, pv);
+    if (iw > N + 1) fl |= RP_FL_WTOP;
+    if (iw == 1) fl |= RP_FL_WBOT;
+    a_bracket(g, g.sw, g.csw, N + 1, iw, zeta, h, zpar, Lw);
+}
+
 template <class S>
 struct AStage {
     ARho<S> rc;
@@ -366,8 +426,7 @@ __device__ __forceinline__ void a_find_currents(const RpStepArgs& A, const AdjFr
     if (aval(Z) < aval(St.tdepth)) Z = St.tdepth + RP_F_0P001;
     if (aval(Z) > aval(St.zeta)) Z = St.zeta - RP_F_0P001;
     APick<S> Lr, Lw;
-    a_walk(g, false, St.zeta, St.tdepth, Z, Lr, fl);
-    a_walk(g, true, St.zeta, St.tdepth, Z, Lw, fl);
+    a_walk2(g, St.zeta, St.tdepth, Z, Lr, Lw, fl);
     const int N = g.N;
     S val3[3];
     {
@@ -569,9 +628,9 @@ struct BFit {
     __device__ __forceinline__ double& yb(int i) const { return at(8, i); }    // adjoints of y
     __device__ __forceinline__ double& zt(int i) const { return at(9, i); }    // sub-step i's start and deviate
     __device__ __forceinline__ double& dev(int i) const { return at(10, i); }
-    // adjoints of the column, over the factor once it has been used
-    __device__ __forceinline__ double& zcb(int k) const { return s1(k); }
-    __device__ __forceinline__ double& khb(int k) const { return s2(k); }
+    // adjoints of the column, over the sub-steps once they have been used
+    __device__ __forceinline__ double& zcb(int k) const { return zt(k); }
+    __device__ __forceinline__ double& khb(int k) const { return dev(k); }
 };
 
 // What the passes of a fit share
@@ -846,26 +905,30 @@ struct BPiece {
     int i;
     double hx, c1, c2, c3, c4, a1n, a3n, d0, d1, d2;   // d: u(i)-u(i-1), u(i+1)-u(i), u(i+2)-u(i+1)
 };
-template <class W>
-__device__ __forceinline__ BPiece b_piece(const W& w, const BPar& B, double p, double x) {
-    BPiece c;
-    const int np = B.np;
+__device__ __forceinline__ int b_piece_at(const BPar& B, double x) {
     const double t = floor((x - B.z1) * B.rh);
-    const int i = (t >= 0.0 && t < (double)(np - 1)) ? (int)t + 1 : ((t >= (double)(np - 1)) ? np - 1 : 1);
-    const double u0 = w.u(i), u1 = w.u(i + 1);
-    c.i = i;
-    c.d0 = (i >= 2) ? u0 - w.u(i - 1) : 0.0;
-    c.d1 = u1 - u0;
-    c.d2 = (i + 2 <= np) ? w.u(i + 2) - u1 : 0.0;
-    const double K1 = 6.0 * (1.0 - p) * B.serr * B.serr;
-    c.c1 = w.y(i) - K1 * ((c.d1 - c.d0) * B.rh);
-    c.a1n = w.y(i + 1) - K1 * ((c.d2 - c.d1) * B.rh);
-    c.c3 = u0 * (6.0 * p);
-    c.a3n = u1 * (6.0 * p);
-    c.c4 = (c.a3n - c.c3) * B.rh;
-    c.c2 = (c.a1n - c.c1) * B.rh - (c.c3 + c.c4 * (1.0 / 3.0) * B.hb) * 0.5 * B.hb;
+    return (t >= 0.0 && t < (double)(B.np - 1)) ? (int)t + 1 : ((t >= (double)(B.np - 1)) ? B.np - 1 : 1);
+}
+// c: a piece of the same fit formed before (c.i = 0: none), formed again where
+// x lies in another one
+template <class W>
+__device__ __forceinline__ void b_piece(const W& w, const BPar& B, double p, double x, BPiece& c) {
+    const int np = B.np, i = b_piece_at(B, x);
+    if (i != c.i) {
+        const double u0 = w.u(i), u1 = w.u(i + 1);
+        c.i = i;
+        c.d0 = (i >= 2) ? u0 - w.u(i - 1) : 0.0;
+        c.d1 = u1 - u0;
+        c.d2 = (i + 2 <= np) ? w.u(i + 2) - u1 : 0.0;
+        const double K1 = 6.0 * (1.0 - p) * B.serr * B.serr;
+        c.c1 = w.y(i) - K1 * ((c.d1 - c.d0) * B.rh);
+        c.a1n = w.y(i + 1) - K1 * ((c.d2 - c.d1) * B.rh);
+        c.c3 = u0 * (6.0 * p);
+        c.a3n = u1 * (6.0 * p);
+        c.c4 = (c.a3n - c.c3) * B.rh;
+        c.c2 = (c.a1n - c.c1) * B.rh - (c.c3 + c.c4 * (1.0 / 3.0) * B.hb) * 0.5 * B.hb;
+    }
     c.hx = x - (B.z1 + (double)(i - 1) * B.hb);
-    return c;
 }
 __device__ __forceinline__ double b_value(const BPiece& c) {
     return ((c.c4 * (1.0 / 3.0) * c.hx + c.c3) * 0.5 * c.hx + c.c2) * c.hx + c.c1;
@@ -910,24 +973,26 @@ __device__ __forceinline__ double b_piece_rev(const W& w, const BPar& B, double 
 struct BSub {
     bool in1, in2, bot, top;       // slope taken; diffusivity taken from the fit; reflected
     double kz, z3, sd, z;          // slope times deltat, z3, sqrt(2 K deltat), the new position
-    BPiece c1, c2;
+    BPiece c1, c2;                 // the pieces at the start and at z3
 };
 template <class W>
 __device__ __forceinline__ BSub b_sub(const W& w, const BPar& B, const RpStepArgs& A, double p, double tdepth,
-                                      double zeta, double z, double dev) {
+                                      double zeta, double z, double dev, const BPiece& last) {
     BSub s;
+    s.c1 = last;
     s.in1 = !(z <= tdepth || z >= zeta);
     double kp = 0.0;
     if (s.in1) {
-        s.c1 = b_piece(w, B, p, z);
+        b_piece(w, B, p, z, s.c1);
         kp = b_slope(s.c1);
     }
     s.kz = kp * A.deltat;
     s.z3 = z + 0.5 * s.kz;
     s.in2 = !(s.z3 < tdepth || s.z3 > zeta);
     double K = A.aksback;
+    s.c2 = s.c1;
     if (s.in2) {
-        s.c2 = b_piece(w, B, p, s.z3);
+        b_piece(w, B, p, s.z3, s.c2);
         K = b_value(s.c2);
         if (K < A.aksback) {
             K = A.aksback;
@@ -970,11 +1035,15 @@ __device__ __forceinline__ double b_vturb(const RpStepArgs& A, const AdjFrames& 
     if (find) p = b_find_p(w, B, A.smth, A.spline_max_iter, fl);
     b_solve<false>(w, B, p);
     double z = Z, dev, dev_next = 0.0;
+    BPiece c;
+    c.i = 0;
 #pragma unroll 1
     for (int i = 1; i <= A.loop; i++) {
         if (i & 1) rp_normal2(A, pid, (uint32_t)(1 + i), i < A.loop, dev, dev_next);
         else dev = dev_next;
-        z = b_sub(w, B, A, p, St.tdepth, St.zeta, z, dev).z;
+        const BSub s = b_sub(w, B, A, p, St.tdepth, St.zeta, z, dev, c);
+        z = s.z;
+        c = s.c2;
     }
     return z - Z;
 }
@@ -1010,19 +1079,24 @@ __device__ __forceinline__ void b_vturb_rev(const RpStepArgs& A, const AdjFrames
             w.yb(i) = 0.0;
         }
         double z = Z, dev = 0.0, dev_next = 0.0;
+        BPiece c;
+        c.i = 0;
 #pragma unroll 1
         for (int i = 1; i <= A.loop; i++) {
             if (i & 1) rp_normal2(A, pid, (uint32_t)(1 + i), i < A.loop, dev, dev_next);
             else dev = dev_next;
             w.zt(i) = z;
             w.dev(i) = dev;
-            z = b_sub(w, B, A, p, St.tdepth, St.zeta, z, dev).z;
+            const BSub s = b_sub(w, B, A, p, St.tdepth, St.zeta, z, dev, c);
+            z = s.z;
+            c = s.c2;
         }
         t[0] = z - Z;
 #pragma unroll 1
         for (int i = A.loop; i >= 1; i--) {
             const double zi = w.zt(i), d = w.dev(i);
-            const BSub s = b_sub(w, B, A, p, St.tdepth, St.zeta, zi, d);
+            const BSub s = b_sub(w, B, A, p, St.tdepth, St.zeta, zi, d, c);
+            c = s.c1;
             if (s.top) {
                 zeb += 2.0 * zb;
                 zb = -zb;
@@ -1042,10 +1116,33 @@ __device__ __forceinline__ void b_vturb_rev(const RpStepArgs& A, const AdjFrames
         }
     }
     const int np = B.np, sw = B.sw;
-    // lambda = M^-1 ub by the fit's factor; u(1) = u(np) = 0
+    // lambda = M^-1 ub by the fit's factor; u(1) = u(np) = 0.  Upwards first,
+    // four rows' values read together
     {
         double w1 = 0.0, w2 = 0.0, q1 = 0.0, q2 = 0.0, q2p = 0.0;   // w(i-1), w(i-2), ratio1(i-1), ratio2(i-1), (i-2)
-        for (int i = 2; i <= np - 1; i++) {
+        int i = 2;
+#pragma unroll 1
+        for (; i + 3 <= np - 2; i += 4) {
+            double v[4], r1[4], r2[4], iv[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                v[k] = w.ub(i + k);
+                r1[k] = w.s1(i + k);
+                r2[k] = w.s2(i + k);
+                iv[k] = w.inv(i + k);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const double wi = fma(-q2p, w2, fma(-q1, w1, v[k]));
+                w.ub(i + k) = wi * iv[k];
+                w2 = w1;
+                w1 = wi;
+                q2p = q2;
+                q1 = r1[k];
+                q2 = r2[k];
+            }
+        }
+        for (; i <= np - 1; i++) {
             const double wi = fma(-q2p, w2, fma(-q1, w1, w.ub(i)));
             w.ub(i) = wi * w.inv(i);
             w2 = w1;
@@ -1056,66 +1153,94 @@ __device__ __forceinline__ void b_vturb_rev(const RpStepArgs& A, const AdjFrames
                 q2 = w.s2(i);
             }
         }
-        double l2 = 0.0, l1 = w.ub(np - 1);
-        for (int i = np - 2; i >= 2; i--) {
-            const double li = fma(-l1, w.s1(i), fma(-l2, w.s2(i), w.ub(i)));
-            w.ub(i) = li;
-            l2 = l1;
-            l1 = li;
-        }
-        w.ub(1) = 0.0;
-        w.ub(np) = 0.0;
     }
-    // bands and right-hand side in hb, then the data: b(i) = (y(i+1) - 2 y(i) + y(i-1)) / hb
-    {
-        const double six1mp = 6.0 * (1.0 - p), dr2 = -2.0 * B.r2 * B.rh;
-        const double Dh = six1mp * 6.0 * dr2 + 4.0 * p, Eh = six1mp * -4.0 * dr2 + p, Fh = six1mp * dr2;
-        double sD = 0.0, sE = 0.0, sF = 0.0, sB = 0.0;
-        double lm2 = 0.0, lm1 = 0.0, um2 = 0.0, um1 = 0.0;
-        for (int i = 2; i <= np - 1; i++) {
-            const double l = w.ub(i), u = w.u(i);
-            sD = fma(l, u, sD);
-            sE = fma(l, um1, fma(lm1, u, sE));
-            sF = fma(l, um2, fma(lm2, u, sF));
-            sB = fma(l, (w.y(i + 1) - 2.0 * w.y(i) + w.y(i - 1)) * B.rh, sB);
-            lm2 = lm1;
-            lm1 = l;
-            um2 = um1;
-            um1 = u;
-        }
-        hbb -= Dh * sD + Eh * sE + Fh * sF + sB * B.rh;
-        for (int i = 1; i <= np; i++) {
-            const double lp = (i < np) ? w.ub(i + 1) : 0.0, lm = (i > 1) ? w.ub(i - 1) : 0.0;
-            w.yb(i) += (lp - 2.0 * w.ub(i) + lm) * B.rh;
-        }
-    }
-    // the resampling: y(i) = K(j) + m (x - z(j)), x = z1 + (i-1) hb
+    // Downwards, all that follows from lambda in one sweep: the bands and the
+    // right-hand side b(i) = (y(i+1) - 2 y(i) + y(i-1)) / hb in hb, the data's
+    // adjoints, and the resampling y(i) = K(j) + m (x - z(j)), x = z1 + (i-1) hb,
+    // whose bracket's sums are put down where it changes
     for (int k = 1; k <= sw; k++) {
         w.zcb(k) = 0.0;
         w.khb(k) = 0.0;
     }
-    w.khb(1) += w.yb(1);
-    w.khb(sw) += w.yb(np);
     {
+        double sD = 0.0, sE = 0.0, sF = 0.0, sB = 0.0;
+        double l1 = 0.0, l2 = 0.0, u1 = 0.0, u2 = 0.0;      // lambda and u of rows i+1, i+2
+        double y1 = w.y(np), y0 = w.y(np - 1);              // y(i+1), y(i)
         int j = 0;
-        double m = 0.0, rz = 0.0, z0 = 0.0;
-        for (int i = 2; i <= np - 1; i++) {
-            const double x = B.z1 + (double)(i - 1) * B.hb, g = w.yb(i);
-            const int jn = b_bracket(w, sw, asc, max(j, 1), x);
-            if (jn != j) {
-                j = jn;
+        double m = 0.0, rz = 0.0, z0 = 0.0, gK = 0.0, gm = 0.0;   // bracket; sums of g and of m's adjoint
+        auto put = [&]() {
+            if (j == 0) return;
+            const double mb = gm * rz;
+            w.khb(j) += gK + mb;
+            w.khb(j + 1) -= mb;
+            w.zcb(j) -= gK * m + mb * m;
+            w.zcb(j + 1) += mb * m;
+        };
+        // adjoint g of y(i): the direct one and lambda's
+        auto data = [&](int i, double g) {
+            const double x = B.z1 + (double)(i - 1) * B.hb;
+            const bool in = asc ? (j != 0 && (j == 1 || w.zc(j) <= x)) : false;
+            if (!in) {
+                put();
+                if (asc) {
+                    j = (j == 0) ? sw - 1 : j;
+                    while (j > 1 && w.zc(j) > x) j--;
+                } else {
+                    j = b_bracket(w, sw, false, 1, x);
+                }
                 z0 = w.zc(j);
                 rz = 1.0 / (z0 - w.zc(j + 1));
                 m = (w.kh(j) - w.kh(j + 1)) * rz;
+                gK = gm = 0.0;
             }
-            const double gm = g * m, mb = g * (x - z0) * rz;
-            z1b += gm;
-            hbb += (double)(i - 1) * gm;
-            w.khb(j) += g + mb;
-            w.khb(j + 1) -= mb;
-            w.zcb(j) -= gm + mb * m;
-            w.zcb(j + 1) += mb * m;
+            gK += g;
+            gm = fma(g, x - z0, gm);
+            const double xb = g * m;
+            z1b += xb;
+            hbb = fma((double)(i - 1), xb, hbb);
+        };
+        // row i: lambda(i) from its forward value; y(i+1)'s adjoint is then complete
+        auto row = [&](int i, double v, double q1, double q2, double ui, double ym, double yb1) {
+            const double l = fma(-l1, q1, fma(-l2, q2, v));
+            sD = fma(l, ui, sD);
+            sE = fma(l, u1, fma(l1, ui, sE));
+            sF = fma(l, u2, fma(l2, ui, sF));
+            sB = fma(l, (y1 - 2.0 * y0 + ym) * B.rh, sB);
+            const double g = fma((l - 2.0 * l1) + l2, B.rh, yb1);
+            if (i + 1 < np) data(i + 1, g);
+            else w.khb(sw) += g;
+            l2 = l1;
+            l1 = l;
+            u2 = u1;
+            u1 = ui;
+            y1 = y0;
+            y0 = ym;
+        };
+        row(np - 1, w.ub(np - 1), 0.0, 0.0, w.u(np - 1), w.y(np - 2), w.yb(np));
+        int i = np - 2;
+#pragma unroll 1
+        for (; i - 3 >= 2; i -= 4) {
+            double v[4], q1[4], q2[4], ui[4], ym[4], yb[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                v[k] = w.ub(i - k);
+                q1[k] = w.s1(i - k);
+                q2[k] = w.s2(i - k);
+                ui[k] = w.u(i - k);
+                ym[k] = w.y(i - k - 1);
+                yb[k] = w.yb(i - k + 1);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) row(i - k, v[k], q1[k], q2[k], ui[k], ym[k], yb[k]);
         }
+#pragma unroll 1
+        for (; i >= 2; i--) row(i, w.ub(i), w.s1(i), w.s2(i), w.u(i), w.y(i - 1), w.yb(i + 1));
+        data(2, fma(l2 - 2.0 * l1, B.rh, w.yb(2)));         // lambda(1) = 0; l1 = lambda(2), l2 = lambda(3)
+        put();
+        w.khb(1) += fma(l1, B.rh, w.yb(1));
+        const double six1mp = 6.0 * (1.0 - p), dr2 = -2.0 * B.r2 * B.rh;
+        const double Dh = six1mp * 6.0 * dr2 + 4.0 * p, Eh = six1mp * -4.0 * dr2 + p, Fh = six1mp * dr2;
+        hbb -= Dh * sD + Eh * sE + Fh * sF + sB * B.rh;
     }
     const double hr = hbb / (double)(np - 1);
     w.zcb(sw) += hr;
@@ -1165,9 +1290,9 @@ __device__ __forceinline__ bool a_active(const RpStepArgs& A, double dob, double
 // displacement (S1: RK stage 1's quantities where have_s1), called with VTurb
 // on.  Returns the sign the new Z carries VTurb's displacement with (0: not at
 // all).
-template <class S, class V>
+template <class S, class VT>
 __device__ __forceinline__ int a_step(const RpStepArgs& A, const AdjFrames& F, double dob, uint32_t pid, S& X, S& Y,
-                                      S& Z, AdjAux& a, uint32_t& fl, V&& vturb) {
+                                      S& Z, AdjAux& a, uint32_t& fl, VT&& vturb) {
     if (!a_active(A, dob, a.status, a.isin)) return 0;
     a.age = a.age + (double)(float)A.idt;
     int gid = a.gid;

@@ -73,6 +73,8 @@ int64_t sort_key_count(const RpStepArgs& A, uint32_t* gbase_host);
 // sorts A.p's columns in place; `scratch8` holds n 8-byte values
 cudaError_t launch_sort(const RpStepArgs& A, int mixed, const SortBufs& b, void* scratch8, cudaStream_t s,
                         int* nlaunch);
+// b.perm: A.p's particles by that order, the columns left as they lie
+cudaError_t launch_order(const RpStepArgs& A, int mixed, const SortBufs& b, cudaStream_t s, int* nlaunch);
 // dst[pid[i] - base] = src[i] for pid[i] - base < nout (elem = 8, 4 or 1 bytes)
 cudaError_t launch_unsort(int elem, const void* src, void* dst, const uint32_t* pid, uint32_t base, int64_t n,
                           int64_t nout, cudaStream_t s);
@@ -86,6 +88,10 @@ struct AdjStateDev {
     double* status;
     int32_t* gid;
     int8_t* isin;
+    // order in which the kernels take the particles (null: as they lie): a
+    // permutation of 0 .. n-1 by grid and cell, so that a warp's gathers share
+    // sectors; the state stays where it is
+    const int32_t* order = nullptr;
 };
 // kind 0: step (find: search and record p in prec, else replay prec);
 // 1: tangent step (t: 12 derivatives per particle); 2: reverse step

@@ -123,8 +123,7 @@ static cudaError_t permute_col(T* col, void* scratch, const int32_t* perm, int64
     return cudaMemcpyAsync(col, tmp, (size_t)n * sizeof(T), cudaMemcpyDeviceToDevice, s);
 }
 
-cudaError_t launch_sort(const RpStepArgs& A, int mixed, const SortBufs& b, void* scratch8, cudaStream_t s,
-                        int* nlaunch) {
+cudaError_t launch_order(const RpStepArgs& A, int mixed, const SortBufs& b, cudaStream_t s, int* nlaunch) {
     const int64_t n = A.p.n;
     if (n <= 0) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(b.hist, 0, sizeof(uint32_t) * (size_t)b.nkeys, s);
@@ -136,7 +135,15 @@ cudaError_t launch_sort(const RpStepArgs& A, int mixed, const SortBufs& b, void*
     k_scan_add<<<(unsigned)nb, kScanBlock, 0, s>>>(b.hist, b.nkeys, b.sums);
     k_sort_scatter<<<blocks_for(n, 256), 256, 0, s>>>(n, b.keys, b.hist, b.perm);
     *nlaunch += 5;
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_sort(const RpStepArgs& A, int mixed, const SortBufs& b, void* scratch8, cudaStream_t s,
+                        int* nlaunch) {
+    const int64_t n = A.p.n;
+    if (n <= 0) return cudaSuccess;
+    cudaError_t e = launch_order(A, mixed, b, s, nlaunch);
+    if (e != cudaSuccess) return e;
     const RpParticlesDev& P = A.p;
     double* d8[] = {P.x, P.y, P.z, P.age, P.dob, P.status, P.wd, P.zeta, P.bath, mixed ? P.qwarm : nullptr,
                     mixed ? P.gwarm : nullptr, P.salt, P.temp, P.mean_salt, P.mean_temp, P.hob, P.bustr, P.bvstr,

@@ -21,20 +21,31 @@ pytestmark = pytest.mark.gpu
     ({}, {"smth": 0.0}), ({}, {"smth": 1e9}), ({}, {"scheme": 0}), ({}, {"nsb": 1}), ({"vtransform": 1}, {}),
     ({"vtransform": 3}, {}), ({}, {"vturb_on": 0})])
 def test_backward_matches_tangent_linear(spec, param):
+    _check(spec, param, 129)
+
+
+# enough particles for the kernels to take them by cell (the tangent-linear
+# reference takes them as they lie), in segments of 4 and of 14 steps
+@pytest.mark.parametrize("ckpt", [4, 14])
+def test_ordered_by_cell(ckpt):
+    _check({"land": "islands"}, {"hturb_on": 1, "constant_hturb": [1.0] * 5}, 8209, ckpt)
+
+
+def _check(spec, param, n, ckpt=4):
     from romspath_b200 import Tracker, schedule
     from romspath_b200.adjoint import Adjoint, attribution_loss, step_table
-    case = harness.make_case("tiny", 129, seed=11, spec_over=spec, param_over=param, s_range=(-1.0, 0.0))
-    T = Tracker(case.specs, case.grids, case.params, numpar=129, field_dtype="f64", seed=7)
+    case = harness.make_case("tiny", n, seed=11, spec_over=spec, param_over=param, s_range=(-1.0, 0.0))
+    T = Tracker(case.specs, case.grids, case.params, numpar=n, field_dtype="f64", seed=7)
     for (k, slot) in schedule.initial_loads():
         T.upload_frame(1, slot, case.frame(k))
     T.locate(case.release, t_b=1)
     steps = step_table(2.0, int(case.params["dt"]), int(case.params["idt"]))[0][:14]
     adj = Adjoint(T)
     adj.load_frames(max(max(s.frame_b, s.frame_c, s.frame_f) for s in steps), lambda ng, k: case.frame(k, ng))
-    adj.forward(steps, kappa=1.25, checkpoint_every=4)
+    adj.forward(steps, kappa=1.25, checkpoint_every=ckpt)
     fin = T.get_particles()
     _, gx, gy = attribution_loss(fin["x"], fin["y"], TARGET)
-    gz = np.linspace(-1.0, 1.0, 129)
+    gz = np.linspace(-1.0, 1.0, n)
     got = adj.backward(gx, gy, gz)
     J = adj.tangent(kappa=1.25)
     T.close()
