@@ -17,10 +17,11 @@ namespace rp {
 // Bound by the latency of the fit's workspace and of the column's gathers
 // (neither the issue slots, about half busy, nor DRAM at 40 %): four blocks of
 // 128 an SM, whose 128 registers hold a quad of rows and the next one's loads
-// without spilling and whose workspaces nearly fit in L2, are faster than eight
+// without spilling and whose workspaces come nearer to L2, are faster than eight
 // at 64 registers.  Per 12-step interval, eight, five and four blocks: 512x384x30
 // with 1,048,576 particles 18.8, 18.7 and 18.5 ms; 130x98x20 with 4,194,304 58.8,
-// 54.1 and 51.3 ms (23.0 and 62.8 ms one row at a time in eight blocks).
+// 54.1 and 51.3 ms (23.0 and 62.8 ms one row at a time in eight blocks), with
+// the data resampled beforehand 17.1 and 49.3 ms at four, 18.0 and 50.0 at five.
 // FEAT: built with the options beyond the passive step (diagnostics,
 // WETDRY, behave); the passive variant is chosen when they are all off.
 // BLK: threads per block (the register cap stays that of 128 x 8 resident
@@ -49,21 +50,22 @@ __global__ void __launch_bounds__(kStepBlock, kMixedVtMinBlocks) k_vturb_mixed(c
 }
 
 // Split form with the fit's workspace in shared memory: VTurb alone, one
-// thread per particle, 64-thread blocks each holding its threads' u, factor
-// prefix and column (1.1 KB per thread at NPMAX 128: 3 blocks per SM).  The
-// fit's passes then read and write shared memory instead of streaming a
-// local-memory workspace through L2 and HBM.
+// thread per particle, 64-thread blocks each holding its threads' u and factor
+// prefix (0.75 KB per thread at NPMAX 128).  The fit's passes then read and
+// write shared memory instead of streaming a local-memory workspace through L2
+// and HBM.
 constexpr int kSmemBlock = 64;
 constexpr int kSmemKs = 32;              // factor rows 2..33 held in shared memory
 template <int NPMAX>
-using SmemView = MSmemSpline<NPMAX, kSmemKs, NPMAX / 4, kSmemBlock>;
+using SmemView = MSmemSpline<NPMAX, kSmemKs, kSmemBlock>;
 
 template <typename E, int NPMAX>
 __global__ void __launch_bounds__(kSmemBlock) k_vturb_smem(const __grid_constant__ RpStepArgs A,
                                                            float* __restrict__ turbv) {
     extern __shared__ float smf[];
     float ovf[2 * (NPMAX + 1)];
-    const SmemView<NPMAX> w{smf + threadIdx.x, ovf};
+    double yl[NPMAX + 4];
+    const SmemView<NPMAX> w{smf + threadIdx.x, ovf, yl};
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < A.p.n; n += stride)
         m_vturb_one<E>(A, n, w, turbv);
@@ -146,12 +148,6 @@ static cudaError_t launch_mixed_t(const RpStepArgs& A, float* turbv, int split, 
         k_advect_mixed<E, FEAT><<<(unsigned)blocks, kStepBlock, 0, s>>>(A, nullptr);
         *nlaunch += 1;
         return cudaGetLastError();
-    }
-    if (split == 2) {
-        // the shared-memory column holds sw <= NPMAX/4 levels
-        int swmax = 0;
-        for (int k = 0; k < A.ngrid; k++) swmax = max(swmax, A.g[k].N + 1);
-        if (swmax > NPMAX / 4) split = 1;
     }
     if (split == 2) {
         const size_t smem = (size_t)SmemView<NPMAX>::kWords * kSmemBlock * sizeof(float);

@@ -25,7 +25,6 @@
 #pragma once
 
 #include <cuda_fp16.h>
-#include <math_constants.h>
 
 #include "rp_step.cuh"
 
@@ -510,33 +509,29 @@ __device__ __forceinline__ void m_find_currents(const RpStepArgs& A, const RpGri
 // backward.
 
 // Workspace: u, the factor ratios of the rows before the factor turns
-// stationary, the resampled data, and the column's pieces, all FP32 (the
-// sweeps of m_chol1d compute in FP32).  The sweeps take rows 2..5, 6..9, ...
-// together and move each quad as one 16-byte access: element i of u and the
-// ratios sits at position i + 2, that of y, resampled two points ahead of its
-// row, at position i.
-constexpr int m_row_words(int npmax) { return (npmax + 6) / 4 * 4; }   // positions 0 .. npmax + 2
+// stationary and the resampled data, all FP32 (the sweeps of m_chol1d compute
+// in FP32).  The sweeps take rows 2..5, 6..9, ... together and move each quad
+// as one 16-byte access: element i of u and the ratios sits at position i + 2,
+// that of y, read two points ahead of its row, at position i.
+constexpr int m_row_words(int npmax) { return (npmax + 6) / 4 * 4; }   // positions 0 .. npmax + 3
 
 struct MFit {
-    int np, sw;
+    int np;
     double z1, h, rh;              // first break, spacing, 1/h
     double serr, dy2;
 };
 
-// The per-thread workspace in local memory (the fused step), the resampled
-// data y stored by the first pass (formed again from the column at each piece
-// instead, 512x384x30 with 1,048,576 particles: 19.9 ms an interval, 18.8 with
-// y stored).  Piece j of the column, [z(j), z(j+1)], is one quad (z(j+1), slope, intercept, -).  PREF: the
-// back substitution loads its next quad ahead (fewer stalls, more registers
-// live; which is faster depends on the workload).
+// The per-thread workspace in local memory (the fused step).  PREF: the back
+// substitution loads its next quad ahead (fewer stalls, more registers live;
+// which is faster depends on the workload).
 template <int NPMAX, bool PREF = true>
 struct MSpline {
-    static constexpr bool kStoreY = true;
+    using YT = float;
     static constexpr int kColBatch = 2;
     static constexpr bool kLightCheck = false;
     static constexpr bool kPrefetch = PREF;
     static constexpr int kRow = m_row_words(NPMAX);
-    static constexpr int kWords = 4 * kRow + 4 * (NPMAX + 1);
+    static constexpr int kWords = 4 * kRow;
     float* base;                   // kWords floats, 16-byte aligned
     __device__ __forceinline__ float& u(int i) const { return base[i + 2]; }              // u(i)/v(i,1), then u(i)
     __device__ __forceinline__ float& s1(int i) const { return base[kRow + i + 2]; }      // ratio1(i)
@@ -546,36 +541,28 @@ struct MSpline {
     __device__ __forceinline__ float4 u4(int i) const { return *reinterpret_cast<const float4*>(&u(i)); }
     __device__ __forceinline__ float4 s14(int i) const { return *reinterpret_cast<const float4*>(&s1(i)); }
     __device__ __forceinline__ float4 s24(int i) const { return *reinterpret_cast<const float4*>(&s2(i)); }
+    __device__ __forceinline__ float4 y4(int i) const { return *reinterpret_cast<const float4*>(&y(i)); }
     __device__ __forceinline__ void set_u4(int i, const float4& v) const { *reinterpret_cast<float4*>(&u(i)) = v; }
     __device__ __forceinline__ void set_s14(int i, const float4& v) const { *reinterpret_cast<float4*>(&s1(i)) = v; }
     __device__ __forceinline__ void set_s24(int i, const float4& v) const { *reinterpret_cast<float4*>(&s2(i)) = v; }
-    __device__ __forceinline__ void set_y4(int i, const float4& v) const { *reinterpret_cast<float4*>(&y(i)) = v; }
-    __device__ __forceinline__ float yat(const MFit&, int i, int&) const { return y(i); }
-    __device__ __forceinline__ float4 seg(int j) const {
-        return *reinterpret_cast<const float4*>(base + 4 * kRow + 4 * j);
-    }
-    __device__ __forceinline__ void set_seg(int j, float zn, float m, float b) const {
-        *reinterpret_cast<float4*>(base + 4 * kRow + 4 * j) = make_float4(zn, m, b, 0.f);
-    }
 };
 
-// The workspace in shared memory (the split step's VTurb kernel): u, the
+// The workspace in shared memory (the split step's VTurb kernel): u and the
 // factor ratios of the rows before the factor turns stationary (rows
 // 2..KSM+1; later rows, met only when it does not, in the thread's local
-// array `ovf`), and the column's breaks, slopes and intercepts (sw <= CMAX).
-// Element k of a thread sits at word k * B of its own column (threads of a
-// block in consecutive banks).  The resampled data are not stored: ppvalu's
-// two values per piece come from the column (the same m x + b the fit's
-// sweep forms).
-template <int NPMAX, int KSM, int CMAX, int B>
+// array `ovf`); the resampled data in a local array, in FP64 for the light
+// pass.  Element k of a thread sits at word k * B of its own column (threads of
+// a block in consecutive banks).
+template <int NPMAX, int KSM, int B>
 struct MSmemSpline {
-    static constexpr bool kStoreY = false;
+    using YT = double;
     static constexpr int kColBatch = 8;
     static constexpr bool kLightCheck = true;
     static constexpr bool kPrefetch = true;
-    static constexpr int kWords = NPMAX + 2 * KSM + 3 * CMAX;
+    static constexpr int kWords = NPMAX + 2 * KSM;
     float* sm;                     // this thread's first word
     float* ovf;                    // 2 (NPMAX + 1) floats, local
+    double* yl;                    // NPMAX + 4 doubles, local
     __device__ __forceinline__ float& u(int i) const { return sm[(i - 1) * B]; }
     __device__ __forceinline__ float& s1(int i) const {
         return (i <= KSM + 1) ? sm[(NPMAX + i - 2) * B] : ovf[i];
@@ -583,8 +570,10 @@ struct MSmemSpline {
     __device__ __forceinline__ float& s2(int i) const {
         return (i <= KSM + 1) ? sm[(NPMAX + KSM + i - 2) * B] : ovf[NPMAX + 1 + i];
     }
-    __device__ __forceinline__ float& y(int) const { return ovf[0]; }        // never stored (kStoreY)
-    __device__ __forceinline__ void set_y4(int, const float4&) const {}
+    __device__ __forceinline__ double& y(int i) const { return yl[i]; }
+    __device__ __forceinline__ float4 y4(int i) const {
+        return make_float4((float)y(i), (float)y(i + 1), (float)y(i + 2), (float)y(i + 3));
+    }
     __device__ __forceinline__ float4 u4(int i) const { return make_float4(u(i), u(i + 1), u(i + 2), u(i + 3)); }
     __device__ __forceinline__ float4 s14(int i) const { return make_float4(s1(i), s1(i + 1), s1(i + 2), s1(i + 3)); }
     __device__ __forceinline__ float4 s24(int i) const { return make_float4(s2(i), s2(i + 1), s2(i + 2), s2(i + 3)); }
@@ -606,76 +595,10 @@ struct MSmemSpline {
         s2(i + 2) = v.z;
         s2(i + 3) = v.w;
     }
-    __device__ __forceinline__ float& cz(int k) const { return sm[(NPMAX + 2 * KSM + k - 1) * B]; }
-    __device__ __forceinline__ float& cm(int k) const { return sm[(NPMAX + 2 * KSM + CMAX + k - 1) * B]; }
-    __device__ __forceinline__ float& cb(int k) const { return sm[(NPMAX + 2 * KSM + 2 * CMAX + k - 1) * B]; }
-    __device__ __forceinline__ float4 seg(int j) const { return make_float4(cz(j + 1), cm(j), cb(j), 0.f); }
-    __device__ __forceinline__ void set_seg(int j, float zn, float m, float b) const {
-        cz(j + 1) = zn;
-        cm(j) = m;
-        cb(j) = b;
-    }
-    __device__ __forceinline__ float yat(const MFit& f, int i, int& j) const;
 };
-
-// linint of the column at ascending points in type R: the current piece
-// (slope, intercept and upper end) and the next one are held in registers,
-// so that an advance waits for no load: in a warp some lane advances at
-// nearly every point.  The last piece's upper end is NaN (m_vturb), which
-// ends the walk also at an infinite point (a frame whose zeta is).
-template <class W, typename R>
-struct MWalk {
-    int j;
-    float4 nx;                     // piece j + 1
-    R zn, m, b;                    // piece j
-    __device__ __forceinline__ void take(const float4& v) {
-        zn = (R)v.x;
-        m = (R)v.y;
-        b = (R)v.z;
-    }
-    __device__ __forceinline__ void init(const W& w, int sw) {
-        j = 1;
-        take(w.seg(1));
-        nx = w.seg(min(2, sw - 1));
-    }
-    __device__ __forceinline__ R at(const W& w, int sw, R x) {
-        while (zn <= x) {
-            j++;
-            take(nx);
-            nx = w.seg(min(j + 1, sw - 1));
-        }
-        return m * x + b;
-    }
-};
-
-// The resampled value y(i) at z1 + (i-1) h as the sweeps form it: linint's
-// piece j (j in 1..sw-1, the last whose lower end is at or below the point; 1
-// below z(2)), found by bisection the first time (j = 0) and from the previous
-// point's piece after that.
-template <class W>
-__device__ __forceinline__ float m_resampled(const W& w, const MFit& f, int i, int& j) {
-    const float x = fmaf((float)(i - 1), (float)f.h, (float)f.z1);
-    if (j == 0) {
-        int lo = 1, hi = f.sw - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (w.seg(mid - 1).x <= x) lo = mid; else hi = mid - 1;
-        }
-        j = lo;
-    }
-    while (j > 1 && !(w.seg(j - 1).x <= x)) j--;
-    float4 v = w.seg(j);
-    while (v.x <= x) v = w.seg(++j);
-    return fmaf(v.y, x, v.z);
-}
-template <int NPMAX, int KSM, int CMAX, int B>
-__device__ __forceinline__ float MSmemSpline<NPMAX, KSM, CMAX, B>::yat(const MFit& f, int i, int& j) const {
-    return m_resampled(*this, f, i, j);
-}
 
 // One chol1d pass at p: factorise, solve for u, form qu = Q u; returns
-// sum_i qu(i)^2 dy^2.  With store_y the resampled values y(i) are also kept
-// (for ppvalu).
+// sum_i qu(i)^2 dy^2.
 // The factor's rows before it turns stationary are formed in FP64 and
 // stored in FP32; the substitutions, qu and its sum run in FP32 (the data,
 // the factor ratios and u are FP32 values).
@@ -685,8 +608,7 @@ __device__ __forceinline__ float MSmemSpline<NPMAX, KSM, CMAX, B>::yat(const MFi
 // a quad.  One row at a time cost 73 thread instructions a row for both
 // sweeps, 28 of them addresses, counters and compares.
 template <class W>
-__device__ __forceinline__ double m_chol1d(const W& w, const MFit& f, double p, bool store_y) {
-    store_y = store_y && W::kStoreY;
+__device__ __forceinline__ double m_chol1d(const W& w, const MFit& f, double p) {
     const int np = f.np;
     const double r = f.serr * f.rh;
     const double r2 = r * r;
@@ -694,18 +616,9 @@ __device__ __forceinline__ double m_chol1d(const W& w, const MFit& f, double p, 
     const double D = six1mp * (6.0 * r2) + 4.0 * p * f.h;
     const double E = six1mp * (-4.0 * r2) + p * f.h;
     const double F = six1mp * r2;
-    const float hf = (float)f.h, rhf = (float)f.rh, z1f = (float)f.z1;
-    // Q'y on the fly: qty(i) = (y(i+1) - 2 y(i) + y(i-1)) / h, y at z1 + (i-1) h
-    MWalk<W, float> wk;
-    wk.init(w, f.sw);
-    float ym = wk.at(w, f.sw, z1f);
-    float y0 = wk.at(w, f.sw, z1f + hf);
-    float yp = wk.at(w, f.sw, fmaf(2.f, hf, z1f));
-    if (store_y) {
-        w.y(1) = ym;
-        w.y(2) = y0;
-        w.y(3) = yp;
-    }
+    const float rhf = (float)f.rh;
+    // Q'y on the fly: qty(i) = (y(i+1) - 2 y(i) + y(i-1)) / h
+    float ym = (float)w.y(1), y0 = (float)w.y(2), yp = (float)w.y(3);
     double a1 = D, a2 = E, b1 = D;
     float uprev = 0.f, ucur = (yp - 2.f * y0 + ym) * rhf, r2prev = 0.f;
     // The bands are constant (uniform breaks), so the factor converges to
@@ -715,7 +628,6 @@ __device__ __forceinline__ double m_chol1d(const W& w, const MFit& f, double p, 
     int ks = np - 2;                                 // first reused row (np-2: none)
     bool held = false;
     float hinv = 0.f, h1 = 0.f, h2 = 0.f;
-    float xi = 3.f;                                  // point i + 1 (0-based), the next to be resampled
     auto factor = [&](float& inv, float& ratio1, float& ratio2) {
         const double invd = rp_rcp_ulp(a1);               // one reciprocal per row
         const double ratio1d = a2 * invd, ratio2d = F * invd;
@@ -727,12 +639,11 @@ __device__ __forceinline__ double m_chol1d(const W& w, const MFit& f, double p, 
         ratio2 = (float)ratio2d;
     };
     // row i's u(i)/v(i,1); advances the substitution to row i + 1
-    auto forward = [&](float inv, float ratio1, float ratio2) -> float {
+    auto forward = [&](float inv, float ratio1, float ratio2, float yn) -> float {
         const float ui = ucur * inv;
         ym = y0;
         y0 = yp;
-        yp = wk.at(w, f.sw, fmaf(xi, hf, z1f));      // y(i+2) at z1 + (i+1) h
-        xi += 1.f;
+        yp = yn;                                     // y(i+2)
         const float qn = (yp - 2.f * y0 + ym) * rhf; // qty(i+1)
         const float unext = qn - ratio1 * ucur - r2prev * uprev;
         uprev = ucur;
@@ -741,9 +652,12 @@ __device__ __forceinline__ double m_chol1d(const W& w, const MFit& f, double p, 
         return ui;
     };
     int i = 2;
+    float4 yn = w.y4(4);                             // the next quad of data, loaded a quad ahead
 #pragma unroll 1
     for (; i + 3 <= np - 3; i += 4) {
-        float inv[4], q1[4], q2[4], uq[4], yq[4];
+        float inv[4], q1[4], q2[4], uq[4];
+        const float yq[4] = {yn.x, yn.y, yn.z, yn.w};
+        yn = w.y4(i + 6);
         if (!held) {
 #pragma unroll
             for (int k = 0; k < 4; k++) factor(inv[k], q1[k], q2[k]);
@@ -765,12 +679,8 @@ __device__ __forceinline__ double m_chol1d(const W& w, const MFit& f, double p, 
             }
         }
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            uq[k] = forward(inv[k], q1[k], q2[k]);
-            yq[k] = yp;
-        }
+        for (int k = 0; k < 4; k++) uq[k] = forward(inv[k], q1[k], q2[k], yq[k]);
         w.set_u4(i, make_float4(uq[0], uq[1], uq[2], uq[3]));
-        if (store_y) w.set_y4(i + 2, make_float4(yq[0], yq[1], yq[2], yq[3]));
     }
     const int it = i;                                // first row after the quads
 #pragma unroll 1
@@ -781,15 +691,13 @@ __device__ __forceinline__ double m_chol1d(const W& w, const MFit& f, double p, 
             w.s1(i) = ratio1;
             w.s2(i) = ratio2;
         }
-        w.u(i) = forward(inv, ratio1, ratio2);
-        if (store_y) w.y(i + 2) = yp;
+        w.u(i) = forward(inv, ratio1, ratio2, (float)w.y(i + 2));
     }
     // row np-2 (F = 0) and u(np-1)
     const double invl = rp_rcp_ulp(a1);
     const double ratiol = a2 * invl;
     const float q1l = (float)ratiol;
-    const float ul = forward((float)invl, q1l, 0.f); // resamples y(np)
-    if (store_y) w.y(np) = yp;
+    const float ul = forward((float)invl, q1l, 0.f, (float)w.y(np));
     const float uend = (float)((double)ucur / (b1 - ratiol * a2));
     // back substitution, descending, with qu and its sum of squares:
     // raw(k) = (u(k) - u(k-1))/h for 2 <= k <= np, raw(1) = raw(np+1) = 0,
@@ -883,12 +791,7 @@ __device__ double m_light_S(const W& w, const MFit& f, double p) {
     const double Dd = -36.0 * r2 + 4.0 * f.h;          // dD/dp, dE/dp, dF/dp
     const double Ed = 24.0 * r2 + f.h;
     const double Fd = -6.0 * r2;
-    MWalk<W, double> wk;
-    wk.init(w, f.sw);
-    double ym = wk.at(w, f.sw, f.z1);
-    double y0 = wk.at(w, f.sw, f.z1 + f.h);
-    double xn = f.z1 + 2.0 * f.h;
-    double yp = wk.at(w, f.sw, xn);
+    double ym = (double)w.y(1), y0 = (double)w.y(2), yp = (double)w.y(3);
     double a1 = D, a2 = E, b1 = D, a1d = Dd, a2d = Ed, b1d = Dd;
     double wc = (yp - 2.0 * y0 + ym) * f.rh, wcd = 0.0, wp = 0.0, wpd = 0.0;   // w(i), w(i-1) and d/dp
     double r2p = 0.0, r2pd = 0.0;                                               // ratio2(i-1)
@@ -927,8 +830,7 @@ __device__ double m_light_S(const W& w, const MFit& f, double p) {
         phid = phid + (2.0 * wc * wcd) * inv + wc * wc * invd;
         ym = y0;
         y0 = yp;
-        xn = xn + f.h;                               // z1 + (i+1) h, accumulated
-        yp = wk.at(w, f.sw, xn);
+        yp = (double)w.y(i + 2);
         const double qn = (yp - 2.0 * y0 + ym) * f.rh;           // qty(i+1)
         const double wn = qn - ratio1 * wc - r2p * wp;
         const double wnd = -(ratio1d * wc + ratio1 * wcd + r2pd * wp + r2p * wpd);
@@ -977,7 +879,6 @@ __device__ double m_smooth(const W& w, const MFit& f, double s, int max_iter, do
     if (warm) q = (q2 > 0.0) ? q_in * fmin(fmax(q_in / q2, 0.5), 2.0) : q_in;
     double prevq = 0.0, prevsf = 0.0;
     int stage = warm ? kGuess : kCold, it = 0;
-    bool ys = false;                                 // y(i) stored by a pass already
     for (passes = 1;; passes++) {
         const double p = (s <= 0.0) ? 1.0 : q / (1.0 + q);
         double sum;
@@ -986,8 +887,7 @@ __device__ double m_smooth(const W& w, const MFit& f, double s, int max_iter, do
             // nothing stored, followed by a full pass when it converged
             sum = m_light_S(w, f, p);
         } else {
-            sum = m_chol1d(w, f, p, !ys);
-            ys = true;
+            sum = m_chol1d(w, f, p);
         }
         if (s <= 0.0 || stage == kGuessFit) return p;
         const double sfq = 36.0 * sum / ((1.0 + q) * (1.0 + q));
@@ -1053,7 +953,6 @@ __device__ double m_smooth(const W& w, const MFit& f, double s, int max_iter, do
 // (pppack.f90:5303-5316) for piece i, from u and y.
 struct MPiece {
     int i;                          // 0: none yet
-    int j;                          // the column's piece at break i (where y is not stored; 0: none yet)
     double xi, c1, c2, c3, c4;
 };
 
@@ -1067,8 +966,7 @@ __device__ __forceinline__ void m_piece(const W& w, const MFit& f, double p, int
     const double raw1 = (u1 - u0) * f.rh;                            // raw(i+1)
     const double raw2 = (i + 2 <= np) ? (u2 - u1) * f.rh : 0.0;      // raw(i+2)
     const double K1 = 6.0 * (1.0 - p) * f.dy2;
-    const double y0 = (double)w.yat(f, i, pc.j);
-    const double y1 = (double)w.yat(f, i + 1, pc.j);
+    const double y0 = (double)w.y(i), y1 = (double)w.y(i + 1);
     const double a1i = y0 - K1 * (raw1 - raw0);
     const double a1n = y1 - K1 * (raw2 - raw1);
     const double a3i = u0 * 6.0 * p;
@@ -1129,7 +1027,6 @@ __device__ float m_vturb(const RpStepArgs& A, const RpGridDev& g, const MStage& 
     const int sw = g.N + 1;
     MFit f;
     f.np = (int)((double)sw * A.sub);
-    f.sw = sw;
     f.serr = A.serr;
     f.dy2 = A.serr * A.serr;
     const double tdepth = (double)S.tdepth, zeta = (double)S.zeta;
@@ -1141,7 +1038,16 @@ __device__ float m_vturb(const RpStepArgs& A, const RpGridDev& g, const MStage& 
     const float4* qs = reinterpret_cast<const float4*>(g.qs_aks);
     const MTime tk = m_time(A, g, 0);
     const bool all[4] = {true, true, true, true};
-    float z1 = 0.f, zprev = 0.f, kprev = 0.f;
+    // Each piece of the column, [z(k-1), z(k)], gives its points of linint's
+    // resampling (ver_turb_module.f90:126-136) as it is formed: a point's piece is
+    // the last whose lower end is at or below it.  Walked up by the sweeps
+    // instead, the pieces' loads were waited for at nearly every row (some lane
+    // of a warp advances): 345 cycles a row of the forward sweep at 512x384x30 with
+    // 1,048,576 particles, 188 so (an interval 18.5 ms, 17.1).
+    using YT = typename W::YT;
+    YT z1 = 0, hq = 0, x = 0;      // first break, spacing, the point's place
+    int i = 1;                     // the next point
+    float zprev = 0.f, kprev = 0.f;
     // levels in batches of kColBatch: the batch's 4 kColBatch corner loads
     // are issued before any is used, so their latencies overlap (a
     // workspace view for a kernel with registers to spare asks for more)
@@ -1166,16 +1072,22 @@ __device__ float m_vturb(const RpStepArgs& A, const RpGridDev& g, const MStage& 
             const float kk = m_level_of<E>(v[b], sc[b], cwt, all, tk);   // getInterpAKs
             if (k >= 2) {
                 const float m = (kk - kprev) / (zk - zprev);
-                w.set_seg(k - 1, (k == sw) ? CUDART_NAN_F : zk, m, kprev - m * zprev);
+                const YT mi = (YT)m, bi = (YT)(kprev - m * zprev);
+                while (i <= f.np && (k == sw || !((YT)zk <= x))) {
+                    w.y(i) = fma(mi, x, bi);
+                    x = fma((YT)i, hq, z1);
+                    i++;
+                }
             } else {
-                z1 = zk;
+                f.z1 = (double)zk;
+                f.h = (zeta - f.z1) / (double)(f.np - 1);
+                z1 = x = (YT)f.z1;
+                hq = (YT)f.h;
             }
             zprev = zk;
             kprev = kk;
         }
     }
-    f.z1 = (double)z1;
-    f.h = (zeta - f.z1) / (double)(f.np - 1);
     f.rh = 1.0 / f.h;
     int passes;
     const double p = m_smooth(w, f, A.smth, A.spline_max_iter, qstate, gstate, q2state, fl, passes);
@@ -1183,7 +1095,7 @@ __device__ float m_vturb(const RpStepArgs& A, const RpGridDev& g, const MStage& 
     const double deltat = A.deltat;
     double ParZc = (double)Zpar;
     MPiece pc;
-    pc.i = pc.j = 0;
+    pc.i = 0;
     double dev_next = 0.0;
     for (int i = 1; i <= A.loop; i++) {
         double DEV;                                    // draw 1+i; pairs (2,3), (4,5), ...
