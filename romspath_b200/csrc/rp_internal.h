@@ -24,7 +24,7 @@ constexpr int kAdvectMinBlocks = RP_ADVECT_MIN_BLOCKS; // exact form: 128-thread
 #define RP_MIXED_MIN_BLOCKS 4
 #endif
 constexpr int kMixedMinBlocks = RP_MIXED_MIN_BLOCKS;   // same, mixed-precision step with VTurb
-constexpr int kMixedAdvectBlocks = 8;                  // same, without VTurb
+constexpr int kMixedAdvectBlocks = 5;                  // same, without VTurb
 #ifndef RP_MIXED_VT_BLOCKS
 #define RP_MIXED_VT_BLOCKS 2
 #endif
