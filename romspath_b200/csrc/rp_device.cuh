@@ -414,6 +414,31 @@ __device__ __forceinline__ void rp_getcoeff(double X, double Y, const double m[4
 
 // ------------------------------------------------------------- stencils
 
+// The ring slots b, c, f of one (point, level), from one 16-byte load (FP64:
+// two): its four slots lie together.  The spare slot, which an upload may be
+// filling, is read and dropped.
+struct RpSlots {
+    double b, c, f;
+};
+template <typename V>
+__device__ __forceinline__ V rp_pick4(V x, V y, V z, V w, int s) {
+    return (s & 2) ? ((s & 1) ? w : z) : ((s & 1) ? y : x);
+}
+template <typename T>
+__device__ __forceinline__ RpSlots rp_ld_slots(const void* base, int64_t idx, int sb, int sc, int sf);
+template <>
+__device__ __forceinline__ RpSlots rp_ld_slots<float>(const void* base, int64_t idx, int sb, int sc, int sf) {
+    const float4 v = __ldg(reinterpret_cast<const float4*>(base) + idx);
+    return {(double)rp_pick4(v.x, v.y, v.z, v.w, sb), (double)rp_pick4(v.x, v.y, v.z, v.w, sc),
+            (double)rp_pick4(v.x, v.y, v.z, v.w, sf)};
+}
+template <>
+__device__ __forceinline__ RpSlots rp_ld_slots<double>(const void* base, int64_t idx, int sb, int sc, int sf) {
+    const double2 p = __ldg(reinterpret_cast<const double2*>(base) + 2 * idx);
+    const double2 q = __ldg(reinterpret_cast<const double2*>(base) + 2 * idx + 1);
+    return {rp_pick4(p.x, p.y, q.x, q.y, sb), rp_pick4(p.x, p.y, q.x, q.y, sc), rp_pick4(p.x, p.y, q.x, q.y, sf)};
+}
+
 // rho-point cell of (ip, jp): the set-up shared by getInterp2D (depth, pm,
 // pn, zeta), the w/AKs paths of getInterp3D and getInterpAKs.
 struct RhoCell {
@@ -481,6 +506,18 @@ __device__ __forceinline__ double rp_zeta_at(const RpGridDev& g, const RhoCell& 
     const double v2 = rp_ld<T>(g.zeta, c.o11 * RP_SLOTS + slot);
     const double v3 = rp_ld<T>(g.zeta, c.o01 * RP_SLOTS + slot);
     return c.ci[0] * v0 + c.ci[1] * v1 + c.ci[2] * v2 + c.ci[3] * v3;
+}
+
+// the same at the three slots b, c, f
+template <typename T>
+__device__ __forceinline__ RpSlots rp_zeta3(const RpGridDev& g, const RhoCell& c) {
+    const RpSlots v0 = rp_ld_slots<T>(g.zeta, c.o00, g.sb, g.sc, g.sf);
+    const RpSlots v1 = rp_ld_slots<T>(g.zeta, c.o10, g.sb, g.sc, g.sf);
+    const RpSlots v2 = rp_ld_slots<T>(g.zeta, c.o11, g.sb, g.sc, g.sf);
+    const RpSlots v3 = rp_ld_slots<T>(g.zeta, c.o01, g.sb, g.sc, g.sf);
+    return {c.ci[0] * v0.b + c.ci[1] * v1.b + c.ci[2] * v2.b + c.ci[3] * v3.b,
+            c.ci[0] * v0.c + c.ci[1] * v1.c + c.ci[2] * v2.c + c.ci[3] * v3.c,
+            c.ci[0] * v0.f + c.ci[1] * v1.f + c.ci[2] * v2.f + c.ci[3] * v3.f};
 }
 
 // u / v corner set of getInterp3D (interpolation_module.f90:608-767).
@@ -981,3 +1018,25 @@ __device__ __forceinline__ double rp_log(double x) {
     return rp_log_pos(x);
 }
 
+// zcff1*zprof(Ibot) + zcff2*zprof(Itop) at the three slots b, c, f: rp_col_uv's
+// (use: the corners that count) and rp_col_rho's (use null) operations
+template <typename T>
+__device__ __forceinline__ RpSlots rp_col3(const RpGridDev& g, const void* f, const int64_t (&o)[4],
+                                           const double* cff, const bool* use, int nlev, const LevelPick& L) {
+    RpSlots vb[4], vt[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int64_t base = o[k] * nlev;
+        vb[k] = rp_ld_slots<T>(f, base + L.ibot - 1, g.sb, g.sc, g.sf);
+        vt[k] = rp_ld_slots<T>(f, base + L.itop - 1, g.sb, g.sc, g.sf);
+        if (use && !use[k]) vb[k] = vt[k] = {0.0, 0.0, 0.0};
+    }
+    RpSlots r;
+    r.b = L.z1 * (cff[0] * vb[0].b + cff[1] * vb[1].b + cff[2] * vb[2].b + cff[3] * vb[3].b) +
+          L.z2 * (cff[0] * vt[0].b + cff[1] * vt[1].b + cff[2] * vt[2].b + cff[3] * vt[3].b);
+    r.c = L.z1 * (cff[0] * vb[0].c + cff[1] * vb[1].c + cff[2] * vb[2].c + cff[3] * vb[3].c) +
+          L.z2 * (cff[0] * vt[0].c + cff[1] * vt[1].c + cff[2] * vt[2].c + cff[3] * vt[3].c);
+    r.f = L.z1 * (cff[0] * vb[0].f + cff[1] * vb[1].f + cff[2] * vb[2].f + cff[3] * vb[3].f) +
+          L.z2 * (cff[0] * vt[0].f + cff[1] * vt[1].f + cff[2] * vt[2].f + cff[3] * vt[3].f);
+    return r;
+}

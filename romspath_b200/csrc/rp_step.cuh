@@ -109,9 +109,10 @@ __device__ __forceinline__ void rp_find_currents(const RpStepArgs& A, const RpGr
                                                  StageState& S, uint32_t& fl) {
     rp_rho_cell(g, X, Y, S.rc, fl);
     S.tdepth = -1.0 * rp_bil(g.h, S.rc);
-    S.zb = rp_zeta_at<T>(g, S.rc, g.sb);
-    S.zc = rp_zeta_at<T>(g, S.rc, g.sc);
-    S.zf = rp_zeta_at<T>(g, S.rc, g.sf);
+    const RpSlots zt = rp_zeta3<T>(g, S.rc);
+    S.zb = zt.b;
+    S.zc = zt.c;
+    S.zf = zt.f;
     if (Z < S.tdepth) Z = S.tdepth + RP_F_0P001;
     S.zeta = rp_polintd(A.pi, S.zb, S.zc, S.zf);
     if (Z > S.zeta) Z = S.zeta - RP_F_0P001;
@@ -123,40 +124,26 @@ __device__ __forceinline__ void rp_find_currents(const RpStepArgs& A, const RpGr
         return;
     }
     const int N = g.N;
+    // at ets == 1 the values are (b, b, c) (advection_module.f90:277-287)
+    auto in_time = [&](const RpSlots& v) -> double {
+        return (A.ets == 1) ? rp_polintd(A.pi, v.b, v.b, v.c) : rp_polintd(A.pi, v.b, v.c, v.f);
+    };
     {
         UVCell cu;
         rp_u_cell(g, X, Y, cu, fl);
-        const double Ub = rp_col_uv<T>(g.u, cu, N, Lr, g.sb);
-        const double Uc = rp_col_uv<T>(g.u, cu, N, Lr, g.sc);
-        if (A.ets == 1) {
-            Uad = rp_polintd(A.pi, Ub, Ub, Uc);
-        } else {
-            const double Uf = rp_col_uv<T>(g.u, cu, N, Lr, g.sf);
-            Uad = rp_polintd(A.pi, Ub, Uc, Uf);
-        }
+        Uad = in_time(rp_col3<T>(g, g.u, cu.o, cu.cff, cu.use, N, Lr));
     }
     {
         UVCell cv;
         rp_v_cell(g, X, Y, cv, fl);
-        const double Vb = rp_col_uv<T>(g.v, cv, N, Lr, g.sb);
-        const double Vc = rp_col_uv<T>(g.v, cv, N, Lr, g.sc);
-        if (A.ets == 1) {
-            Vad = rp_polintd(A.pi, Vb, Vb, Vc);
-        } else {
-            const double Vf = rp_col_uv<T>(g.v, cv, N, Lr, g.sf);
-            Vad = rp_polintd(A.pi, Vb, Vc, Vf);
-        }
+        Vad = in_time(rp_col3<T>(g, g.v, cv.o, cv.cff, cv.use, N, Lr));
     }
     {
-        const double* cw = S.rc.wet4 ? S.rc.cb : S.rc.ci;
-        const double Wb = rp_col_rho<T>(g.w, S.rc, cw, N + 1, Lw, g.sb);
-        const double Wc = rp_col_rho<T>(g.w, S.rc, cw, N + 1, Lw, g.sc);
-        if (A.ets == 1) {
-            Wad = rp_polintd(A.pi, Wb, Wb, Wc);
-        } else {
-            const double Wf = rp_col_rho<T>(g.w, S.rc, cw, N + 1, Lw, g.sf);
-            Wad = rp_polintd(A.pi, Wb, Wc, Wf);
-        }
+        const int64_t o[4] = {S.rc.o00, S.rc.o10, S.rc.o11, S.rc.o01};
+        double cw[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) cw[k] = S.rc.wet4 ? S.rc.cb[k] : S.rc.ci[k];
+        Wad = in_time(rp_col3<T>(g, g.w, o, cw, nullptr, N + 1, Lw));
     }
 }
 
