@@ -871,7 +871,7 @@ def adjoint_run(args):
                "eps_1e-6_fraction_within_1e-4": float(np.mean(r6 < 1e-4)), "eps_1e-6_median_rel": float(np.median(r6)),
                "eps_1e-3_fraction_within_1e-4": float(np.mean(r3 < 1e-4)), "eps_1e-3_median_rel": float(np.median(r3))},
            "note": "times include the host loop over steps; backward = recompute of each 48-step segment from its "
-                   "checkpoint + reverse steps (per-step Jacobians by 4-direction dual numbers)"}
+                   "checkpoint + reverse steps (VTurb's reverse by hand, the rest by 3-direction dual numbers)"}
     T.close()
     del ev
     print(json.dumps(out), flush=True)

@@ -1,8 +1,8 @@
 // rp_adjoint.cu -- kernels of the adjoint pair (rp_forward / rp_backward),
 // the tangent-linear reference and the replay used by finite differences.
-// All of them run the one generic step of rp_adjoint.cuh; compiled without
-// FMA contraction so that the double and the dual instantiations take the
-// same values.
+// The steps run the generic step of rp_adjoint.cuh, with VTurb's displacements
+// (and their derivatives) from kernels of their own; compiled without FMA
+// contraction so that a replayed step takes its forward step's bits.
 #include <cuda_runtime.h>
 
 #include "rp_internal.h"
@@ -14,7 +14,6 @@ constexpr int kAdjBlock = 128;
 constexpr int kAdjVtBlock = 64;
 constexpr int kAdjStepBlocks = 4;      // blocks of the steps in doubles and in dual numbers an SM
 constexpr int kAdjReverseBlocks = 3;
-
 
 __device__ __forceinline__ void adj_load(const AdjStateDev& s, int64_t n, double& x, double& y, double& z,
                                          AdjAux& a) {
