@@ -37,11 +37,11 @@ __device__ __forceinline__ void adj_store_aux(const AdjStateDev& s, int64_t n, c
 // record it in prec[n], else use prec[n].
 //
 // Bound by the fit's chains of dependent FP64 operations (a pivot, its
-// reciprocal, the next pivot): 64-thread blocks, eight an SM, hold 65,536
-// particles in one wave; the search's seven or so passes store nothing.  On the
-// 130x98x20 grid with 65,536 particles a forward step (this kernel and the
-// rest) takes 0.29 ms, 1.5 in one kernel whose passes kept their factor and
-// divided three times a row.
+// reciprocal, the next pivot) and the traffic of the passes' factor and u:
+// 64-thread blocks, eight an SM, hold 65,536 particles in one wave.  On the
+// 130x98x20 grid with 65,536 particles a forward step (this kernel, 0.50 ms, and
+// the rest) takes 0.57 ms, 1.5 in one kernel whose passes divided three times a
+// row by the IEEE operator; a replayed step, one pass, 0.18 ms.
 template <int NPMAX>
 __global__ void __launch_bounds__(kAdjVtBlock, 512 / kAdjVtBlock)
     k_adj_vturb(const __grid_constant__ RpStepArgs A, const __grid_constant__ AdjFrames F, AdjStateDev s,

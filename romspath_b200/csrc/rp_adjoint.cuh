@@ -729,108 +729,47 @@ __device__ __forceinline__ void b_column(const RpStepArgs& A, const AdjFrames& F
     }
 }
 
-// chol1d's sum S(p) = sum qu^2 dy^2 and smooth's utru (which the search needs
-// at p = 0) from one forward sweep, with nothing stored and no back
-// substitution.  With M(p) = 6(1-p) T + p R the matrix of chol1d and b = Q'y,
-// phi(p) = b'M^-1 b = sum_i w_i^2 / d_i over the forward-substituted values w
-// and the pivots d; u'Mu = phi and dphi/dp = -u'M'u = 6 u'Tu - u'Ru, so that
-//   S = u'Tu = (phi + p phi') / 6,   at p = 0:  utru = u'Ru / 2 = (phi - phi') / 2,
-// and phi' is carried through the sweep as derivatives in p of the factor and
-// of w.  A row is one chain (pivot, reciprocal, ratio, pivot).
-template <class W>
-__device__ __forceinline__ void b_light(const W& w, const BPar& B, double p, double& sum, double& utru) {
+// The pass below with every quotient left to the IEEE operator, for fits whose
+// operands leave the shared-reciprocal division's range (NaN frames, a zero or
+// a tiny data weight).
+template <bool REV, class W>
+__device__ __noinline__ void b_solve_ieee(const W w, const BPar& B, double p) {
     const int np = B.np;
     double D, E, F;
     B.bands(p, D, E, F);
-    const double Dd = -36.0 * B.r2 + 4.0 * B.hb, Ed = 24.0 * B.r2 + B.hb, Fd = -6.0 * B.r2;
-    double a1 = D, a2 = E, b1 = D, a1d = Dd, a2d = Ed, b1d = Dd;
-    double y0 = w.y(2), yp = w.y(3);
-    double wc = (yp - 2.0 * y0 + w.y(1)) * B.rh, wcd = 0.0, wp = 0.0, wpd = 0.0;   // w(i), w(i-1) and d/dp
-    double r2p = 0.0, r2pd = 0.0;                                                  // ratio2(i-1)
-    double phi = 0.0, phid = 0.0;
-    auto row = [&](double yn, double Fi, double Fid) {
-        const double inv = rp_rcp_ulp(a1);
-        const double invd = -(a1d * inv) * inv;
-        const double wi = wc * inv;
-        phi = fma(wc, wi, phi);
-        phid = fma(2.0 * wcd, wi, fma(wc * wc, invd, phid));
-        const double q1 = a2 * inv, q1d = fma(a2d, inv, a2 * invd);
-        const double q2 = Fi * inv, q2d = fma(Fid, inv, Fi * invd);
-        const double a1n = fma(-q1, a2, b1);
-        const double a1dn = fma(-q1d, a2, fma(-q1, a2d, b1d));
-        a2 = fma(-q1, Fi, E);
-        a2d = fma(-q1d, Fi, fma(-q1, Fid, Ed));
-        b1 = fma(-q2, Fi, D);
-        b1d = fma(-q2d, Fi, fma(-q2, Fid, Dd));
-        a1 = a1n;
-        a1d = a1dn;
-        const double qn = (yn - 2.0 * yp + y0) * B.rh;                             // qty(i+1)
-        y0 = yp;
-        yp = yn;
-        const double wn = fma(-r2p, wp, fma(-q1, wc, qn));
-        const double wnd = -fma(q1d, wc, fma(q1, wcd, fma(r2pd, wp, r2p * wpd)));
-        wp = wc;
-        wpd = wcd;
-        wc = wn;
-        wcd = wnd;
+    double a1 = D, a2 = E, b1 = D;
+    double uc = (w.y(3) - 2.0 * w.y(2) + w.y(1)) * B.rh, up = 0.0, r2p = 0.0;
+    for (int i = 2; i <= np - 2; i++) {
+        const double Fi = (i <= np - 3) ? F : 0.0;
+        const double q1 = a2 / a1, q2 = Fi / a1;
+        w.s1(i) = q1;
+        w.s2(i) = q2;
+        w.u(i) = uc / a1;
+        if (REV) w.inv(i) = 1.0 / a1;
+        a1 = b1 - q1 * a2;
+        a2 = E - q1 * Fi;
+        b1 = D - q2 * Fi;
+        const double qn = (w.y(i + 2) - 2.0 * w.y(i + 1) + w.y(i)) * B.rh;
+        const double un = qn - q1 * uc - r2p * up;
+        up = uc;
+        uc = un;
         r2p = q2;
-        r2pd = q2d;
-    };
-    int i = 2;
-#pragma unroll 1
-    for (; i + 3 <= np - 3; i += 4) {            // the rows' data read together
-        const double ya = w.y(i + 2), yb = w.y(i + 3), yc = w.y(i + 4), yd = w.y(i + 5);
-        row(ya, F, Fd);
-        row(yb, F, Fd);
-        row(yc, F, Fd);
-        row(yd, F, Fd);
     }
-#pragma unroll 1
-    for (; i <= np - 2; i++) row(w.y(i + 2), i <= np - 3 ? F : 0.0, i <= np - 3 ? Fd : 0.0);
-    {                                                                              // row np-1
-        const double inv = rp_rcp_ulp(a1);
-        const double invd = -(a1d * inv) * inv;
-        const double wi = wc * inv;
-        phi = fma(wc, wi, phi);
-        phid = fma(2.0 * wcd, wi, fma(wc * wc, invd, phid));
-    }
-    sum = fma(p, phid, phi) * (1.0 / 6.0);
-    utru = 0.5 * (phi - phid);
+    if (REV) w.inv(np - 1) = 1.0 / a1;
+    w.u(np) = 0.0;
+    w.u(np - 1) = uc / a1;
+    for (int i = np - 2; i >= 2; i--) w.u(i) = w.u(i) - w.u(i + 1) * w.s1(i) - w.u(i + 2) * w.s2(i);
+    w.u(1) = 0.0;
 }
 
-// smooth()'s secant search for p (pppack.f90:5108-5317, reference cold
-// start) on uniform breaks
-template <class W>
-__device__ __forceinline__ double b_find_p(const W& w, const BPar& B, double s, int max_iter, uint32_t& fl) {
-    if (s <= 0.0) return 1.0;
-    const double ooss = 1.0 / sqrt(s);
-    double q = 0.0, prevq = 0.0, prevsf = 0.0;
-#pragma unroll 1
-    for (int it = 0;; it++) {
-        const double p = q / (1.0 + q);
-        double sum, utru;
-        b_light(w, B, p, sum, utru);
-        const double sfq = 36.0 * sum / ((1.0 + q) * (1.0 + q));
-        const double oosf = 1.0 / sqrt(sfq);
-        if (it == 0) {
-            if (!(s < sfq)) return 0.0;
-            q = -(oosf - ooss) * sfq / (6.0 * utru * oosf);
-        } else {
-            if (fabs(sfq - s) <= 0.01 * s) return p;
-            if (it >= max_iter) {
-                fl |= RP_FL_SPLINE;
-                return p;
-            }
-            const double change = (q - prevq) / (oosf - prevsf) * (oosf - ooss);
-            prevq = q;
-            q = q - change;
-        }
-        prevsf = oosf;
-    }
-}
-
-// chol1d (pppack.f90:1428-1566) at p; leaves u(1..np), the ratios and, REV,
-// the pivots' reciprocals
+// chol1d (pppack.f90:1428-1566) at p: leaves u(1..np), the ratios and, REV,
+// the pivots' reciprocals.
+//
+// The operations are a_chol1d's, in its order, the three quotients of a row
+// correctly rounded on one reciprocal of the pivot; as in rp_chol1d a row holds
+// no branch and the pass is made again by the IEEE operator where an operand
+// was out of that division's range.  A row is one chain (pivot, reciprocal,
+// ratio, pivot).
 template <bool REV, class W>
 __device__ __forceinline__ void b_solve(const W& w, const BPar& B, double p) {
     const int np = B.np;
@@ -839,27 +778,30 @@ __device__ __forceinline__ void b_solve(const W& w, const BPar& B, double p) {
     double a1 = D, a2 = E, b1 = D;
     double y0 = w.y(2), yp = w.y(3);
     double uc = (yp - 2.0 * y0 + w.y(1)) * B.rh, up = 0.0, r2p = 0.0;
+    uint32_t off = rp_exp_off_z(F), ones = 0;
     auto row = [&](int i, double yn, double Fi) {
-        const double inv = rp_rcp_ulp(a1);
-        const double q1 = a2 * inv, q2 = Fi * inv;
+        off = max(max(off, rp_exp_off(a1)), max(rp_exp_off_z(a2), rp_exp_off_z(uc)));
+        ones = max(ones, rp_ones(a1));
+        const RpRcp y = rp_rcp3(a1);
+        const double q1 = rp_div_rcp(a2, a1, y), q2 = rp_div_rcp(Fi, a1, y);
         w.s1(i) = q1;
         w.s2(i) = q2;
-        w.u(i) = uc * inv;
-        if (REV) w.inv(i) = inv;
-        a1 = fma(-q1, a2, b1);
-        a2 = fma(-q1, Fi, E);
-        b1 = fma(-q2, Fi, D);
+        w.u(i) = rp_div_rcp(uc, a1, y);
+        if (REV) w.inv(i) = y.y;
+        a1 = b1 - q1 * a2;
+        a2 = E - q1 * Fi;
+        b1 = D - q2 * Fi;
         const double qn = (yn - 2.0 * yp + y0) * B.rh;
         y0 = yp;
         yp = yn;
-        const double un = fma(-r2p, up, fma(-q1, uc, qn));
+        const double un = qn - q1 * uc - r2p * up;
         up = uc;
         uc = un;
         r2p = q2;
     };
     int i = 2;
 #pragma unroll 1
-    for (; i + 3 <= np - 3; i += 4) {
+    for (; i + 3 <= np - 3; i += 4) {            // the rows' data read together
         const double ya = w.y(i + 2), yb = w.y(i + 3), yc = w.y(i + 4), yd = w.y(i + 5);
         row(i, ya, F);
         row(i + 1, yb, F);
@@ -868,9 +810,12 @@ __device__ __forceinline__ void b_solve(const W& w, const BPar& B, double p) {
     }
 #pragma unroll 1
     for (; i <= np - 2; i++) row(i, w.y(i + 2), i <= np - 3 ? F : 0.0);
-    const double inv = rp_rcp_ulp(a1);
-    if (REV) w.inv(np - 1) = inv;
-    double u2 = 0.0, u1 = uc * inv;              // u(i+2), u(i+1)
+    if (off >= kDivSpan || ones == 0xffffffffu) {
+        b_solve_ieee<REV>(w, B, p);
+        return;
+    }
+    if (REV) w.inv(np - 1) = rp_rcp(a1);
+    double u2 = 0.0, u1 = uc / a1;               // u(i+2), u(i+1)
     w.u(np) = 0.0;
     w.u(np - 1) = u1;
     w.u(1) = 0.0;
@@ -886,17 +831,91 @@ __device__ __forceinline__ void b_solve(const W& w, const BPar& B, double p) {
         }
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            const double ui = fma(-u1, q1[k], fma(-u2, q2[k], v[k]));
+            const double ui = v[k] - u1 * q1[k] - u2 * q2[k];
             w.u(i - k) = ui;
             u2 = u1;
             u1 = ui;
         }
     }
     for (; i >= 2; i--) {
-        const double ui = fma(-u1, w.s1(i), fma(-u2, w.s2(i), w.u(i)));
+        const double ui = w.u(i) - u1 * w.s1(i) - u2 * w.s2(i);
         w.u(i) = ui;
         u2 = u1;
         u1 = ui;
+    }
+}
+
+// sum qu^2 dy^2 of the pass just made, qu = Q u, in the reference's order.
+// (From the forward sweep alone, as (phi + p phi') / 6 of phi(p) = b'M^-1 b,
+// it needs no back substitution but cancels: with the data's weight at 1e-4
+// and spacings of 0.02 to 50 m its error was up to 4e-4 where this sum's is
+// 1e-9, with 1e-6 up to 2.5.)
+template <class W>
+__device__ __forceinline__ double b_sum(const W& w, const BPar& B) {
+    const int np = B.np;
+    const double dy2 = B.serr * B.serr;
+    double prev = 0.0, sum = 0.0, ul = 0.0;      // raw(i), u(i)
+    auto term = [&](double ui) {
+        const double raw = (ui - ul) * B.rh;
+        const double fin = raw - prev;
+        sum = sum + fin * fin * dy2;
+        prev = raw;
+        ul = ui;
+    };
+    int i = 2;
+#pragma unroll 1
+    for (; i + 3 <= np; i += 4) {
+        const double ua = w.u(i), ub = w.u(i + 1), uc = w.u(i + 2), ud = w.u(i + 3);
+        term(ua);
+        term(ub);
+        term(uc);
+        term(ud);
+    }
+    for (; i <= np; i++) term(w.u(i));
+    return sum + prev * prev * dy2;
+}
+
+// utru (pppack.f90:5219-5223) of the pass just made
+template <class W>
+__device__ __forceinline__ double b_utru(const W& w, const BPar& B) {
+    double utru = 0.0, ul = 0.0;
+    for (int i = 2; i <= B.np; i++) {
+        const double ui = w.u(i);
+        utru = utru + B.hb * (ul * (ul + ui) + ui * ui);
+        ul = ui;
+    }
+    return utru;
+}
+
+// The fit at p; find: at the p of smooth()'s secant search (pppack.f90:
+// 5108-5317, reference cold start).  Returns p; the last pass made is p's.
+template <class W>
+__device__ __forceinline__ double b_fit(const W& w, const BPar& B, bool find, double p, double s, int max_iter,
+                                        uint32_t& fl) {
+    if (find) p = (s <= 0.0) ? 1.0 : 0.0;
+    const double ooss = 1.0 / sqrt(s);
+    double q = 0.0, prevq = 0.0, prevsf = 0.0;
+#pragma unroll 1
+    for (int it = 0;; it++) {
+        b_solve<false>(w, B, p);
+        if (!find || s <= 0.0) return p;
+        const double sfq = 36.0 * b_sum(w, B) / ((1.0 + q) * (1.0 + q));
+        const double oosf = 1.0 / sqrt(sfq);
+        if (it == 0) {
+            if (!(s < sfq)) return p;
+            q = -(oosf - ooss) * sfq / (6.0 * b_utru(w, B) * oosf);
+        } else {
+            if (fabs(sfq - s) <= 0.01 * s) return p;
+            if (it >= max_iter) {
+                fl |= RP_FL_SPLINE;
+                return p;
+            }
+            const double change = (q - prevq) / (oosf - prevsf) * (oosf - ooss);
+            prevq = q;
+            q = q - change;
+        }
+        prevsf = oosf;
+        p = q / (1.0 + q);
     }
 }
 
@@ -1032,8 +1051,7 @@ __device__ __forceinline__ double b_vturb(const RpStepArgs& A, const AdjFrames& 
     BPar B;
     bool asc;
     b_column(A, F, gi, St, kappa, w, B, asc);
-    if (find) p = b_find_p(w, B, A.smth, A.spline_max_iter, fl);
-    b_solve<false>(w, B, p);
+    p = b_fit(w, B, find, p, A.smth, A.spline_max_iter, fl);
     double z = Z, dev, dev_next = 0.0;
     BPiece c;
     c.i = 0;
