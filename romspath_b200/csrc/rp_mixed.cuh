@@ -643,7 +643,7 @@ __device__ __forceinline__ double m_chol1d(const W& w, const MFit& f, double p) 
     bool held = false;
     float hinv = 0.f, h1 = 0.f, h2 = 0.f;
     auto factor = [&](float& inv, float& ratio1, float& ratio2) {
-        const double invd = rp_rcp_ulp(a1);               // one reciprocal per row
+        const double invd = rp_rcp_in(a1);           // one reciprocal per row
         const double ratio1d = a2 * invd, ratio2d = F * invd;
         a1 = b1 - ratio1d * a2;
         a2 = E - ratio1d * F;
@@ -708,7 +708,7 @@ __device__ __forceinline__ double m_chol1d(const W& w, const MFit& f, double p) 
         w.u(i) = forward(inv, ratio1, ratio2, (float)w.y(i + 2));
     }
     // row np-2 (F = 0) and u(np-1)
-    const double invl = rp_rcp_ulp(a1);
+    const double invl = rp_rcp_in(a1);
     const double ratiol = a2 * invl;
     const float q1l = (float)ratiol;
     const float ul = forward((float)invl, q1l, 0.f, (float)w.y(np));
