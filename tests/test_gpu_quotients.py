@@ -14,7 +14,8 @@ pytestmark = pytest.mark.gpu
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(HERE), "romspath_b200", "csrc")
-OUT = ["rcp", "rcp_in", "rcp3"]
+P = C.POINTER(C.c_double)
+OUT = ["rcp", "rcp_in", "rcp3", "quot", "div_by", "div_rcp", "div_fast"]
 
 
 def _operands(rng, n):
@@ -57,18 +58,23 @@ def _same(x, y):
 
 
 @pytest.fixture(scope="module")
-def run(tmp_path_factory):
+def lib(tmp_path_factory):
     so = str(tmp_path_factory.mktemp("quot") / "quot.so")
     subprocess.run(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-fmad=false", "-shared",
                     "-Xcompiler", "-fPIC", "-I", CSRC, os.path.join(HERE, "gpu_quot_selftest.cu"), "-o", so],
                    check=True)
     L = C.CDLL(so)
-    P = C.POINTER(C.c_double)
     L.quot_selftest.argtypes = [C.c_int64, P, P, P]
+    L.polint_selftest.argtypes = [C.c_int64, P, C.c_double, C.c_int, P, P, P]
+    return L
+
+
+@pytest.fixture(scope="module")
+def run(lib):
     n = 1 << 22
     a, b = _operands(np.random.default_rng(17), n)
     out = np.empty((len(OUT), n))
-    assert L.quot_selftest(n, *[v.ctypes.data_as(P) for v in (a, b, out)]) == 0
+    assert lib.quot_selftest(n, *[v.ctypes.data_as(P) for v in (a, b, out)]) == 0
     return a, b, dict(zip(OUT, out))
 
 
@@ -81,3 +87,46 @@ def test_reciprocals(run):
     assert ok.sum() > b.size // 2
     for k in ("rcp_in", "rcp3"):
         assert _same(out[k][ok], want[ok]).all(), k
+
+
+def test_quotients(run):
+    a, b, out = run
+    with np.errstate(all="ignore"):
+        want = a / b
+    assert _same(out["quot"], want).all()
+    assert _same(out["div_by"], want).all()
+    ok = _in_range(a) & _in_range(b) & ~_all_ones(b)
+    assert ok.sum() > b.size // 2
+    for k in ("div_rcp", "div_fast"):
+        assert _same(out[k][ok], want[ok]).all(), k
+    zero = (a == 0.0) & _in_range(b) & ~_all_ones(b)       # a zero of either sign
+    assert zero.any()
+    for k in ("div_rcp", "div_fast"):
+        assert (out[k][zero] == 0.0).all(), k
+
+
+# nodes and place as a run meets them (frames an hour apart, the nearest node each
+# in turn), and frame times whose differences leave the helpers' range
+@pytest.mark.parametrize("xa,x,ns", [
+    ((0.0, 3600.0, 7200.0), 3900.0, 1), ((0.0, 3600.0, 7200.0), 300.0, 0), ((0.0, 3600.0, 7200.0), 6900.0, 2),
+    ((3600.0, 7200.0, 10800.0), 7200.0, 1), ((0.0, 1e-160, 3e-160), 1.1e-160, 1), ((0.0, 3600.0, 7200.0), 3600.0, 1)])
+def test_polintd_pair(lib, xa, x, ns):
+    rng = np.random.default_rng(5)
+    n = 1 << 18
+    u = rng.uniform(-1.0, 1.0, (3, n)) * 10.0 ** rng.uniform(-8, 3, n)
+    v = rng.uniform(-1.0, 1.0, (3, n)) * 10.0 ** rng.uniform(-8, 3, n)
+    k = n // 8
+    u[:, :k] = u[0, :k]                                     # no change in time
+    v[1, k:2 * k] = v[0, k:2 * k]
+    u[:, 2 * k:3 * k] = 0.0
+    v[:, 3 * k:4 * k] *= 1e-200                             # one of the pair out of range
+    u[2, 4 * k:4 * k + 9] = np.nan
+    v[1, 4 * k + 9:4 * k + 18] = np.inf
+    u[:, 5 * k:5 * k + 9] = 5e-324
+    r = np.empty((4, n))
+    t = np.array(xa)
+    args = [np.ascontiguousarray(q) for q in (u, v)]
+    assert lib.polint_selftest(n, t.ctypes.data_as(P), x, ns, *[q.ctypes.data_as(P) for q in args],
+                               r.ctypes.data_as(P)) == 0
+    for got, want in ((r[0], r[2]), (r[1], r[3])):
+        assert np.array_equal(got, want, equal_nan=True)
