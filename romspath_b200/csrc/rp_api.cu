@@ -536,15 +536,21 @@ int sort_buffers(rp_ctx* ctx) {
     A.ngrid = ctx->ngrid;
     fill_grids(ctx, A, 1, 1, 1);
     uint32_t gb[RP_MAXNGRID] = {};
-    ctx->sb.nkeys = rp::sort_key_count(A, gb);
-    if (ctx->sb.nkeys > rp::kSortMaxKeys)
+    rp::SortBufs b;
+    b.nkeys = rp::sort_key_count(A, gb);
+    if (b.nkeys > rp::kSortMaxKeys)
         return fail(ctx, RP_ERR_UNSUPPORTED, "re-sort: grids exceed 1,048,576 cells in all");
     const size_t cap = (size_t)ctx->cap;
-    if (dalloc(&ctx->sb.keys, cap * 4) || dalloc(&ctx->sb.perm, cap * 4) ||
-        dalloc(&ctx->sb.hist, (size_t)ctx->sb.nkeys * 4) || dalloc(&ctx->sb.sums, 1024 * 4) ||
-        dalloc(&ctx->sb.gbase, sizeof(gb)))
-        return fail(ctx, RP_ERR_NOMEM, "re-sort buffers");
-    CK(cudaMemcpy(ctx->sb.gbase, gb, sizeof(gb), cudaMemcpyHostToDevice));
+    // all or none: `keys` alone says that they are there
+    const bool have = !dalloc(&b.keys, cap * 4) && !dalloc(&b.perm, cap * 4) && !dalloc(&b.hist, (size_t)b.nkeys * 4) &&
+                      !dalloc(&b.sums, 1024 * 4) && !dalloc(&b.gbase, sizeof(gb));
+    if (!have || cudaMemcpy(b.gbase, gb, sizeof(gb), cudaMemcpyHostToDevice) != cudaSuccess) {
+        const char* why = cudaGetErrorString(cudaGetLastError());
+        void* got[] = {b.keys, b.perm, b.hist, b.sums, b.gbase};
+        for (void* p : got) if (p) cudaFree(p);
+        return fail(ctx, have ? RP_ERR_CUDA : RP_ERR_NOMEM, std::string("re-sort buffers: ") + why);
+    }
+    ctx->sb = b;
     return RP_OK;
 }
 
