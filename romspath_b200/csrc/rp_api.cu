@@ -1597,6 +1597,7 @@ int rp_forward(rp_ctx* ctx, int32_t nsteps, const rp_adj_step* steps, double kap
     const int64_t n = ctx->n;
     const int nseg = (nsteps + checkpoint_every - 1) / checkpoint_every;
     const size_t blk = adj_block_bytes(n);
+    J.steps.clear();               // the record is this run's once it is whole
     // the buffers are kept from one run to the next that they hold
     if (n != J.cap_n || nseg > J.cap_seg || nsteps > J.cap_steps || checkpoint_every > J.cap_ckpt) {
         double** bufs[] = {&J.ck, &J.prec, &J.seg, &J.work, &J.lx, &J.ly, &J.lz, &J.kbar, &J.tan, &J.tv};
@@ -1604,7 +1605,6 @@ int rp_forward(rp_ctx* ctx, int32_t nsteps, const rp_adj_step* steps, double kap
             if (*b) cudaFree(*b);
             *b = nullptr;
         }
-        J.steps.clear();
         J.cap_n = -1;
         if (dalloc(&J.ck, blk * (size_t)(nseg + 1)) || dalloc(&J.prec, (size_t)nsteps * n * 8) ||
             dalloc(&J.seg, blk * (size_t)checkpoint_every) || dalloc(&J.work, blk) || dalloc(&J.lx, (size_t)n * 8) ||
@@ -1616,10 +1616,6 @@ int rp_forward(rp_ctx* ctx, int32_t nsteps, const rp_adj_step* steps, double kap
         J.cap_steps = nsteps;
         J.cap_ckpt = checkpoint_every;
     }
-    J.steps.assign(steps, steps + nsteps);
-    J.ckpt = checkpoint_every;
-    J.n = n;
-    J.kappa = kappa;
     cudaStream_t s = ctx->s_comp;
     rp::AdjStateDev cur = adj_ctx_state(ctx);
     int since = -1, rc;
@@ -1628,7 +1624,7 @@ int rp_forward(rp_ctx* ctx, int32_t nsteps, const rp_adj_step* steps, double kap
             CK(adj_copy(cur, adj_view((char*)J.ck + blk * (size_t)(k / checkpoint_every), n), n, s));
         RpStepArgs A;
         AdjFrames F;
-        adj_args(ctx, J.steps[k], A, F, n);
+        adj_args(ctx, steps[k], A, F, n);
         if ((rc = adj_order(ctx, A, cur, n, since)) != RP_OK) return rc;
         CK(rp::launch_adj(0, A, F, cur, J.prec + (size_t)k * n, 1, kappa, J.tv, nullptr, nullptr, nullptr, nullptr, nullptr,
                           ctx->npmax, s, ctx->num_sms));
@@ -1636,6 +1632,10 @@ int rp_forward(rp_ctx* ctx, int32_t nsteps, const rp_adj_step* steps, double kap
     }
     CK(adj_copy(cur, adj_view((char*)J.ck + blk * (size_t)nseg, n), n, s));   // final state
     CK(cudaStreamSynchronize(s));
+    J.steps.assign(steps, steps + nsteps);
+    J.ckpt = checkpoint_every;
+    J.n = n;
+    J.kappa = kappa;
     return RP_OK;
 }
 

@@ -80,3 +80,42 @@ def test_resort_buffers_are_all_or_none(fake, tracker, k):
     for _ in range(3):
         T.step((0.0, 3600.0, 7200.0), (0.0, 300.0, 600.0), 2, 1, 2, 3)
     assert fake.fake_sorts() == 1 and fake.fake_null_bufs() == 0
+
+
+def _adjoint(T, nsteps):
+    from romspath_b200.adjoint import Adjoint, step_table
+    case = harness.make_case("tiny", 16, seed=1)
+    A = Adjoint(T)
+    A.load_frames(3, lambda ng, k: case.frame(k, ng))
+    return A, step_table(2.0, int(case.params["dt"]), int(case.params["idt"]))[0][:nsteps]
+
+
+@pytest.mark.parametrize("where", ["first", "later", "second run"])
+def test_failed_forward_leaves_no_record(fake, tracker, where):
+    T = tracker(64)
+    A, steps = _adjoint(T, 6)
+    z = np.zeros(64)
+    if where == "second run":
+        A.forward(steps, checkpoint_every=3)
+        A.backward(z, z, z)
+    fake.fake_fail_adj(0 if where == "first" else 4)
+    with pytest.raises(Exception, match="ERR_CUDA"):
+        A.forward(steps, checkpoint_every=3)
+    A.n = 64
+    fake.fake_reset()
+    for use in (lambda: A.backward(z, z, z), lambda: A.replay(kappa=1.0), lambda: A.tangent(1.0)):
+        with pytest.raises(Exception, match="ERR_STATE.*call rp_forward first"):
+            use()
+    assert fake.fake_adj() == 0
+    A.forward(steps, checkpoint_every=3)
+    A.backward(z, z, z)
+
+
+def test_refused_forward_keeps_the_record(fake, tracker):
+    T = tracker(64)
+    A, steps = _adjoint(T, 6)
+    z = np.zeros(64)
+    A.forward(steps, checkpoint_every=3)
+    with pytest.raises(Exception, match="ERR_ARG"):
+        A.forward(steps, checkpoint_every=0)
+    A.backward(z, z, z)
