@@ -596,16 +596,23 @@ cudaError_t adj_copy(const rp::AdjStateDev& a, const rp::AdjStateDev& b, int64_t
 // grid and cell as they lie now, kept for kAdjOrderSteps launches (a particle
 // crosses a few tenths of a cell meanwhile).  130x98x20 with 65,536 particles:
 // 24 steps forward and back 33.5 ms, 38.6 as they lie.  Few particles are bound by latency, not by their
-// gathers, and stay as they lie.
+// gathers, and stay as they lie.  So do all where there is no memory for the
+// order's buffers: since = kAdjAsTheyLie for the rest of the call.
 constexpr int kAdjOrderSteps = 12;
 constexpr int64_t kAdjOrderMin = 8192;
+constexpr int kAdjAsTheyLie = -2;
 int adj_order(rp_ctx* ctx, const RpStepArgs& A0, rp::AdjStateDev& s, int64_t n, int& since) {
     s.order = nullptr;
     uint32_t gb[RP_MAXNGRID] = {};
-    if (n < kAdjOrderMin || rp::sort_key_count(A0, gb) > rp::kSortMaxKeys) return RP_OK;
+    if (since == kAdjAsTheyLie || n < kAdjOrderMin || rp::sort_key_count(A0, gb) > rp::kSortMaxKeys) return RP_OK;
     if (since < 0 || since >= kAdjOrderSteps) {
-        int rc, nl = 0;
-        if ((rc = sort_buffers(ctx)) != RP_OK) return rc;
+        const int rc = sort_buffers(ctx);
+        if (rc == RP_ERR_NOMEM) {
+            since = kAdjAsTheyLie;
+            return RP_OK;
+        }
+        if (rc != RP_OK) return rc;
+        int nl = 0;
         RpStepArgs A = A0;
         A.p.x = s.x; A.p.y = s.y; A.p.gid = s.gid;
         CK(rp::launch_order(A, 0, ctx->sb, ctx->s_comp, &nl));

@@ -119,3 +119,20 @@ def test_refused_forward_keeps_the_record(fake, tracker):
     with pytest.raises(Exception, match="ERR_ARG"):
         A.forward(steps, checkpoint_every=0)
     A.backward(z, z, z)
+
+
+# the order by cell is a speed-up: without the memory for it the particles are taken as they lie
+@pytest.mark.parametrize("k", range(5))
+def test_forward_goes_on_without_its_order(fake, tracker, k):
+    n = 8192
+    T = tracker(n)
+    A, steps = _adjoint(T, 14)
+    z = np.zeros(n)
+    fake.fake_fail_malloc(10 + k, 1)                   # the run's ten buffers and k of the order's, then no more
+    A.forward(steps, checkpoint_every=7)
+    A.backward(z, z, z)
+    A.replay()
+    assert fake.fake_ordered() == 0 and fake.fake_sorts() == 0 and fake.fake_adj() == 14 + 12 + 14 + 14
+    fake.fake_reset()
+    A.forward(steps, checkpoint_every=7)               # memory is there again
+    assert fake.fake_ordered() == 14 and fake.fake_null_bufs() == 0
