@@ -1605,8 +1605,11 @@ int rp_forward(rp_ctx* ctx, int32_t nsteps, const rp_adj_step* steps, double kap
     const int nseg = (nsteps + checkpoint_every - 1) / checkpoint_every;
     const size_t blk = adj_block_bytes(n);
     J.steps.clear();               // the record is this run's once it is whole
-    // the buffers are kept from one run to the next that they hold
-    if (n != J.cap_n || nseg > J.cap_seg || nsteps > J.cap_steps || checkpoint_every > J.cap_ckpt) {
+    // the buffers are kept from one run to the next that they hold, unless it
+    // needs less than half of them
+    auto size = [&](int seg, int st, int ck) { return blk * ((size_t)seg + 2 + ck) + (size_t)n * 8 * ((size_t)st + 21); };
+    if (n != J.cap_n || nseg > J.cap_seg || nsteps > J.cap_steps || checkpoint_every > J.cap_ckpt ||
+        size(J.cap_seg, J.cap_steps, J.cap_ckpt) > 2 * size(nseg, nsteps, checkpoint_every)) {
         double** bufs[] = {&J.ck, &J.prec, &J.seg, &J.work, &J.lx, &J.ly, &J.lz, &J.kbar, &J.tan, &J.tv};
         for (double** b : bufs) {
             if (*b) cudaFree(*b);

@@ -136,3 +136,20 @@ def test_forward_goes_on_without_its_order(fake, tracker, k):
     fake.fake_reset()
     A.forward(steps, checkpoint_every=7)               # memory is there again
     assert fake.fake_ordered() == 14 and fake.fake_null_bufs() == 0
+
+
+# what a long run needed is not held through short ones: no more than twice what the run needs stays
+@pytest.mark.parametrize("first,second", [((12, 12), (3, 3)), ((12, 1), (3, 1)), ((12, 12), (12, 1)), ((6, 3), (6, 3)),
+                                          ((6, 3), (5, 3))])
+def test_kept_adjoint_buffers_are_bounded(fake, tracker, first, second):
+    n = 256
+    T = tracker(n)
+    A, steps = _adjoint(T, 12)
+    z = np.zeros(n)
+    empty = fake.fake_bytes()
+    A.forward(steps[:second[0]], checkpoint_every=second[1])
+    need = fake.fake_bytes() - empty
+    A.forward(steps[:first[0]], checkpoint_every=first[1])
+    A.forward(steps[:second[0]], checkpoint_every=second[1])
+    A.backward(z, z, z)
+    assert fake.fake_bytes() - empty <= 2 * need
