@@ -244,12 +244,14 @@ static unsigned adj_grid(K kernel, int64_t n, int num_sms, int block) {
 template <int NPMAX>
 static cudaError_t adj_launch_t(int kind, const RpStepArgs& A, const AdjFrames& F, const AdjStateDev& s,
                                 double* prec, int find, double kappa, double* tv, double* t, double* lx, double* ly,
-                                double* lz, double* kbar, cudaStream_t st, int num_sms) {
+                                double* lz, double* kbar, cudaStream_t st, int num_sms, int64_t* nlaunch) {
     const int64_t n = A.p.n;
     if (kind == 0) {
-        if (A.vturb_on)
+        if (A.vturb_on) {
             k_adj_vturb<NPMAX><<<adj_grid(k_adj_vturb<NPMAX>, n, num_sms, kAdjVtBlock), kAdjVtBlock, 0, st>>>(
                 A, F, s, prec, find, kappa, tv);
+            *nlaunch += 1;
+        }
         k_adj_step<<<adj_grid(k_adj_step, n, num_sms, kAdjBlock), kAdjBlock, 0, st>>>(A, F, s, tv);
     } else if (kind == 1) {
         k_adj_tangent<NPMAX><<<adj_grid(k_adj_tangent<NPMAX>, n, num_sms, kAdjBlock), kAdjBlock, 0, st>>>(
@@ -258,22 +260,27 @@ static cudaError_t adj_launch_t(int kind, const RpStepArgs& A, const AdjFrames& 
         k_adj_reverse_dual<NPMAX><<<adj_grid(k_adj_reverse_dual<NPMAX>, n, num_sms, kAdjBlock), kAdjBlock, 0, st>>>(
             A, F, s, prec, kappa, lx, ly, lz, kbar);
     } else {
-        if (A.vturb_on)
+        if (A.vturb_on) {
             k_adj_vturb_rev<NPMAX><<<adj_grid(k_adj_vturb_rev<NPMAX>, n, num_sms, kAdjVtBlock), kAdjVtBlock, 0,
                                      st>>>(A, F, s, prec, kappa, tv);
+            *nlaunch += 1;
+        }
         k_adj_reverse<<<adj_grid(k_adj_reverse, n, num_sms, kAdjBlock), kAdjBlock, 0, st>>>(A, F, s, tv, lx, ly, lz,
                                                                                             kbar);
     }
+    *nlaunch += 1;
     return cudaGetLastError();
 }
 
 cudaError_t launch_adj(int kind, const RpStepArgs& A, const AdjFrames& F, const AdjStateDev& s, double* prec, int find,
                        double kappa, double* tv, double* t, double* lx, double* ly, double* lz, double* kbar,
-                       int npmax, cudaStream_t st, int num_sms) {
+                       int npmax, cudaStream_t st, int num_sms, int64_t* nlaunch) {
     if (A.p.n <= 0) return cudaSuccess;
-    if (npmax <= 88) return adj_launch_t<88>(kind, A, F, s, prec, find, kappa, tv, t, lx, ly, lz, kbar, st, num_sms);
-    if (npmax <= 128) return adj_launch_t<128>(kind, A, F, s, prec, find, kappa, tv, t, lx, ly, lz, kbar, st, num_sms);
-    return adj_launch_t<144>(kind, A, F, s, prec, find, kappa, tv, t, lx, ly, lz, kbar, st, num_sms);
+    if (npmax <= 88)
+        return adj_launch_t<88>(kind, A, F, s, prec, find, kappa, tv, t, lx, ly, lz, kbar, st, num_sms, nlaunch);
+    if (npmax <= 128)
+        return adj_launch_t<128>(kind, A, F, s, prec, find, kappa, tv, t, lx, ly, lz, kbar, st, num_sms, nlaunch);
+    return adj_launch_t<144>(kind, A, F, s, prec, find, kappa, tv, t, lx, ly, lz, kbar, st, num_sms, nlaunch);
 }
 
 // Fortran-ordered field (+ Stokes term, summed in FP64) -> [j][i][k] FP64

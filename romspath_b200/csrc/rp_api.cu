@@ -1637,8 +1637,7 @@ int rp_forward(rp_ctx* ctx, int32_t nsteps, const rp_adj_step* steps, double kap
         adj_args(ctx, steps[k], A, F, n);
         if ((rc = adj_order(ctx, A, cur, n, since)) != RP_OK) return rc;
         CK(rp::launch_adj(0, A, F, cur, J.prec + (size_t)k * n, 1, kappa, J.tv, nullptr, nullptr, nullptr, nullptr, nullptr,
-                          ctx->npmax, s, ctx->num_sms));
-        ctx->launches++;
+                          ctx->npmax, s, ctx->num_sms, &ctx->launches));
     }
     CK(adj_copy(cur, adj_view((char*)J.ck + blk * (size_t)nseg, n), n, s));   // final state
     CK(cudaStreamSynchronize(s));
@@ -1679,8 +1678,7 @@ int rp_backward(rp_ctx* ctx, const double* dL_dx, const double* dL_dy, const dou
                 adj_args(ctx, J.steps[k], A, F, n);
                 if ((rc = adj_order(ctx, A, work, n, since)) != RP_OK) return rc;
                 CK(rp::launch_adj(0, A, F, work, J.prec + (size_t)k * n, 0, J.kappa, J.tv, nullptr, nullptr, nullptr,
-                                  nullptr, nullptr, ctx->npmax, s, ctx->num_sms));
-                ctx->launches++;
+                                  nullptr, nullptr, ctx->npmax, s, ctx->num_sms, &ctx->launches));
             }
         }
         // reverse steps of the segment
@@ -1691,8 +1689,8 @@ int rp_backward(rp_ctx* ctx, const double* dL_dx, const double* dL_dy, const dou
             rp::AdjStateDev at = adj_view((char*)J.seg + blk * (size_t)(k - k0), n);
             if ((rc = adj_order(ctx, A, at, n, since)) != RP_OK) return rc;
             CK(rp::launch_adj(2, A, F, at, J.prec + (size_t)k * n, 0,
-                              J.kappa, J.tv, nullptr, J.lx, J.ly, J.lz, J.kbar, ctx->npmax, s, ctx->num_sms));
-            ctx->launches++;
+                              J.kappa, J.tv, nullptr, J.lx, J.ly, J.lz, J.kbar, ctx->npmax, s, ctx->num_sms,
+                              &ctx->launches));
         }
     }
     if ((dL_dx0 && (rc = d2h(ctx, dL_dx0, J.lx, (size_t)n * 8, s))) ||
@@ -1729,8 +1727,7 @@ int rp_adj_replay(rp_ctx* ctx, const double* x0, const double* y0, const double*
         adj_args(ctx, J.steps[k], A, F, n);
         if ((rc = adj_order(ctx, A, work, n, since)) != RP_OK) return rc;
         CK(rp::launch_adj(0, A, F, work, J.prec + k * n, 0, kappa, J.tv, nullptr, nullptr, nullptr, nullptr, nullptr,
-                          ctx->npmax, s, ctx->num_sms));
-        ctx->launches++;
+                          ctx->npmax, s, ctx->num_sms, &ctx->launches));
     }
     if ((xf && (rc = d2h(ctx, xf, work.x, (size_t)n * 8, s))) || (yf && (rc = d2h(ctx, yf, work.y, (size_t)n * 8, s))) ||
         (zf && (rc = d2h(ctx, zf, work.z, (size_t)n * 8, s))))
@@ -1748,13 +1745,13 @@ int rp_tangent(rp_ctx* ctx, double kappa, double* jac) {
     const rp::AdjStateDev work = adj_view(J.work, n);
     CK(adj_copy(adj_view(J.ck, n), work, n, s));
     CK(rp::launch_adj_tangent_init(J.tan, n, s));
+    ctx->launches++;
     for (size_t k = 0; k < J.steps.size(); k++) {
         RpStepArgs A;
         AdjFrames F;
         adj_args(ctx, J.steps[k], A, F, n);
         CK(rp::launch_adj(1, A, F, work, J.prec + k * n, 0, kappa, J.tv, J.tan, nullptr, nullptr, nullptr, nullptr,
-                          ctx->npmax, s, ctx->num_sms));
-        ctx->launches++;
+                          ctx->npmax, s, ctx->num_sms, &ctx->launches));
     }
     return d2h(ctx, jac, J.tan, (size_t)n * 12 * 8, s);
 }

@@ -96,10 +96,10 @@ struct AdjStateDev {
 // kind 0: step (find: search and record p in prec, else replay prec);
 // 1: tangent step (t: 12 derivatives per particle); 2: reverse step
 // (lx/ly/lz: lambda in/out, kbar: += dL/dkappa per particle).  tv: 5 n doubles
-// of scratch (VTurb's displacements and their derivatives)
+// of scratch (VTurb's displacements and their derivatives); *nlaunch: += kernels launched
 cudaError_t launch_adj(int kind, const RpStepArgs& A, const AdjFrames& F, const AdjStateDev& s, double* prec, int find,
                        double kappa, double* tv, double* t, double* lx, double* ly, double* lz, double* kbar,
-                       int npmax, cudaStream_t st, int num_sms);
+                       int npmax, cudaStream_t st, int num_sms, int64_t* nlaunch);
 cudaError_t launch_adj_store(const double* src, const double* add, double* dst, int ni, int nj, int nk, int64_t e0,
                              int64_t count, cudaStream_t s);
 cudaError_t launch_adj_tangent_init(double* t, int64_t n, cudaStream_t s);

@@ -35,7 +35,8 @@ cudaError_t launch_order(const RpStepArgs&, int, const SortBufs& b, cudaStream_t
 }
 cudaError_t launch_unsort(int, const void*, void*, const uint32_t*, uint32_t, int64_t, int64_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t launch_adj(int, const RpStepArgs&, const AdjFrames&, const AdjStateDev& s, double*, int, double, double*, double*,
-                       double*, double*, double*, double*, int, cudaStream_t, int) {
+                       double*, double*, double*, double*, int, cudaStream_t, int, int64_t* nlaunch) {
+    *nlaunch += 2;
     return fake_note_adj(s.order != nullptr) ? cudaErrorLaunchFailure : cudaGetLastError();
 }
 cudaError_t launch_adj_store(const double*, const double*, double*, int, int, int, int64_t, int64_t, cudaStream_t) { return cudaSuccess; }

@@ -120,3 +120,31 @@ def test_forward_matches_oracle(spec, param):
     assert np.array_equal(got["status"], want["status"])
     for c, tol in (("x", 1e-7), ("y", 1e-7), ("z", 1e-6)):
         assert np.abs(got[c] - want[c]).max() <= tol, c
+
+
+# kernels of the adjoint pair by what rp_kernel_launches tells: VTurb is a kernel of
+# its own but in the tangent and where the sub-steps are more than its reverse keeps
+@pytest.mark.parametrize("param,fwd,rev", [({}, 2, 2), ({"vturb_on": 0}, 1, 1), ({"deltat": 3.0}, 2, 1)])
+def test_launches_are_counted(param, fwd, rev):
+    from romspath_b200 import Tracker, schedule
+    from romspath_b200.adjoint import Adjoint, step_table
+    n = 128
+    case = harness.make_case("tiny", n, seed=11, param_over=param)
+    T = Tracker(case.specs, case.grids, case.params, numpar=n, field_dtype="f64", seed=7)
+    for (k, slot) in schedule.initial_loads():
+        T.upload_frame(1, slot, case.frame(k))
+    T.locate(case.release, t_b=1)
+    steps = step_table(2.0, int(case.params["dt"]), int(case.params["idt"]))[0][:6]
+    adj = Adjoint(T)
+    adj.load_frames(max(max(s.frame_b, s.frame_c, s.frame_f) for s in steps), lambda ng, k: case.frame(k, ng))
+    z = np.zeros(n)
+
+    def launches(f):
+        l0 = T.kernel_launches()
+        f()
+        return T.kernel_launches() - l0
+
+    assert launches(lambda: adj.forward(steps, checkpoint_every=3)) == 6 * fwd
+    assert launches(lambda: adj.backward(z, z, z)) == 4 * fwd + 6 * rev
+    assert launches(adj.replay) == 6 * fwd
+    T.close()

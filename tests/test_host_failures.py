@@ -153,3 +153,17 @@ def test_kept_adjoint_buffers_are_bounded(fake, tracker, first, second):
     A.forward(steps[:second[0]], checkpoint_every=second[1])
     A.backward(z, z, z)
     assert fake.fake_bytes() - empty <= 2 * need
+
+
+def test_adjoint_launches_are_counted_as_told(fake, tracker):
+    T = tracker(64)
+    A, steps = _adjoint(T, 6)
+    z = np.zeros(64)
+    l0 = T.kernel_launches()
+    A.forward(steps, checkpoint_every=3)               # each launcher call of the fake tells two kernels
+    assert T.kernel_launches() - l0 == 2 * 6
+    A.backward(z, z, z)
+    assert T.kernel_launches() - l0 == 2 * (6 + 4 + 6)
+    A.replay()
+    A.tangent()
+    assert T.kernel_launches() - l0 == 2 * (6 + 4 + 6 + 6 + 6) + 1    # the tangent's start is one more
