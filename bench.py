@@ -85,8 +85,8 @@ def parse():
                          "frames and noise and report the mixed form's position / profile error")
     ap.add_argument("--days", type=float, default=10.0, help="error study length")
     ap.add_argument("--kernel-form", default="fused", choices=["fused", "split", "smem", "fused-noprefetch"],
-                    help="kernel form of the timed forms (rp_set_kernel_form; smem and fused-noprefetch: mixed "
-                         "forms only, the exact forms run those fused)")
+                    help="kernel form of the timed mixed forms (rp_set_kernel_form; the exact forms run the same "
+                         "kernels under every one)")
     ap.add_argument("--param", action="append", default=[], metavar="KEY=VALUE",
                     help="override one of the workload's run parameters in the timed forms (e.g. vturb_on=0, "
                          "sub=2, deltat=300) to time parts of the step; the line's config lists the overrides")
@@ -671,8 +671,7 @@ def features_run(args):
         ("behave10+wetdry", dict(synth.FUCHS_SAMPLE, behavior=10, va_flag=0, wetdry=1)),
         ("all", dict(synth.FUCHS_SAMPLE, behavior=10, va_flag=0, wetdry=1, **synth_diag)),
     ]
-    variants += [("passive/split", {}), ("all/split", variants[-1][1]),
-                 ("mixed/passive", {}), ("mixed/diagnostics", dict(synth_diag)),
+    variants += [("mixed/passive", {}), ("mixed/diagnostics", dict(synth_diag)),
                  ("mixed/behave10", dict(synth.FUCHS_SAMPLE, behavior=10, va_flag=0)),
                  ("mixed/wetdry", {"wetdry": 1}),
                  ("mixed/all", dict(synth.FUCHS_SAMPLE, behavior=10, va_flag=0, wetdry=1, **synth_diag))]
@@ -684,7 +683,7 @@ def features_run(args):
         params = dict(params0, **pov)
         form = "mixed" if name.startswith("mixed/") else spec.field_dtype
         T = Tracker([spec], [grid], params, numpar=npart, field_dtype=form, stokes=spec.stokes,
-                    seed=7, resort=args.resort, variant="split" if name.endswith("/split") else "fused")
+                    seed=7, resort=args.resort)
         for k, slot in enumerate((1, 2, 3)):
             T.upload_frame(1, slot, frames[k])
         T.locate(rel, t_b=1)

@@ -465,17 +465,18 @@ int rp_adj_replay(rp_ctx *ctx, const double *x0, const double *y0, const double 
  * the run under each setting).  No counterpart in the reference. */
 int rp_set_launch(rp_ctx *ctx, int32_t resort, int32_t blocks_per_sm);
 
-/* Change the kernel form of rp_params.reserved[0] between steps: 0 fused
- * (one kernel per step, the fit's workspace in local memory), 1 split (a
- * VTurb kernel writing each particle's displacement, then the advection
- * kernel), and for the mixed forms 2, the split form with the VTurb
- * kernel's spline workspace in shared memory, 3, the fused kernel whose
- * back substitution does not load u ahead, and 4 and 5, the fused kernel
- * in blocks of 64 and 256 threads instead of 128 (the exact forms run 2-5
- * fused).  Results do not change beyond rounding (the exact forms:
- * not at all); which form is fastest depends on the grid and the particle
- * count, so an autotuner times them on the run.  No counterpart in the
- * reference. */
+/* Change the kernel form of rp_params.reserved[0] between steps.  Mixed
+ * forms, with VTurb on: 0 fused (one kernel per step, the fit's workspace in
+ * local memory), 1 split (a VTurb kernel writing each particle's
+ * displacement, then the advection kernel), 2 the split form with the VTurb
+ * kernel's spline workspace in shared memory, 3 the fused kernel whose back
+ * substitution does not load u ahead, 4 and 5 the fused kernel in blocks of
+ * 64 and 256 threads instead of 128; without VTurb every form is the
+ * advection kernel alone.  The exact forms take every value and run the same
+ * kernels, VTurb's and the advection's.  Results do not change beyond
+ * rounding (the exact forms: not at all); which form is fastest depends on
+ * the grid and the particle count, so an autotuner times them on the run.  No
+ * counterpart in the reference. */
 int rp_set_kernel_form(rp_ctx *ctx, int32_t form);
 
 /* Timing of the last rp_step launch sequence on the compute stream, in ms

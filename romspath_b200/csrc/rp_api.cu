@@ -62,8 +62,9 @@ struct rp_ctx {
     int32_t* gid = nullptr;
     int8_t* isin = nullptr;
     uint32_t *pid = nullptr, *flags = nullptr;
-    double* turbv = nullptr;                   // scratch, 12 B per particle: the re-sort's gathers; the mixed
-                                               // form's VTurb displacement, tdepth and ZBehav (3 floats)
+    double* turbv = nullptr;                   // scratch, 12 B per particle: the re-sort's gathers; the exact
+                                               // step's VTurb displacements (a double); the mixed form's,
+                                               // tdepth and ZBehav (3 floats)
     // diagnostics (RP_DIAG_* bits of reserved[3]); null when off
     int diag = 0;
     double *d_salt = nullptr, *d_temp = nullptr, *d_mean_salt = nullptr, *d_mean_temp = nullptr;

@@ -68,11 +68,12 @@ class Tracker:
             P.constant_hturb[i] = float(v)
         P.seed = int(seed)
         P.device = int(device)
-        # kernel form: "fused" (one kernel, spline workspace in local
-        # memory), "split" (a VTurb kernel writing each particle's
-        # displacement to a scratch array, then the advection kernel) or,
-        # in the mixed form, "smem" (the split form with the VTurb kernel's
-        # spline workspace in shared memory)
+        # kernel form of the mixed forms: "fused" (one kernel, spline
+        # workspace in local memory), "split" (a VTurb kernel writing each
+        # particle's displacement to a scratch array, then the advection
+        # kernel), "smem" (the split form with the VTurb kernel's spline
+        # workspace in shared memory) and set_kernel_form's; the exact forms
+        # take every one and always run their VTurb and advection kernels
         P.reserved[0] = self.FORMS[variant]
         # re-sort the particle state by grid and cell every `resort` internal
         # steps (0: never); results are unchanged
@@ -336,9 +337,10 @@ class Tracker:
     FORMS = {"fused": 0, "split": 1, "smem": 2, "fused-noprefetch": 3, "fused-b64": 4, "fused-b256": 5}
 
     def set_kernel_form(self, form: str):
-        """Kernel form between steps (rp_set_kernel_form): "fused", "split",
-        and in the mixed forms "smem", "fused-noprefetch", "fused-b64" and
-        "fused-b256" (64- and 256-thread blocks)."""
+        """Kernel form of the mixed forms between steps (rp_set_kernel_form):
+        "fused", "split", "smem", "fused-noprefetch", "fused-b64" and
+        "fused-b256" (64- and 256-thread blocks); the exact forms take every
+        one and run the same kernels."""
         self._check(self.L.rp_set_kernel_form(self.h, self.FORMS[form]), "rp_set_kernel_form")
 
     def set_launch(self, resort: int, blocks_per_sm: int):
