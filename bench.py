@@ -37,9 +37,11 @@ from __future__ import annotations
 
 import argparse
 import dataclasses
+import hashlib
 import json
 import math
 import os
+import re
 import subprocess
 import sys
 import tempfile
@@ -190,6 +192,47 @@ def profile_fp64(workload, kernel):
             return None
         return d.get("kernels", {}).get(kernel)
     return None
+
+
+# the sources of the step's kernels; counters taken from another build of them
+# say nothing about this one
+STEP_SOURCES = ("rp_internal.h", "rp_device.cuh", "rp_step.cuh", "rp_mixed.cuh", "rp_kernels.cu", "rp_mixed.cu")
+
+
+def kernel_build():
+    """Id of the step's kernels as they stand: a hash of their sources without
+    comments and white space."""
+    h = hashlib.sha256()
+    for f in STEP_SOURCES:
+        text = open(os.path.join(ROOT, "romspath_b200", "csrc", f)).read()
+        text = re.sub(r"//[^\n]*|/\*.*?\*/", "", text, flags=re.S)
+        h.update(f.encode() + re.sub(r"\s+", " ", text).encode())
+    return h.hexdigest()[:12]
+
+
+def step_counters(workload, form):
+    """ncu's counts of one internal step of `form`, summed over its kernels: DRAM
+    and L2 bytes, FP64 operations, the FP64 pipe's activity over their time.  None
+    where a kernel has no summary of this build in that form."""
+    tot = {"particles": None, "ncu_ms": 0.0, "dram_bytes": 0, "lts_bytes": 0, "fp64_flop": 0, "pipe": 0.0}
+    for k in KERNELS[form]:
+        p = os.path.join(ROOT, "profiles", f"step_{workload}_traffic.json")
+        try:
+            t = json.load(open(p)).get("kernels", {}).get(k)
+        except (OSError, ValueError):
+            return None
+        f = profile_fp64(workload, k)
+        if not t or not f or {t.get("build"), f.get("build")} != {kernel_build()} or {t["form"], f["form"]} != {form}:
+            return None
+        tot["particles"] = f["particles"]
+        tot["ncu_ms"] += t["ncu_ms"]
+        tot["dram_bytes"] += t["dram_bytes_per_launch"]
+        tot["lts_bytes"] += t["lts_bytes_per_launch"]
+        tot["fp64_flop"] += f["fp64_flop_per_launch"]
+        tot["pipe"] += f["fp64_pipe_active_pct"] * t["ncu_ms"]
+        tot["source"] = f["source"]
+    tot["pipe"] /= tot["ncu_ms"]
+    return tot
 
 
 # B200 FP64 (vector and tensor core) nominal peak: 296 TFLOP/s per 8-GPU
@@ -886,7 +929,9 @@ FORM_DESC = {
     "f32": "exact: FP64 arithmetic on FP32-stored fields (bit-identical to the CPU oracle)",
     "f64": "plain FP64: FP64-stored fields, FP64 arithmetic (bit-identical to the CPU oracle)",
 }
-KERNEL = {"mixed": "k_step_mixed", "mixed-i16": "k_step_mixed", "f32": "k_step_fused", "f64": "k_step_fused"}
+# the kernels of one internal step with VTurb on
+KERNELS = {"mixed": ("k_step_mixed",), "mixed-i16": ("k_step_mixed",), "f32": ("k_vturb", "k_advect"),
+           "f64": ("k_vturb", "k_advect")}
 # algorithmic bytes per particle-step of each form on the cfg2 / cfg3 grids
 B_ALG_FORM = {("cfg2", "mixed"): 1872, ("cfg2", "mixed-i16"): 1872, ("cfg2", "f32"): 3192, ("cfg2", "f64"): 6248,
               ("cfg3", "mixed"): 1632, ("cfg3", "mixed-i16"): 1632, ("cfg3", "f64"): 5288, ("cfg1", "f64"): 5288}
@@ -1107,8 +1152,11 @@ def main():
     peak, peak_src = measured_peaks()
     balg = B_ALG_FORM.get((wl, head), 1872)
     achieved = balg * npart / (hr["avg_launch_ms"] / 1e3) / 1e9
-    traffic = profile_traffic(wl, KERNEL[head])
-    l2_traffic = profile_traffic(wl, KERNEL[head], "lts_bytes_per_launch")
+    # counts of another kernel form, or with other run parameters, are not these launches'
+    counted = args.kernel_form == "fused" and not overrides and npart == synth.CONFIG_PARTICLES[wl]
+    counters = {f: step_counters(wl, f) if counted else None for f in results}
+    traffic = counters[head]["dram_bytes"] if counters[head] else None
+    l2_traffic = counters[head]["lts_bytes"] if counters[head] else None
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "traffic": traffic, "peak_source": peak_src,
                 "dram_gbs_from_traffic": (traffic / (hr["avg_launch_ms"] / 1e3) / 1e9) if traffic else None,
@@ -1117,7 +1165,7 @@ def main():
                 "note": "achieved counts the field and particle bytes the reference arithmetic consumes at the "
                         "form's storage widths; DRAM traffic is dominated by the smoothing-spline workspace in "
                         "local memory (see profiles/)",
-                "kernel": f"{KERNEL[head]} (one launch per internal step)",
+                "kernel": f"{' + '.join(KERNELS[head])} (one launch per internal step)",
                 "avg_launch_ms": hr["avg_launch_ms"],
                 "algorithmic_bytes": f"{balg} B/particle-step x {npart} particles per launch"}
 
@@ -1129,13 +1177,12 @@ def main():
         f, p = r["spline_fits"], r["spline_passes"]
         d = {"fits_per_particle_step": f / (npart * 12), "chol1d_passes_per_fit": (p / f) if f else None,
              "np": np_fit}
-        prof = profile_fp64(wl, KERNEL[form])
-        if prof and prof.get("form") == form:
-            fl = prof["fp64_flop_per_launch"] / prof["particles"]
+        prof = counters[form]
+        if prof:
+            fl = prof["fp64_flop"] / prof["particles"]
             d.update({"fp64_flop_per_particle_step": fl,
                       "fp64_tflops": fl * npart / (r["avg_launch_ms"] / 1e3) / 1e12,
-                      "fp64_pipe_active_pct": prof.get("fp64_pipe_active_pct"),
-                      "fp64_source": prof.get("source")})
+                      "fp64_pipe_active_pct": prof["pipe"], "fp64_source": prof["source"]})
         return d
 
     spline = {"form": head, **spline_of(head),
