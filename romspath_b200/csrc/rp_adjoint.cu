@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(kAdjVtBlock, 512 / kAdjVtBlock)
 
 // The same with its derivatives in the start's x, y, z and in kappa: tv[q n],
 // q = 0..4 (b_vturb_rev).  A reverse step (this kernel and k_adj_reverse) on
-// the workload above takes 0.62 ms, 1.9 with the fit carried in dual numbers.
+// the workload above takes 0.65 ms, 1.9 with the fit carried in dual numbers.
 template <int NPMAX>
 __global__ void __launch_bounds__(kAdjVtBlock, 512 / kAdjVtBlock)
     k_adj_vturb_rev(const __grid_constant__ RpStepArgs A, const __grid_constant__ AdjFrames F, AdjStateDev s,

@@ -596,8 +596,8 @@ cudaError_t adj_copy(const rp::AdjStateDev& a, const rp::AdjStateDev& b, int64_t
 // The order in which the adjoint kernels take the particles of state `s`: by
 // grid and cell as they lie now, kept for kAdjOrderSteps launches (a particle
 // crosses a few tenths of a cell meanwhile).  130x98x20 with 65,536 particles:
-// 24 steps forward and back 33.5 ms, 38.6 as they lie.  Few particles are bound by latency, not by their
-// gathers, and stay as they lie.  So do all where there is no memory for the
+// 24 steps forward and back 36.4 ms, 41.9 as they lie.  Few particles are bound
+// by latency, not by their gathers, and stay as they lie.  So do all where there is no memory for the
 // order's buffers: since = kAdjAsTheyLie for the rest of the call.
 constexpr int kAdjOrderSteps = 12;
 constexpr int64_t kAdjOrderMin = 8192;

@@ -243,8 +243,8 @@ __device__ __forceinline__ double rp_ld(const void* base, int64_t idx) {
 // Dev. 34(1), 1990), if y = RN(1/b) and q is within one ulp of a/b, then
 // RN(q + (a - bq) y) = RN(a/b); the first correction brings RN(a y) within
 // one ulp.  Operands outside about [1e-150, 1e150] in magnitude (where a residual
-// could underflow), zero, Inf or NaN take the IEEE division instead, so the
-// result is always the correctly rounded quotient -- the value `a / b`
+// could underflow), a zero divisor, Inf or NaN take the IEEE division instead, so
+// the result is always the correctly rounded quotient -- the value `a / b`
 // gives -- while divisions sharing a denominator share one reciprocal.
 // (2^-498 and 2^498 here: the test is one of the biased exponent, in the
 // integer pipe.)

@@ -16,19 +16,21 @@ namespace rp {
 //
 // k_vturb: eight chol1d passes of some 124 rows per particle.  With few
 // particles a warp's chain of dependent FP64 operations sets the time, with
-// many the passes' traffic: 72 B a row and pass through L2 and DRAM, about
-// 5 TB/s.  On the 512x384x30 grid with 1,048,576 particles the step (both
-// kernels) takes 14.3 ms, 24.9 as one kernel whose rows divided by the IEEE
-// operator four times (102,000 FP64 instructions per warp and fit, 65,000
-// now); on the 130x98x20 grid with 10,000 particles 0.33 ms, 0.73 before.
+// many the passes' traffic: 72 B a row and pass through L2 and DRAM (70 GB a
+// launch, 5.2 TB/s).  On the 512x384x30 grid with 1,048,576 particles the step
+// (both kernels) takes 14.4 ms, 24.9 as one kernel whose rows divided by the
+// IEEE operator four times (102,000 FP64 instructions per warp and fit, 65,000
+// now); on the 130x98x20 grid with 10,000 particles, waited for, 0.33 ms, 0.70
+// before.
 //
 // k_advect: four stages of gathers.  Five 128-thread blocks an SM (96
 // registers) took 0.78 ms at 1,048,576 particles, four 0.83, six 0.79, eight
 // 0.82; its stages unrolled and its levels walked, 2.1 ms in blocks of 168
-// registers and 1.1 ms fused at 64.  A (point, level)'s ring slots come
+// registers and 1.1 ms fused at 64 (with the loads below five take 0.73, four
+// 0.80, three 0.97).  A (point, level)'s ring slots come
 // from one 16-byte load (FP64 fields: two) instead of one for each slot: an
 // interval of the 512x384x30 run without VTurb 10.9 -> 9.9 ms, a step of the
-// 130x98x20 run with 10,000 particles 166 -> 150 us.
+// 130x98x20 run with 10,000 particles 166 -> 150 us (three such runs at once).
 
 // VTurb alone, one warp per block.  SU: the fits' u in shared memory.
 template <typename T, int NPMAX, bool SU>
@@ -69,10 +71,11 @@ static cudaError_t launch_vturb(const RpStepArgs& A, int np, double* turbv, cuda
     const size_t smem = (size_t)np * 32 * sizeof(double);      // the warp's u
     // Where every warp can be resident with its u in shared memory (1 KB a
     // particle at 124 points: 7 warps an SM) it is: the rows then wait for
-    // L2 less often (130x98x20 grid, 10,000 particles: 0.33 ms a step, 0.37
-    // with u in local memory).  With more particles than that, 16 warps an
-    // SM with u in local memory hide more than shared memory saves
-    // (512x384x30, 1,048,576 particles: 14.3 ms against 18.3).
+    // L2 less often (a step of 10,000 particles on the 130x98x20 grid 326 us,
+    // 332 with u in local memory; of 500 on 24x20x6 138 and 145).  With more
+    // particles than that, 16 warps an SM with u in local memory hide more than
+    // shared memory saves (512x384x30, 1,048,576 particles: 14.6 ms against
+    // 17.8).
     const int64_t need = (A.p.n + 31) / 32;
     const int64_t fit = grid_for(k_vturb<T, NPMAX, true>, 32, smem, A.p.n, num_sms, &e, cap);
     if (e != cudaSuccess) return e;

@@ -24,7 +24,7 @@ namespace rp {
 // the data resampled beforehand 17.1 and 49.3 ms at four, 18.0 and 50.0 at five.
 // FEAT: built with the options beyond the passive step (diagnostics,
 // WETDRY, behave); the passive variant is chosen when they are all off.
-// BLK: threads per block (the register cap stays that of 128 x 8 resident
+// BLK: threads per block (the register cap stays that of 128 x 4 resident
 // threads; the block is the scheduling unit of the grid-stride loop).
 template <typename E, int NPMAX, bool FEAT, bool PREF = true, int BLK = kStepBlock>
 __global__ void __launch_bounds__(BLK, kMixedMinBlocks * kStepBlock / BLK)
